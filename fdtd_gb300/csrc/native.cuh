@@ -71,7 +71,8 @@ struct NativeConsts {
     // per plane of the chunk whose tile holds only classes without
     // relaxation (R stays +0 there: not loaded, not stored); may be null
     const unsigned long long *memless;
-    int memless_rows;      // tile rows the masks were made for (other tile heights ignore them)
+    int memless_rows;      // tile rows and planes per chunk the masks were made for (a launch with
+    int memless_zchunk;    // others ignores them)
     // Mur slabs that hold one value (slab s: x0, y0, z0, x_end, y_end, z_end,
     // i.e. face normal s % 3, far face s / 3; set when every entry of both
     // layers of the slab is that value, as for slabs made from the default
@@ -223,6 +224,11 @@ int fused_tile_height();
 int fused_zchunk(int nz);
 int compact_zchunk(int nz);
 int zchunk_limited(int nz, int max_planes);  // nz in equal chunks of at most max_planes planes
+// z chunk of one solve's launch: equal chunks of at most max_planes planes,
+// shorter ones where columns (column tiles) x chunks would leave the device's
+// `resident` CTAs idle in the first wave or nearly empty in the last; start:
+// what a CTA costs before its first plane, in planes.
+int balanced_zchunk(int nz, int max_planes, long long columns, int resident, double start);
 // One batched step: fused kernel over all units, Mur faces, step counters.
 int launch_batch_step(const BatchLaunch &b, cudaStream_t s);
 int batch_persistent_ctas(bool compact, int nclasses, bool r16 = false);
@@ -236,10 +242,12 @@ int batch_strip_ctas(bool r16, int shape, int nclasses);
 // multiple of 16 cells, 16-byte aligned bases, R updated in place).
 bool strip_usable(const NativeConsts &c, bool r16);
 // Strip shapes (0 .. 3) and their tile rows; the shape a single solve runs
-// (FDTD_STRIP_SHAPE overrides); the z chunk of a single solve's strip launch.
+// (FDTD_STRIP_SHAPE overrides); the default z chunk, and that of a single
+// solve's launch.
 int strip_shape_rows(int shape);
 int strip_single_shape(bool r16);
 int strip_zchunk(int nz);
+int strip_solve_zchunk(int nx, int ny, int nz, bool r16, int nclasses);
 // Memoryless tile-planes (see NativeConsts::memless): strip_plane_flags marks
 // each (z, 32 x 8 tile) whose cells all have classes with tau
 // (specs[4 k + 3]) = 0, for a class volume of row pitch `pitch`, laid out

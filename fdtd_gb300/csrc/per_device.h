@@ -9,9 +9,36 @@
 // GPU.
 #pragma once
 
+#include <atomic>
 #include <mutex>
 
 namespace fdtd {
+
+// A small positive number per device and key (a kernel's resident CTAs at a
+// class count, say) that is looked up once and then read without a lock.
+// compute() returns the number, or a value below 1 when it has none (asked
+// again on the next call).  Two threads may both compute it on first use; it
+// is the same number.
+template <int KEYS, int MAX_DEVICES = 64>
+class PerDeviceValue {
+public:
+    template <class F>
+    int get(int dev, int key, F &&compute)
+    {
+        if (dev < 0 || dev >= MAX_DEVICES || key < 0 || key >= KEYS)
+            return compute();
+        int v = value_[dev][key].load(std::memory_order_relaxed);
+        if (v < 1) {
+            v = compute();
+            if (v >= 1)
+                value_[dev][key].store(v, std::memory_order_relaxed);
+        }
+        return v;
+    }
+
+private:
+    std::atomic<int> value_[MAX_DEVICES][KEYS] = {};
+};
 
 template <int MAX_DEVICES = 64>
 class PerDeviceOnce {

@@ -49,6 +49,7 @@ NativeConsts solver_consts(const fdtd_solver *s, int n)
     c.r_exp = s->rexp;
     c.memless = s->d_memless;
     c.memless_rows = s->memless_rows;
+    c.memless_zchunk = s->memless_zchunk;
     return c;
 }
 
@@ -410,7 +411,8 @@ int fdtd_solver_create(const fdtd_solver_config *cfg, fdtd_solver **out)
         const std::vector<unsigned char> flags =
             strip_plane_flags(cfg->material, p->nx, p->ny, p->nz, p->nx, cfg->specs, ncls);
         s->memless_rows = strip_shape_rows(strip_single_shape(cfg->kernel == FDTD_KERNEL_COMPACT_R16));
-        const int zchunk = strip_zchunk(p->nz);
+        const int zchunk = strip_solve_zchunk(p->nx, p->ny, p->nz, r16, ncls);
+        s->memless_zchunk = zchunk;
         std::vector<unsigned long long> masks((size_t)((p->nz + zchunk - 1) / zchunk) *
                                               ((p->ny + s->memless_rows - 1) / s->memless_rows) * ((p->nx + 31) / 32));
         s->memless_fraction =

@@ -37,7 +37,8 @@ struct fdtd_solver {
     uint32_t *rexp = nullptr;  // FDTD_KERNEL_COMPACT_R16: scale words (d[0] holds the FP16 residuals)
     unsigned long long *d_memless = nullptr;  // compact forms: the strip kernel's memoryless-plane masks
     double memless_fraction = 0.0;            // share of the cell-updates on such planes
-    int memless_rows = 0;                     // tile rows of those masks
+    int memless_rows = 0;                     // tile rows and planes per chunk of those masks
+    int memless_zchunk = 0;
     int *counter = nullptr;
     int steps = 0;
     std::map<std::pair<int, int>, cudaGraphExec_t> graphs;  // (parity, length) -> exec

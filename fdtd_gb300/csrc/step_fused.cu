@@ -26,6 +26,7 @@
 #include <cuda.h>
 #include <cudaTypedefs.h>
 
+#include <algorithm>
 #include <cstdlib>
 #include <cstring>
 
@@ -790,8 +791,9 @@ constexpr int TY_SEL = FDTD_TILE_ROWS;
 constexpr int S_SEL = FDTD_RING_STAGES;
 
 
+// zmax: the form's largest z chunk.
 template <bool TMA, bool COMPACT, bool R16 = false>
-int launch_fused_impl(const FusedArgs &a, const FusedMaps &maps, cudaStream_t s)
+int launch_fused_impl(FusedArgs &a, int zmax, const FusedMaps &maps, cudaStream_t s)
 {
     auto kernel = fused_step_kernel<TY_SEL, S_SEL, TMA, COMPACT, R16>;
     using G = GeoOf<TY_SEL, COMPACT, R16>;
@@ -810,8 +812,12 @@ int launch_fused_impl(const FusedArgs &a, const FusedMaps &maps, cudaStream_t s)
     if (so != 0)
         return so < 0 ? FDTD_ERR_INVALID : so;
     const int smem = fused_smem_bytes<S_SEL, G>(a.c.nclasses);
+    static PerDeviceValue<FDTD_MAX_CLASSES + 1> resident;
+    const int r = resident.get(dev, a.c.nclasses, [&] { return resident_ctas(kernel, FTX * TY_SEL, smem); });
+    const int tiles_x = (a.c.nx + FTX - 1) / FTX, tiles_y = (a.c.ny + TY_SEL - 1) / TY_SEL;
+    a.zchunk = balanced_zchunk(a.c.nz, zmax, (long long)tiles_x * tiles_y, r, 1.25);
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((a.c.nx + FTX - 1) / FTX, (a.c.ny + TY_SEL - 1) / TY_SEL, (a.c.nz + a.zchunk - 1) / a.zchunk);
+    cfg.gridDim = dim3(tiles_x, tiles_y, (a.c.nz + a.zchunk - 1) / a.zchunk);
     cfg.blockDim = dim3(FTX, TY_SEL);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
@@ -831,6 +837,41 @@ int zchunk_limited(int nz, int max_planes)
 {
     const int chunks = (nz + max_planes - 1) / max_planes;
     return (nz + chunks - 1) / chunks;
+}
+
+// The default chunk serves grids of many waves of CTAs.  Small and middle
+// grids are chunked by whole waves: a grid of 64^3 in 64-plane chunks has 16
+// CTAs for 152 SMs and takes as long as one CTA needs for 66 planes.  With W
+// = ceil(CTAs / resident) waves, W (chunk + start) orders the measured step
+// times of ten grids from 64^3 to 512 x 512 x 400 to within 4 % of the best
+// of 13 chunk lengths (D form, us per step, 64-plane chunks against this
+// choice: 64^3 85.6 -> 10.2, 128^3 109.6 -> 41.0, 224 x 208 x 176 188 -> 138,
+// 256 x 239 x 160 186 -> 165; the compact strip kernel, 24-plane chunks:
+// 64^3 44.0 -> 10.3, 128^3 53.9 -> 34.1, 256 x 239 x 160 128.9 -> 118.6).
+// Beyond six waves the CTAs have drifted apart, no wave ends as one, and the
+// default chunk is as good or better (512 x 512 x 400: 1568 us with 58
+// planes, 1579 with 24).
+int balanced_zchunk(int nz, int max_planes, long long columns, int resident, double start)
+{
+    const int longest = zchunk_limited(nz, max_planes);
+    auto chunks_of = [&](int c) { return (long long)((nz + c - 1) / c); };
+    if (resident < 1 || columns * chunks_of(longest) > 6LL * resident)
+        return longest;
+    int best = longest;
+    double best_cost = 0.0;
+    for (int c = longest; c >= std::min(2, longest); c--) {
+        const long long ctas = columns * chunks_of(c);
+        if (c != zchunk_limited(nz, c))
+            continue;  // the same number of chunks as a shorter, more even one
+        if (ctas > 6LL * resident)
+            break;
+        const double cost = (double)((ctas + resident - 1) / resident) * (c + start);
+        if (c == longest || cost < best_cost) {
+            best = c;
+            best_cost = cost;
+        }
+    }
+    return best;
 }
 
 #ifndef FDTD_ZCHUNK
@@ -982,11 +1023,10 @@ int launch_h_de_fused(const NativeConsts &c, cudaStream_t s)
 {
     FusedArgs a;
     a.c = c;
-    a.zchunk = fused_zchunk(c.nz);
     FusedMaps maps;
     if (encode_step_maps(c, false, &maps))
-        return launch_fused_impl<true, false>(a, maps, s);
-    return launch_fused_impl<false, false>(a, maps, s);
+        return launch_fused_impl<true, false>(a, FDTD_ZCHUNK, maps, s);
+    return launch_fused_impl<false, false>(a, FDTD_ZCHUNK, maps, s);
 }
 
 // The compact forms run the strip kernel (step_strip.cu) wherever its TMA
@@ -1008,11 +1048,10 @@ int launch_h_e_compact(const NativeConsts &c, cudaStream_t s)
     static_assert(FDTD_COMPACT_ZCHUNK >= 4, "z chunks hold at least four planes");
     FusedArgs a;
     a.c = c;
-    a.zchunk = compact_zchunk(c.nz);  // the compact form reads no source-plane mask
     FusedMaps maps;
     if (encode_step_maps(c, true, &maps))
-        return launch_fused_impl<true, true>(a, maps, s);
-    return launch_fused_impl<false, true>(a, maps, s);
+        return launch_fused_impl<true, true>(a, FDTD_COMPACT_ZCHUNK, maps, s);
+    return launch_fused_impl<false, true>(a, FDTD_COMPACT_ZCHUNK, maps, s);
 }
 
 int launch_h_e_compact16(const NativeConsts &c, cudaStream_t s)
@@ -1023,11 +1062,10 @@ int launch_h_e_compact16(const NativeConsts &c, cudaStream_t s)
         return launch_strip_compact16(c, s);
     FusedArgs a;
     a.c = c;
-    a.zchunk = compact_zchunk(c.nz);
     FusedMaps maps;
     if (encode_step_maps(c, true, &maps, true))
-        return launch_fused_impl<true, true, true>(a, maps, s);
-    return launch_fused_impl<false, true, true>(a, maps, s);
+        return launch_fused_impl<true, true, true>(a, FDTD_COMPACT_ZCHUNK, maps, s);
+    return launch_fused_impl<false, true, true>(a, FDTD_COMPACT_ZCHUNK, maps, s);
 }
 
 int launch_step(const NativeConsts &c0, cudaStream_t s)

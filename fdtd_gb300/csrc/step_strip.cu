@@ -61,6 +61,44 @@ __global__ void __launch_bounds__(32 * W) strip_step_kernel(const __grid_constan
 #endif
 static_assert(FDTD_STRIP_ZCHUNK >= 2 && FDTD_STRIP_ZCHUNK <= 64, "a unit's memoryless-plane mask has 64 bits");
 
+// The shared-memory opt-in of a shape's kernel (it holds for the current
+// device only): a CUDA status, or -1.
+template <int SHAPE, bool R16>
+int opt_in()
+{
+    constexpr int RY = Shape<SHAPE>::RY, W = Shape<SHAPE>::W;
+    static PerDeviceOnce<> once;
+    int dev = 0;
+    const cudaError_t de = cudaGetDevice(&dev);
+    if (de != cudaSuccess)
+        return (int)de;
+    return once.run(dev, [&] {
+        return (int)cudaFuncSetAttribute(strip_step_kernel<RY, W, S_SEL, R16>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         strip_smem_bytes<RY, W, S_SEL, R16>(FDTD_MAX_CLASSES));
+    });
+}
+
+// z chunk of a single solve in this shape: at most FDTD_STRIP_ZCHUNK planes,
+// balanced over the CTAs the device holds (balanced_zchunk); the limit alone
+// where FDTD_STRIP_ZCHUNK is set in the environment.
+template <int SHAPE, bool R16>
+int solve_zchunk(int nx, int ny, int nz, int nclasses)
+{
+    constexpr int RY = Shape<SHAPE>::RY, W = Shape<SHAPE>::W;
+    using G = StripGeo<RY, W, R16>;
+    int dev = 0;
+    if (std::getenv("FDTD_STRIP_ZCHUNK") || nclasses < 1 || nclasses > FDTD_MAX_CLASSES ||
+        cudaGetDevice(&dev) != cudaSuccess || opt_in<SHAPE, R16>() != 0)
+        return strip_zchunk(nz);
+    static PerDeviceValue<FDTD_MAX_CLASSES + 1> resident;
+    const int r = resident.get(dev, nclasses, [&] {
+        return resident_ctas(strip_step_kernel<RY, W, S_SEL, R16>, G::NTH, strip_smem_bytes<RY, W, S_SEL, R16>(nclasses));
+    });
+    const long long columns = (long long)((nx + SX - 1) / SX) * ((ny + G::TY - 1) / G::TY);
+    return balanced_zchunk(nz, FDTD_STRIP_ZCHUNK, columns, r, 0.5);
+}
+
 template <int SHAPE, bool R16>
 int launch_shape(const NativeConsts &c, cudaStream_t s)
 {
@@ -71,21 +109,13 @@ int launch_shape(const NativeConsts &c, cudaStream_t s)
         return FDTD_ERR_INVALID;
     StripArgs a;
     a.c = c;
-    if (a.c.memless_rows != G::TY)
-        a.c.memless = nullptr;  // masks made for another tile height
-    a.zchunk = strip_zchunk(c.nz);
+    a.zchunk = solve_zchunk<SHAPE, R16>(c.nx, c.ny, c.nz, c.nclasses);
+    if (a.c.memless_rows != G::TY || a.c.memless_zchunk != a.zchunk)
+        a.c.memless = nullptr;  // masks made for other units
     StripMaps maps;
     if (!encode_strip_maps(c, R16, G::TY, &maps))
         return FDTD_ERR_INVALID;
-    static PerDeviceOnce<> smem_opt_in;  // the opt-in holds for the current device only
-    int dev = 0;
-    const cudaError_t de = cudaGetDevice(&dev);
-    if (de != cudaSuccess)
-        return (int)de;
-    const int so = smem_opt_in.run(dev, [&] {
-        return (int)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         strip_smem_bytes<RY, W, S_SEL, R16>(FDTD_MAX_CLASSES));
-    });
+    const int so = opt_in<SHAPE, R16>();
     if (so != 0)
         return so < 0 ? FDTD_ERR_INVALID : so;
     cudaLaunchConfig_t cfg = {};
@@ -174,6 +204,17 @@ int strip_shape_rows(int shape)
 }
 
 int strip_single_shape(bool r16) { return strip::single_shape(r16); }
+
+int strip_solve_zchunk(int nx, int ny, int nz, bool r16, int nclasses)
+{
+    switch (strip::single_shape(r16)) {
+    case 0: return r16 ? strip::solve_zchunk<0, true>(nx, ny, nz, nclasses) : strip::solve_zchunk<0, false>(nx, ny, nz, nclasses);
+    case 1: return r16 ? strip::solve_zchunk<1, true>(nx, ny, nz, nclasses) : strip::solve_zchunk<1, false>(nx, ny, nz, nclasses);
+    case 2: return r16 ? strip::solve_zchunk<2, true>(nx, ny, nz, nclasses) : strip::solve_zchunk<2, false>(nx, ny, nz, nclasses);
+    case 3: return r16 ? strip::solve_zchunk<3, true>(nx, ny, nz, nclasses) : strip::solve_zchunk<3, false>(nx, ny, nz, nclasses);
+    default: return strip_zchunk(nz);
+    }
+}
 
 int strip_zchunk(int nz)
 {

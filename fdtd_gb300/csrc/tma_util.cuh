@@ -149,6 +149,18 @@ inline bool encode_map(PFN_cuTensorMapEncodeTiled_v12000 fn, CUtensorMap *m, con
                          is_u8 ? 1 : 4, nx, ny, nz, (size_t)pitch, (size_t)pitch * ny, bx, by);
 }
 
+// CTAs of `kernel` that the current device holds at once.
+template <class K>
+int resident_ctas(K kernel, int threads, int smem)
+{
+    int dev = 0, sms = 0, per_sm = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem) != cudaSuccess)
+        return 0;
+    return sms * per_sm;
+}
+
 inline bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
 }  // namespace tma
