@@ -26,9 +26,9 @@ ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 # another ring depth (a changed value needs a forced rebuild)
 EXTRA = os.environ.get("FDTD_NVCC_FLAGS", "").split()
 
-CU_SOURCES = ["compat.cu", "native.cu", "step_fused.cu", "step_strip.cu", "batch_strip.cu", "step_static.cu", "solver.cu", "monitor.cu", "batch.cu", "cuda_util.cu"]
+CU_SOURCES = ["compat.cu", "native.cu", "step_fused.cu", "step_strip.cu", "batch_strip.cu", "step_static.cu", "solver.cu", "monitor.cu", "batch.cu", "rows.cu", "cuda_util.cu"]
 CPP_SOURCES = ["host_io.cpp"]
-HEADERS = ["fdtd_internal.h", "device_common.cuh", "native.cuh", "solver_internal.cuh", "tma_util.cuh", "per_device.h", "cell_math.cuh", "strip_unit.cuh"]
+HEADERS = ["fdtd_internal.h", "device_common.cuh", "native.cuh", "solver_internal.cuh", "tma_util.cuh", "per_device.h", "cell_math.cuh", "strip_unit.cuh", "rows.h"]
 
 
 def _run(cmd: list[str]) -> str:

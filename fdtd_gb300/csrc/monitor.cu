@@ -22,6 +22,15 @@ namespace {
 
 int cu(cudaError_t e) { return e == cudaSuccess ? FDTD_OK : (int)e; }
 
+// Element of the i-th cell of a run of rows of nx cells, pitch elements apart.
+__device__ __forceinline__ size_t row_element(size_t i, unsigned nx, unsigned pitch)
+{
+    if (nx == pitch)
+        return i;
+    const size_t row = i / nx;
+    return row * pitch + (i - row * nx);
+}
+
 struct MonitorArgs {
     const int *counter;        // completed steps (advanced by the step's last kernel)
     const float *e[3];         // E after the step
@@ -33,7 +42,8 @@ struct MonitorArgs {
     int dft_on, stride;
     double omega, wdt;         // 2 pi f, stride * dt
     double dt;
-    size_t base, count;        // first cell and number of cells of the DFT planes
+    size_t base, count;        // first element and number of cells of the DFT planes
+    unsigned nx, pitch;        // cells per row, elements between rows of E
     double *acc;               // re x,y,z then im x,y,z (count each)
 };
 
@@ -63,9 +73,10 @@ __global__ void __launch_bounds__(256) monitor_kernel(MonitorArgs a)
     __syncthreads();
     const double c = cs[0], s = cs[1];
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < a.count; i += (size_t)gridDim.x * blockDim.x) {
+        const size_t j = a.base + row_element(i, a.nx, a.pitch);
 #pragma unroll
         for (int comp = 0; comp < 3; comp++) {
-            const double e = a.e[comp][a.base + i];
+            const double e = a.e[comp][j];
             a.acc[comp * a.count + i] += e * c;
             a.acc[(3 + comp) * a.count + i] += e * s;
         }
@@ -74,7 +85,9 @@ __global__ void __launch_bounds__(256) monitor_kernel(MonitorArgs a)
 
 struct SarArgs {
     const double *acc;
-    size_t base, count;
+    size_t base, count;        // first cell and number of cells of the planes
+    size_t mat_base;           // element of that cell in the class array
+    unsigned nx, pitch;
     const uint8_t *mat;
     float sigma[FDTD_MAX_CLASSES];
     float inv_2rho[FDTD_MAX_CLASSES];
@@ -93,7 +106,7 @@ __global__ void __launch_bounds__(256) sar_kernel(SarArgs a)
             const double re = a.acc[comp * a.count + i], im = a.acc[(3 + comp) * a.count + i];
             e2 += re * re + im * im;
         }
-        const int cls = a.mat[a.base + i];
+        const int cls = a.mat[a.mat_base + row_element(i, a.nx, a.pitch)];
         const double sar = (double)a.sigma[cls] * e2 * (double)a.inv_2rho[cls];
         if (sar > best) {
             best = sar;
@@ -146,8 +159,10 @@ int launch_monitor(fdtd_solver *s, int n)
     a.omega = 2.0 * M_PI * s->dft_freq;
     a.dt = s->plan->dt;
     a.wdt = (double)s->dft_stride * s->plan->dt;
-    a.base = (size_t)s->dft_z0 * s->nx * s->ny;
+    a.base = (size_t)s->dft_z0 * s->pitch * s->ny;
     a.count = (size_t)s->dft_np * s->nx * s->ny;
+    a.nx = s->nx;
+    a.pitch = s->pitch;
     a.acc = s->d_dft;
     monitor_kernel<<<s->dft_on ? monitor_blocks() : 1, 256, 0, s->stream>>>(a);
     return cu(cudaGetLastError());
@@ -166,7 +181,7 @@ int fdtd_solver_set_probes(fdtd_solver *s, int nprobes, const int *xyz, int capa
         const int x = xyz[3 * p], y = xyz[3 * p + 1], z = xyz[3 * p + 2];
         if (x < 0 || x >= s->nx || y < 0 || y >= s->ny || z < 0 || z >= s->nz)
             return FDTD_ERR_INVALID;
-        idx[p] = (long long)cell_index(x, y, z, s->nx, s->ny);
+        idx[p] = (long long)cell_index(x, y, z, s->pitch, s->ny);
     }
     int st = fdtd_solver_synchronize(s);
     if (st != FDTD_OK)
@@ -268,6 +283,9 @@ int fdtd_solver_peak_sar(fdtd_solver *s, const float *rho, double *peak, long lo
     a.base = (size_t)s->dft_z0 * s->nx * s->ny;
     a.count = (size_t)s->dft_np * s->nx * s->ny;
     a.mat = s->mat;
+    a.mat_base = (size_t)s->dft_z0 * s->pitch * s->ny;
+    a.nx = s->nx;
+    a.pitch = s->pitch;
     for (int k = 0; k < s->nclasses; k++) {
         const float r = rho ? rho[k] : 1000.0f;
         if (!(r > 0.0f))
@@ -329,7 +347,9 @@ static uint32_t ckp_version(const fdtd_solver *s)
 
 // The state blocks after `count` steps: H, E^n, E^{n-1}, then D^n, D^{n-1}
 // (D form), R (compact form) or the FP16 residuals and the scale words.
-static int state_blocks(fdtd_solver *s, int count, void *ptr[16], size_t bytes[16])
+// elem[k]: bytes per cell of block k, rows of which are padded on the device
+// and dense in the file; 0 for the scale words, the same in both.
+static int state_blocks(fdtd_solver *s, int count, void *ptr[16], size_t bytes[16], size_t elem[16])
 {
     const int hb = s->kernel != FDTD_KERNEL_TWO_PASS ? (count & 1) : 0;
     const int l = latest_slot(count), p = previous_slot(count);
@@ -340,6 +360,7 @@ static int state_blocks(fdtd_solver *s, int count, void *ptr[16], size_t bytes[1
         ptr[n + 3] = s->e[l][c];
         ptr[n + 6] = s->e[p][c];
         bytes[n] = bytes[n + 3] = bytes[n + 6] = fb;
+        elem[n] = elem[n + 3] = elem[n + 6] = sizeof(float);
         n++;
     }
     n = 9;
@@ -347,21 +368,38 @@ static int state_blocks(fdtd_solver *s, int count, void *ptr[16], size_t bytes[1
         for (int c = 0; c < 3; c++, n++) {
             ptr[n] = s->d[0][c];
             bytes[n] = sizeof(uint16_t) * s->ncell;
+            elem[n] = sizeof(uint16_t);
         }
         ptr[n] = s->rexp;
+        elem[n] = 0;
         bytes[n++] = sizeof(uint32_t) * r16_words(s->nx, s->ny, s->nz);
         return n;
     }
     for (int c = 0; c < 3; c++, n++) {
         ptr[n] = s->d[l][c];
         bytes[n] = fb;
+        elem[n] = sizeof(float);
     }
     if (s->kernel != FDTD_KERNEL_COMPACT)
         for (int c = 0; c < 3; c++, n++) {
             ptr[n] = s->d[p][c];
             bytes[n] = fb;
+            elem[n] = sizeof(float);
         }
     return n;
+}
+
+// A state block to or from its dense host copy.
+static int copy_block(fdtd_solver *s, void *dev, char *host, size_t bytes, size_t elem, bool to_host)
+{
+    void *dst = to_host ? (void *)host : dev;
+    const void *src = to_host ? dev : (void *)host;
+    const cudaMemcpyKind kind = to_host ? cudaMemcpyDeviceToHost : cudaMemcpyHostToDevice;
+    if (elem == 0 || s->pitch == s->nx)
+        return cu(cudaMemcpy(dst, src, bytes, kind));
+    const size_t dense = elem * s->nx, padded = elem * s->pitch;
+    return cu(cudaMemcpy2D(dst, to_host ? dense : padded, src, to_host ? padded : dense, dense,
+                           (size_t)s->ny * s->nz, kind));
 }
 
 int fdtd_solver_checkpoint(fdtd_solver *s, const char *path)
@@ -384,12 +422,12 @@ int fdtd_solver_checkpoint(fdtd_solver *s, const char *path)
     h.material_hash = s->material_hash;
     bool ok = std::fwrite(&h, sizeof h, 1, f) == 1;
     void *ptr[16];
-    size_t bytes[16];
-    const int nb = state_blocks(s, s->steps, ptr, bytes);
+    size_t bytes[16], elem[16];
+    const int nb = state_blocks(s, s->steps, ptr, bytes, elem);
     std::vector<char> buf(sizeof(float) * s->ncell);
     for (int k = 0; k < nb && ok; k++) {
         buf.resize(bytes[k]);
-        st = cu(cudaMemcpy(buf.data(), ptr[k], bytes[k], cudaMemcpyDeviceToHost));
+        st = copy_block(s, ptr[k], buf.data(), bytes[k], elem[k], true);
         ok = st == FDTD_OK && std::fwrite(buf.data(), 1, bytes[k], f) == bytes[k];
     }
     if (std::fclose(f) != 0)
@@ -419,15 +457,15 @@ int fdtd_solver_restore(fdtd_solver *s, const char *path)
         return FDTD_ERR_FORMAT;
     }
     void *ptr[16];
-    size_t bytes[16];
-    const int nb = state_blocks(s, h.steps, ptr, bytes);
+    size_t bytes[16], elem[16];
+    const int nb = state_blocks(s, h.steps, ptr, bytes, elem);
     std::vector<char> buf;
     bool ok = true;
     for (int k = 0; k < nb && ok && st == FDTD_OK; k++) {
         buf.resize(bytes[k]);
         ok = std::fread(buf.data(), 1, bytes[k], f) == bytes[k];
         if (ok)
-            st = cu(cudaMemcpy(ptr[k], buf.data(), bytes[k], cudaMemcpyHostToDevice));
+            st = copy_block(s, ptr[k], buf.data(), bytes[k], elem[k], false);
     }
     std::fclose(f);
     if (st != FDTD_OK)
@@ -438,7 +476,7 @@ int fdtd_solver_restore(fdtd_solver *s, const char *path)
     // produced the saved H read (zero where H is never updated); copy it too
     if (s->kernel != FDTD_KERNEL_TWO_PASS)
         for (int c = 0; c < 3 && st == FDTD_OK; c++)
-            st = cu(cudaMemcpy(s->h[(h.steps + 1) & 1][c], ptr[c], sizeof(float) * s->ncell,
+            st = cu(cudaMemcpy(s->h[(h.steps + 1) & 1][c], ptr[c], sizeof(float) * s->pcell,
                                cudaMemcpyDeviceToDevice));
     int steps = h.steps;
     if (st == FDTD_OK)

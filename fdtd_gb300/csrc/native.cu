@@ -166,8 +166,8 @@ __global__ void __launch_bounds__(TX *TY) native_h_kernel(NativeConsts c)
     const int x = blockIdx.x * TX + threadIdx.x, y = blockIdx.y * TY + threadIdx.y, z = blockIdx.z;
     if (x >= nx - 1 || y >= ny - 1 || z >= nz - 1)
         return;  // no H component is updated at x = nx-1, y = ny-1 or z = nz-1
-    const size_t i = cell_index(x, y, z, nx, ny);
-    const size_t sx = 1, sy = nx, sz = (size_t)nx * ny;
+    const size_t i = cell_index(x, y, z, c.pitch, ny);
+    const size_t sx = 1, sy = c.pitch, sz = (size_t)c.pitch * ny;
     const float *__restrict__ ex = c.e_cur[0];
     const float *__restrict__ ey = c.e_cur[1];
     const float *__restrict__ ez = c.e_cur[2];
@@ -193,8 +193,8 @@ __global__ void __launch_bounds__(TX *TY) native_de_kernel(NativeConsts c)
     const int x = blockIdx.x * TX + threadIdx.x, y = blockIdx.y * TY + threadIdx.y, z = blockIdx.z;
     if (x >= nx || y >= ny)
         return;
-    const size_t i = cell_index(x, y, z, nx, ny);
-    const size_t sx = 1, sy = nx, sz = (size_t)nx * ny;
+    const size_t i = cell_index(x, y, z, c.pitch, ny);
+    const size_t sx = 1, sy = c.pitch, sz = (size_t)c.pitch * ny;
     const float *__restrict__ hx = c.h_out[0];
     const float *__restrict__ hy = c.h_out[1];
     const float *__restrict__ hz = c.h_out[2];

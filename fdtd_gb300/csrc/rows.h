@@ -1,0 +1,28 @@
+// rows.h -- dense host volumes to and from device arrays of padded rows.
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include <cstddef>
+#include <cstdint>
+
+namespace fdtd {
+
+// Row pitch of a grid's arrays: a multiple of 16 cells (TMA wants 16-byte
+// strides of the class bytes too).  Rows below 16 cells stay as they are, so
+// that padding never doubles a state.
+inline int padded_rows_pitch(int nx) { return nx < 16 ? nx : (nx + 15) & ~15; }
+
+// Queues on s the copy of `rows` rows of nx floats, pitch floats apart, into
+// the dense host volume.  Page-locked memory is written by a kernel, other
+// memory through scratch (device memory that work on s may use, scratch_floats
+// long; without it a strided copy).
+cudaError_t read_rows(float *host, const float *src, size_t rows, int nx, int pitch, float *scratch,
+                      size_t scratch_floats, cudaStream_t s);
+
+// Queues on s the copy of a dense host byte volume into rows pitch bytes
+// apart; scratch: rows * nx bytes of device memory (unused where pitch is nx).
+cudaError_t write_byte_rows(uint8_t *dst, const uint8_t *host, size_t rows, int nx, int pitch, uint8_t *scratch,
+                            cudaStream_t s);
+
+}  // namespace fdtd

@@ -15,6 +15,7 @@
 #include <thread>
 #include <vector>
 
+#include "rows.h"
 #include "solver_internal.cuh"
 
 using namespace fdtd;
@@ -46,6 +47,7 @@ NativeConsts solver_consts(const fdtd_solver *s, int n)
 {
     const fdtd_native_fields f = step_fields(s, n);
     NativeConsts c = make_consts(s->plan, &f, n);
+    c.pitch = s->pitch;
     c.r_exp = s->rexp;
     c.memless = s->d_memless;
     c.memless_rows = s->memless_rows;
@@ -80,6 +82,10 @@ void reset_graphs(fdtd_solver *s)
 namespace {
 
 int cu(cudaError_t e) { return e == cudaSuccess ? FDTD_OK : (int)e; }
+
+// Staging of padded rows read into pageable memory: 16 MB (10 M floats in
+// pieces of 4 MB went as fast as in one piece).
+constexpr size_t PACK_SCRATCH_FLOATS = size_t(4) << 20;
 
 int enqueue_step(fdtd_solver *s, int n)
 {
@@ -262,11 +268,11 @@ int enqueue_snapshot(fdtd_solver *s, int step)
         st = cu(cudaEventRecord(s->ev_step, s->stream));
     if (st == FDTD_OK)
         st = cu(cudaStreamWaitEvent(s->copy_stream, s->ev_step, 0));
-    const size_t plane = (size_t)s->nx * s->ny;
+    const size_t plane = (size_t)s->pitch * s->ny;
     for (size_t k = 0; k < s->snap_fields.size() && st == FDTD_OK; k++) {
         const float *src = field_buffer(s, s->snap_fields[k], step + 1) + (size_t)s->snap.z0 * plane;
-        st = cu(cudaMemcpyAsync(sl->host + k * s->snap_floats_per_field, src, sizeof(float) * s->snap_floats_per_field,
-                                cudaMemcpyDeviceToHost, s->copy_stream));
+        st = cu(read_rows(sl->host + k * s->snap_floats_per_field, src, (size_t)s->snap.nplanes * s->ny, s->nx,
+                          s->pitch, nullptr, 0, s->copy_stream));
     }
     if (st == FDTD_OK)
         st = cu(cudaEventRecord(s->ev_copy, s->copy_stream));
@@ -352,11 +358,27 @@ int fdtd_solver_create(const fdtd_solver_config *cfg, fdtd_solver **out)
     const bool r16 = cfg->kernel == FDTD_KERNEL_COMPACT_R16;
     const int nh = cfg->kernel == FDTD_KERNEL_TWO_PASS ? 1 : 2;
     const int nd = stores_no_d(cfg->kernel) ? 1 : 2;
-    const size_t fbytes = ((n * sizeof(float)) + 255) & ~size_t(255);
-    const size_t dbytes = r16 ? ((n * sizeof(uint16_t)) + 255) & ~size_t(255) : fbytes;
-    const size_t xbytes = r16 ? ((r16_words(p->nx, p->ny, p->nz) * sizeof(uint32_t)) + 255) & ~size_t(255) : 0;
-    const size_t total = fbytes * (3 * nh + 6) + dbytes * 3 * nd + xbytes + ((n + 255) & ~size_t(255)) + 256;
-    st = cu(cudaMalloc(&s->d_block, total));
+    // Rows are padded to a multiple of 16 cells so that every solve gets TMA
+    // staging: a 217 x 253 x 181 D-form step took 382 us on dense rows (nx %
+    // 16 != 0: 4-byte cp.async) and takes 168 on padded ones, the compact form
+    // on 301 x 245 x 187 384 and 159.  A grid that only fits with dense rows
+    // keeps them.
+    size_t fbytes = 0, dbytes = 0, xbytes = 0, mbytes = 0, total = 0;
+    for (int pitch : {padded_rows_pitch(p->nx), p->nx}) {
+        const size_t m = (size_t)pitch * p->ny * p->nz;
+        s->pitch = pitch;
+        s->pcell = m;
+        s->scratch_floats = pitch == p->nx ? 0 : std::min(n, PACK_SCRATCH_FLOATS);
+        fbytes = ((m * sizeof(float)) + 255) & ~size_t(255);
+        dbytes = r16 ? ((m * sizeof(uint16_t)) + 255) & ~size_t(255) : fbytes;
+        xbytes = r16 ? ((r16_words(p->nx, p->ny, p->nz) * sizeof(uint32_t)) + 255) & ~size_t(255) : 0;
+        mbytes = (m + 255) & ~size_t(255);
+        total = fbytes * (3 * nh + 6) + dbytes * 3 * nd + xbytes + mbytes + 256;
+        st = cu(cudaMalloc(&s->d_block, total + s->scratch_floats * sizeof(float)));
+        if (st != cudaErrorMemoryAllocation || pitch == p->nx)
+            break;
+        cudaGetLastError();
+    }
     if (st == FDTD_OK) {
         char *q = s->d_block;
         for (int b = 0; b < nh; b++)
@@ -379,8 +401,10 @@ int fdtd_solver_create(const fdtd_solver_config *cfg, fdtd_solver **out)
             q += xbytes;
         }
         s->mat = reinterpret_cast<uint8_t *>(q);
-        q += (n + 255) & ~size_t(255);
+        q += mbytes;
         s->counter = reinterpret_cast<int *>(q);
+        if (s->scratch_floats > 0)
+            s->scratch = reinterpret_cast<float *>(s->d_block + total);
         st = cu(cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking));
     }
     if (st == FDTD_OK)
@@ -392,7 +416,11 @@ int fdtd_solver_create(const fdtd_solver_config *cfg, fdtd_solver **out)
     if (st == FDTD_OK)
         st = cu(cudaMemsetAsync(s->d_block, 0, total, s->stream));
     if (st == FDTD_OK)
-        st = cu(cudaMemcpyAsync(s->mat, cfg->material, n, cudaMemcpyHostToDevice, s->stream));
+        // padded rows: by way of the first H array (n bytes of its 4 pcell), cleared again
+        st = cu(write_byte_rows(s->mat, cfg->material, (size_t)p->ny * p->nz, p->nx, s->pitch,
+                                reinterpret_cast<uint8_t *>(s->h[0][0]), s->stream));
+    if (st == FDTD_OK && s->pitch != p->nx)
+        st = cu(cudaMemsetAsync(s->h[0][0], 0, n, s->stream));
     if (helper.joinable())
         helper.join();
     s->plan = plan;  // destroyed with the solver on any failure below
@@ -532,8 +560,13 @@ int fdtd_solver_get_field(fdtd_solver *s, int field, float *host_out)
     if (!src)
         return FDTD_ERR_INVALID;
     int st = fdtd_solver_synchronize(s);
+    if (st == FDTD_OK && s->pitch == s->nx)
+        return cu(cudaMemcpy(host_out, src, sizeof(float) * s->ncell, cudaMemcpyDeviceToHost));
     if (st == FDTD_OK)
-        st = cu(cudaMemcpy(host_out, src, sizeof(float) * s->ncell, cudaMemcpyDeviceToHost));
+        st = cu(read_rows(host_out, src, (size_t)s->ny * s->nz, s->nx, s->pitch, s->scratch, s->scratch_floats,
+                          s->stream));
+    if (st == FDTD_OK)
+        st = cu(cudaStreamSynchronize(s->stream));
     return st;
 }
 

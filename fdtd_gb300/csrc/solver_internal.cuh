@@ -24,7 +24,9 @@ struct SnapshotSlot {
 struct fdtd_solver {
     int device = 0;
     int nx = 0, ny = 0, nz = 0;
-    size_t ncell = 0;
+    size_t ncell = 0;           // nx * ny * nz
+    int pitch = 0;              // cells between rows of the device arrays
+    size_t pcell = 0;           // pitch * ny * nz, the length of each
     int kernel = FDTD_KERNEL_SINGLE_PASS;
     fdtd_plan *plan = nullptr;
     cudaStream_t stream = nullptr;
@@ -40,6 +42,8 @@ struct fdtd_solver {
     int memless_rows = 0;                     // tile rows and planes per chunk of those masks
     int memless_zchunk = 0;
     int *counter = nullptr;
+    float *scratch = nullptr;  // padded rows: staging of reads into pageable memory
+    size_t scratch_floats = 0;
     int steps = 0;
     std::map<std::pair<int, int>, cudaGraphExec_t> graphs;  // (parity, length) -> exec
     // snapshots
