@@ -29,6 +29,7 @@
 #include <vector>
 
 #include "native.cuh"
+#include "rows.h"
 #include "strip_unit.cuh"
 
 using namespace fdtd;
@@ -604,9 +605,13 @@ int fdtd_batch_add(fdtd_batch *b, const fdtd_solver_config *cfg, int steps, int 
         v->mat = reinterpret_cast<uint8_t *>(q);
         q += (v->ncell + 255) & ~size_t(255);
         v->counter = reinterpret_cast<int *>(q);
-        // dense host classes -> padded rows (one 2-D copy per z plane range)
-        st = cu(cudaMemcpy2DAsync(v->mat, v->pitch, cfg->material, p->nx, p->nx, (size_t)p->ny * p->nz,
-                                  cudaMemcpyHostToDevice, b->side));
+        // dense host classes -> padded rows, by way of the first H array,
+        // which is cleared again
+        const size_t n = (size_t)p->nx * p->ny * p->nz;
+        st = cu(write_byte_rows(v->mat, cfg->material, (size_t)p->ny * p->nz, p->nx, v->pitch,
+                                reinterpret_cast<uint8_t *>(v->h[0][0]), b->side));
+        if (st == FDTD_OK && v->pitch != p->nx)
+            st = cu(cudaMemsetAsync(v->h[0][0], 0, n, b->side));
     }
     if (st == FDTD_OK)
         st = cu(cudaEventCreateWithFlags(&v->ready, cudaEventDisableTiming));
@@ -809,8 +814,7 @@ int fdtd_batch_read_async(fdtd_batch *b, int id, int field, int z0, int nplanes,
         src = field < 6 ? v->d[slot][comp] : v->e[slot][comp];
     }
     src += (size_t)z0 * v->pitch * v->ny;
-    st = cu(cudaMemcpy2DAsync(host_out, sizeof(float) * v->nx, src, sizeof(float) * v->pitch, sizeof(float) * v->nx,
-                              (size_t)v->ny * nplanes, cudaMemcpyDeviceToHost, b->stream));
+    st = cu(read_rows(host_out, src, (size_t)v->ny * nplanes, v->nx, v->pitch, nullptr, 0, b->stream));
     if (st != FDTD_OK)
         return st;
     return fdtd_batch_mark(b, ticket);
@@ -914,8 +918,20 @@ int fdtd_batch_get_field(fdtd_batch *b, int id, int field, int z0, int nplanes, 
         src = field < 6 ? v->d[slot][comp] : v->e[slot][comp];
     }
     src += (size_t)z0 * v->pitch * v->ny;
-    return cu(cudaMemcpy2D(host_out, sizeof(float) * v->nx, src, sizeof(float) * v->pitch, sizeof(float) * v->nx,
-                           (size_t)v->ny * nplanes, cudaMemcpyDeviceToHost));
+    // staging for pageable memory (a strided copy where the pool has none left)
+    const size_t rows = (size_t)v->ny * nplanes;
+    const size_t floats = v->pitch == v->nx ? 0 : std::min(rows * v->nx, size_t(4) << 20);
+    void *scratch = nullptr;
+    if (floats > 0 && pool_alloc(b, &scratch, sizeof(float) * floats, b->stream) != FDTD_OK) {
+        scratch = nullptr;
+        cudaGetLastError();
+    }
+    st = cu(read_rows(host_out, src, rows, v->nx, v->pitch, static_cast<float *>(scratch), scratch ? floats : 0,
+                      b->stream));
+    if (scratch)
+        cudaFreeAsync(scratch, b->stream);
+    const int sync = cu(cudaStreamSynchronize(b->stream));
+    return st == FDTD_OK ? sync : st;
 }
 
 int fdtd_batch_tuning(const fdtd_batch *b, int *zchunk_max, int *tile_rows, int *strip_kernel)

@@ -77,6 +77,11 @@ def test_every_exit_sees_the_dense_grid(cuda, tmp_path, dims, kernel):
     sid = b.add(p, codes, specs, steps + 5, scheme=fg.SCHEME_CORRECTED)
     b.run(steps + 5)
     got = b.fields(sid)
+    name = "ey"
+    b.done(b.read_async(sid, name, pinned.view(codes.shape)), wait=True)
+    assert np.array_equal(_bits(pinned.view(codes.shape)), _bits(got[name]))
+    b.done(b.read_async(sid, name, pinned.view((1, ny, nx)), z0=nz // 2, nplanes=1), wait=True)
+    assert np.array_equal(_bits(pinned.view((1, ny, nx))[0]), _bits(got[name][nz // 2]))
     b.close()
     assert all(np.array_equal(_bits(got[k]), _bits(v)) for k, v in after.items())
 
