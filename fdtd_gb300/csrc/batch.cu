@@ -6,9 +6,8 @@
 // rows padded to a multiple of 16 cells, so every solve gets TMA staging, and
 // its own plan (class table, source table, Mur slabs) and step counter.  A
 // batched step is three launches: one kernel over the work units (column
-// tile x z chunk) of all solves (compact forms: one CTA per unit; D form: a
-// persistent kernel taking units from a counter), one Mur launch over all solves' face
-// cells, and a one-block kernel that advances the step counters.  Step n of a
+// tile x z chunk) of all solves, one CTA per unit, one Mur launch over all
+// solves' face cells, and a one-block kernel that advances the step counters.  Step n of a
 // solve uses its counter's parity to pick pointers and tensor maps, so one
 // captured graph serves every step; a solve stops once it reaches its target
 // step count.  Adding or removing a solve rebuilds the descriptors and the
@@ -120,7 +119,7 @@ struct fdtd_batch {
     int zchunk_max = 0;  // largest z chunk (fdtd_batch_autotune); 0: the form's default
     int strip_shape = 0;  // compact forms: strip kernel shape, -1 the z-marching kernel (fdtd_batch_autotune)
     bool strip = false;   // the current launch runs the strip kernel
-    BatchUnit *d_units = nullptr;  // strip kernel: per unit its solve and memoryless planes
+    BatchUnit *d_units = nullptr;  // per unit its solve, tile and memoryless planes
     size_t units_cap = 0;
 };
 
@@ -267,6 +266,25 @@ int rebuild(fdtd_batch *b)
             strip = strip_usable(c, b->r16);
         }
     const int ty = strip ? strip_shape_rows(b->strip_shape) : fused_tile_height();
+    int max_classes = 1;
+    for (auto *v : b->solves)
+        max_classes = std::max(max_classes, v->plan->nclasses);
+    const int ctas = strip ? batch_strip_ctas(b->r16, b->strip_shape, max_classes)
+                           : batch_fused_ctas(b->compact, max_classes, b->r16);
+    if (ctas < 1)
+        return FDTD_ERR_INVALID;
+    // z chunks: the autotuner's limit, else the form's, shorter where its
+    // units would leave the device idle
+    int zmax = b->zchunk_max;
+    if (zmax <= 0) {
+        zmax = strip ? strip_zchunk_max() : (b->compact ? compact_zchunk_max() : fused_zchunk_max());
+        if (!(strip && strip_zchunk_fixed())) {
+            std::vector<std::array<int, 2>> grids;
+            for (auto *v : b->solves)
+                grids.push_back({((v->nx + 31) / 32) * ((v->ny + ty - 1) / ty), v->nz});
+            zmax = balanced_batch_limit(grids, zmax, ctas, strip ? 0.5 : 1.25);
+        }
+    }
     for (size_t i = 0; i < b->solves.size(); i++) {
         BatchSolve *v = b->solves[i];
         BatchDesc &d = descs[i];
@@ -278,9 +296,7 @@ int rebuild(fdtd_batch *b)
                       : !encode_step_maps(d.c[par], b->compact, &d.maps[par], b->r16))
                 return FDTD_ERR_INVALID;
         }
-        d.zchunk = b->zchunk_max > 0 ? zchunk_limited(v->nz, b->zchunk_max)
-                                     : (strip ? strip_zchunk(v->nz)
-                                              : (b->compact ? compact_zchunk(v->nz) : fused_zchunk(v->nz)));
+        d.zchunk = zchunk_limited(v->nz, zmax);
         d.tiles_x = (v->nx + 31) / 32;
         d.tiles_y = (v->ny + ty - 1) / ty;
         d.chunks = (v->nz + d.zchunk - 1) / d.zchunk;
@@ -329,34 +345,32 @@ int rebuild(fdtd_batch *b)
         st = pool_alloc(b, reinterpret_cast<void **>(&b->d_mur), sizeof(BatchMurBlock) * cap, b->stream);
         b->mur_cap = st == FDTD_OK ? cap : 0;
     }
-    // strip kernel: per unit its tile, z chunk, solve and the planes whose
-    // tile holds no Debye memory
-    std::vector<BatchUnit> recs;
-    if (strip) {
-        std::vector<unsigned long long> masks((size_t)units, 0ull);
-        recs.resize((size_t)units);
-        for (size_t i = 0; i < b->solves.size(); i++) {
-            const BatchSolve *v = b->solves[i];
-            const BatchDesc &d = descs[i];
-            if (d.tiles_x > 65535 || d.tiles_y > 65535 || d.chunks > 65535 || d.zchunk > 65535)
-                return FDTD_ERR_INVALID;
+    // per unit its tile, z chunk and solve (strip kernel: and the planes
+    // whose tile holds no Debye memory)
+    std::vector<unsigned long long> masks((size_t)units, 0ull);
+    std::vector<BatchUnit> recs((size_t)units);
+    for (size_t i = 0; i < b->solves.size(); i++) {
+        const BatchSolve *v = b->solves[i];
+        const BatchDesc &d = descs[i];
+        if (strip && (d.tiles_x > 65535 || d.tiles_y > 65535 || d.chunks > 65535 || d.zchunk > 65535))
+            return FDTD_ERR_INVALID;
+        if (strip)
             strip_unit_masks(v->memless8, v->nx, v->ny, v->nz, ty, d.zchunk, masks.data() + d.unit_begin);
-            for (int j = 0; j < d.unit_count; j++) {
-                const int per_z = d.tiles_x * d.tiles_y, rem = j % per_z;
-                recs[(size_t)d.unit_begin + j] =
-                    BatchUnit{masks[(size_t)d.unit_begin + j], v->counter,           (int)i,
-                              (unsigned short)(rem % d.tiles_x), (unsigned short)(rem / d.tiles_x),
-                              (unsigned short)(j / per_z),       (unsigned short)d.zchunk, d.steps_target};
-            }
+        for (int j = 0; j < d.unit_count; j++) {
+            const int per_z = d.tiles_x * d.tiles_y, rem = j % per_z;
+            recs[(size_t)d.unit_begin + j] =
+                BatchUnit{masks[(size_t)d.unit_begin + j], v->counter,           (int)i,
+                          (unsigned short)(rem % d.tiles_x), (unsigned short)(rem / d.tiles_x),
+                          (unsigned short)(j / per_z),       (unsigned short)d.zchunk, d.steps_target};
         }
-        if (st == FDTD_OK && recs.size() > b->units_cap) {
-            if (b->d_units)
-                cudaFreeAsync(b->d_units, b->stream);
-            b->d_units = nullptr;
-            const size_t cap = std::max(recs.size() * 2, size_t(1024));
-            st = pool_alloc(b, reinterpret_cast<void **>(&b->d_units), sizeof(BatchUnit) * cap, b->stream);
-            b->units_cap = st == FDTD_OK ? cap : 0;
-        }
+    }
+    if (st == FDTD_OK && recs.size() > b->units_cap) {
+        if (b->d_units)
+            cudaFreeAsync(b->d_units, b->stream);
+        b->d_units = nullptr;
+        const size_t cap = std::max(recs.size() * 2, size_t(1024));
+        st = pool_alloc(b, reinterpret_cast<void **>(&b->d_units), sizeof(BatchUnit) * cap, b->stream);
+        b->units_cap = st == FDTD_OK ? cap : 0;
     }
     if (st == FDTD_OK)
         st = staged_upload(b, {Upload{b->d_descs, descs.data(), sizeof(BatchDesc) * descs.size()},
@@ -364,16 +378,8 @@ int rebuild(fdtd_batch *b)
                                Upload{b->d_units, recs.data(), sizeof(BatchUnit) * recs.size()}});
     if (st != FDTD_OK)
         return st;
-    int max_classes = 1;
-    for (auto *v : b->solves)
-        max_classes = std::max(max_classes, v->plan->nclasses);
-    const int ctas = strip ? batch_strip_ctas(b->r16, b->strip_shape, max_classes)
-                           : batch_persistent_ctas(b->compact, max_classes, b->r16);
-    if (ctas < 1)
-        return FDTD_ERR_INVALID;
-    b->launch = BatchLaunch{b->d_descs, (int)descs.size(), units, b->d_work, b->d_mur, (int)mur.size(), ctas,
-                            b->compact ? 1 : 0, max_classes, b->r16 ? 1 : 0, strip ? 1 : 0, b->strip_shape,
-                            strip ? b->d_units : nullptr};
+    b->launch = BatchLaunch{b->d_descs, (int)descs.size(), units, b->d_mur, (int)mur.size(), b->compact ? 1 : 0,
+                            max_classes, b->r16 ? 1 : 0, strip ? 1 : 0, b->strip_shape, b->d_units};
     b->strip = strip;
     drop_graphs(b);
     b->dirty = false;

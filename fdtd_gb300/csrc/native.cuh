@@ -3,6 +3,7 @@
 
 #include <cuda.h>
 
+#include <array>
 #include <vector>
 
 #include "device_common.cuh"
@@ -178,7 +179,8 @@ struct alignas(64) BatchDesc {
     int pad;
 };
 
-// One work unit of the batched strip kernel, found by its index: the planes
+// One work unit of a batched kernel, found by its index (the z-marching
+// kernel works out the tile and chunk from the index itself): the planes
 // of its tile that hold no Debye memory (bit j: plane zc0 + j), its solve's
 // step counter and step target, the solve, the tile (bx, by), the z chunk bz
 // and the chunk length.
@@ -205,35 +207,39 @@ struct BatchLaunch {
     const BatchDesc *descs;
     int nsolves;
     int total_units;
-    int *work_counter;
     const BatchMurBlock *mur_blocks;
     int nmur_blocks;
-    int persistent_ctas;
     int compact;      // the batch's solves keep the compact state (d_cur == d_prev == R)
     int max_classes;  // largest class count of the batch's solves (shared-memory table)
     int r16;          // the compact state holds R in 16 bits (compact is set too)
     int strip;        // compact forms: run by the strip kernel of shape strip_shape
     int strip_shape;
-    const BatchUnit *units;  // strip kernel: one record per unit
+    const BatchUnit *units;  // one record per unit
 };
 
 // Tensor maps of a single-pass launch over c's buffers (false: not encodable).
 bool encode_fused_maps(const NativeConsts &c, FusedMaps *maps);
 bool encode_step_maps(const NativeConsts &c, bool compact, FusedMaps *maps, bool r16 = false);
 int fused_tile_height();
-int fused_zchunk(int nz);
-int compact_zchunk(int nz);
 int zchunk_limited(int nz, int max_planes);  // nz in equal chunks of at most max_planes planes
 // z chunk of one solve's launch: equal chunks of at most max_planes planes,
 // shorter ones where columns (column tiles) x chunks would leave the device's
 // `resident` CTAs idle in the first wave or nearly empty in the last; start:
 // what a CTA costs before its first plane, in planes.
 int balanced_zchunk(int nz, int max_planes, long long columns, int resident, double start);
+// z chunk limit of a batch's default launch, for its solves' (column tiles,
+// planes): the form's limit, or a shorter one where that leaves the device idle.
+int balanced_batch_limit(const std::vector<std::array<int, 2>> &grids, int max_planes, int resident, double start);
+int fused_zchunk_max();
+int compact_zchunk_max();
+int strip_zchunk_max();
+bool strip_zchunk_fixed();  // set in the environment: not balanced
 // One batched step: fused kernel over all units, Mur faces, step counters.
 int launch_batch_step(const BatchLaunch &b, cudaStream_t s);
-int batch_persistent_ctas(bool compact, int nclasses, bool r16 = false);
-// The batch's persistent strip kernel (batch_strip.cu): its launch and the
-// CTAs that fill the device at the given shape and class count.
+// CTAs of the batched z-marching kernel that the device holds at once.
+int batch_fused_ctas(bool compact, int nclasses, bool r16);
+// The batch's strip kernel (batch_strip.cu): its launch and the CTAs that
+// the device holds at once at the given shape and class count.
 int launch_batch_strip(const BatchLaunch &b, cudaStream_t s);
 int batch_strip_ctas(bool r16, int shape, int nclasses);
 

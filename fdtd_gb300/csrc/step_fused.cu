@@ -663,73 +663,43 @@ __global__ void __launch_bounds__(FTX *TY) fused_step_kernel(const __grid_consta
                                          stall);
 }
 
-// Many solves: persistent CTAs take work units from a counter; a unit's solve
-// descriptor supplies the constants (copied to shared memory) and tensor maps
-// (read by TMA from device memory).  Units of finished solves are skipped.
-// The compact forms are bounded for 4 resident CTAs per SM (the 64-solve
-// workload ran 4.8 % faster than with 5: fewer units in flight, more
-// registers per thread; with 16-bit R 11 % faster than with 3 or 5).
+// Many solves: one CTA per work unit (the grid is the batch's work list); the
+// unit's record names its solve, whose descriptor supplies the constants
+// (copied to shared memory) and tensor maps (read by TMA from device memory).
+// Units of finished solves exit at once.  A persistent form, CTAs taking
+// units from an atomic counter, ran as fast (D form, 20 solves of 24-128 cells
+// per axis 152 us per step against 150, 48-256 668 against 668) with more code.
+// The compact forms are bounded for 4 resident CTAs per SM (measured in the
+// persistent form: the 64-solve workload ran 4.8 % faster than with 5; with
+// 16-bit R 11 % faster than with 3 or 5).
 template <int TY, int S, bool COMPACT, bool R16 = false>
-__global__ void __launch_bounds__(FTX *TY, COMPACT ? 4 : 3) batch_step_kernel(const BatchDesc *__restrict__ descs, int nsolves,
-                                                             int total_units, int *work_counter)
+__global__ void __launch_bounds__(FTX *TY, COMPACT ? 4 : 3) batch_step_kernel(const BatchDesc *__restrict__ descs,
+                                                                             const BatchUnit *__restrict__ units)
 {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     unsigned char *smem = smem_raw + ((128 - (smem_addr(smem_raw) & 127)) & 127);
     __shared__ NativeConsts s_c;
-    __shared__ int s_unit, s_solve;
+    const BatchUnit rec = units[blockIdx.x];
+    const int n = *rec.counter;
+    if (n >= rec.steps_target)  // the solve is done (uniform over the CTA)
+        return;
     DebyeCoef *coef;
     uint64_t *bars;
     fused_cta_setup<S, true, GeoOf<TY, COMPACT, R16>>(smem, &coef, &bars);
     const int tid = threadIdx.y * FTX + threadIdx.x;
-    int loaded = -1;
-    unsigned g = 0;
-    __syncthreads();
-    for (;;) {
-        if (tid == 0) {
-            const int u = atomicAdd(work_counter, 1);
-            int lo = 0, hi = nsolves - 1;
-            if (u < total_units) {
-                while (lo < hi) {  // last solve with unit_begin <= u
-                    const int mid = (lo + hi + 1) >> 1;
-                    if (descs[mid].unit_begin <= u)
-                        lo = mid;
-                    else
-                        hi = mid - 1;
-                }
-            }
-            s_unit = u;
-            s_solve = lo;
-        }
-        __syncthreads();
-        const int u = s_unit, sv = s_solve;
-        if (u >= total_units)
-            break;
-        const BatchDesc &d = descs[sv];
-        const int n = *d.c[0].step_counter;
-        if (n < d.steps_target) {
-            const int par = n & 1;
-            {
-                const int *src = reinterpret_cast<const int *>(&d.c[par]);
-                int *dst = reinterpret_cast<int *>(&s_c);
-                for (int i = tid; i < (int)(sizeof(NativeConsts) / 4); i += FTX * TY)
-                    dst[i] = src[i];
-            }
-            if (sv != loaded)
-                load_coef(d.c[par], coef, FTX * TY);
-            __syncthreads();
-            loaded = sv;
-            const int local = u - d.unit_begin;
-            const int per_z = d.tiles_x * d.tiles_y;
-            const int bz = local / per_z, rem = local % per_z;
-            const int by = rem / d.tiles_x, bx = rem % d.tiles_x;
-            const int zc0 = bz * d.zchunk, zc1 = min(s_c.nz, zc0 + d.zchunk);
-            const int nplanes = min(zc1, s_c.nz - 1) - max(zc0 - 1, 0) + 1;
-            if (!fused_unit<TY, S, true, COMPACT, R16>(s_c, d.maps[par], d.zchunk, bx, by, bz, smem, coef, bars, g))
-                return;
-            g += (unsigned)nplanes;
-        }
-        __syncthreads();
+    const BatchDesc &d = descs[rec.solve];
+    const int par = n & 1;
+    {
+        const int *src = reinterpret_cast<const int *>(&d.c[par]);
+        int *dst = reinterpret_cast<int *>(&s_c);
+        for (int i = tid; i < (int)(sizeof(NativeConsts) / 4); i += FTX * TY)
+            dst[i] = src[i];
     }
+    load_coef(d.c[par], coef, FTX * TY);
+    __syncthreads();
+    const int local = (int)blockIdx.x - d.unit_begin, per_z = d.tiles_x * d.tiles_y, rem = local % per_z;
+    fused_unit<TY, S, true, COMPACT, R16>(s_c, d.maps[par], d.zchunk, rem % d.tiles_x, rem / d.tiles_x, local / per_z,
+                                          smem, coef, bars, 0u);
 }
 
 __global__ void __launch_bounds__(256) batch_mur_kernel(const BatchDesc *__restrict__ descs,
@@ -759,11 +729,9 @@ __global__ void __launch_bounds__(256) batch_mur_kernel(const BatchDesc *__restr
                                             c.scheme == FDTD_SCHEME_CORRECTED, (unsigned)b.limit);
 }
 
-__global__ void batch_advance_kernel(const BatchDesc *__restrict__ descs, int nsolves, int *work_counter)
+__global__ void batch_advance_kernel(const BatchDesc *__restrict__ descs, int nsolves)
 {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s == 0)
-        *work_counter = 0;
     if (s < nsolves) {
         int *ctr = descs[s].c[0].step_counter;
         if (*ctr < descs[s].steps_target)
@@ -874,20 +842,52 @@ int balanced_zchunk(int nz, int max_planes, long long columns, int resident, dou
     return best;
 }
 
+// The same for a batch, whose units differ in length: the limit that
+// minimises the CTAs' planes over the device plus half of the longest CTA
+// (the last ones to finish run alone), never less than the longest CTA.
+// us per step with the form's limit and with this choice: D form, 20 solves
+// of 24-128 cells per axis 194 and 150, 3 solves of 32-64 128 and 23, one of
+// 204 x 145 x 208 192 and 140; compact form 119 and 112, 16-bit R 128 and
+// 122, its 3 small solves 49 and 25.  Limits below 8 were no better there (24,
+// 154): those steps are bound by their three launches.
+int balanced_batch_limit(const std::vector<std::array<int, 2>> &grids, int max_planes, int resident, double start)
+{
+    const int limits[] = {max_planes, 48, 32, 24, 16, 8};
+    int best = max_planes;
+    double best_cost = -1.0;
+    for (int limit : limits) {
+        if (limit > max_planes)
+            continue;
+        double planes = 0.0, longest = 0.0;
+        long long ctas = 0;
+        for (const auto &g : grids) {  // column tiles, planes
+            const int c = zchunk_limited(g[1], limit);
+            const long long n = (long long)g[0] * ((g[1] + c - 1) / c);
+            ctas += n;
+            planes += (double)n * (c + start);
+            longest = std::max(longest, c + start);
+        }
+        if (resident < 1 || (best_cost < 0.0 && ctas > 6LL * resident))
+            return max_planes;
+        const double cost = std::max(planes / resident + 0.5 * longest, longest);
+        if (best_cost < 0.0 || cost < best_cost) {
+            best = limit;
+            best_cost = cost;
+        }
+    }
+    return best;
+}
+
 #ifndef FDTD_ZCHUNK
 #define FDTD_ZCHUNK 64
 #endif
 static_assert(FDTD_ZCHUNK >= 4 && FDTD_ZCHUNK <= 64, "a unit's per-thread source mask covers 66 planes");
 
-int fused_zchunk(int nz)
-{
-    // about 64 planes per CTA: enough CTAs per wave on 152 SMs, little
-    // prologue/epilogue traffic at chunk borders.  At most 64: a unit's
-    // per-thread source mask covers 66 planes.
-    return zchunk_limited(nz, FDTD_ZCHUNK);
-}
-
-int compact_zchunk(int nz) { return zchunk_limited(nz, FDTD_COMPACT_ZCHUNK); }
+// Largest z chunks of the D form (about 64 planes per CTA: little prologue and
+// epilogue traffic at chunk borders; at most 64, as a unit's per-thread source
+// mask covers 66 planes) and of the compact form.
+int fused_zchunk_max() { return FDTD_ZCHUNK; }
+int compact_zchunk_max() { return FDTD_COMPACT_ZCHUNK; }
 
 bool fused_uses_tma(const NativeConsts &c)
 {
@@ -939,81 +939,60 @@ bool encode_fused_maps(const NativeConsts &c, FusedMaps *maps) { return encode_s
 
 int fused_tile_height() { return TY_SEL; }
 
-// Shared memory of the persistent batch kernel: tiles of the form and a class
-// table for the batch's largest class count.
+// The batch kernel of a form: tiles of the form and a class table for the
+// batch's largest class count in shared memory, whose opt-in holds for the
+// current device only and is made on the first use there.
 template <bool COMPACT, bool R16 = false>
-int batch_smem(int nclasses) { return fused_smem_bytes<S_SEL, GeoOf<TY_SEL, COMPACT, R16>>(nclasses); }
+struct BatchStep {
+    static constexpr auto fn = batch_step_kernel<TY_SEL, S_SEL, COMPACT, R16>;
+    static int smem(int nclasses) { return fused_smem_bytes<S_SEL, GeoOf<TY_SEL, COMPACT, R16>>(nclasses); }
+    static int opt_in()
+    {
+        static PerDeviceOnce<> once;
+        int dev = 0;
+        const cudaError_t e = cudaGetDevice(&dev);
+        if (e != cudaSuccess)
+            return (int)e;
+        const int so = once.run(dev, [] {
+            return (int)cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem(FDTD_MAX_CLASSES));
+        });
+        return so < 0 ? FDTD_ERR_INVALID : so;
+    }
+    static int ctas(int nclasses) { return opt_in() == FDTD_OK ? resident_ctas(fn, FTX * TY_SEL, smem(nclasses)) : 0; }
+    static int launch(const BatchLaunch &b, cudaStream_t s)
+    {
+        const int st = opt_in();
+        if (st != FDTD_OK)
+            return st;
+        fn<<<b.total_units, dim3(FTX, TY_SEL), smem(b.max_classes), s>>>(b.descs, b.units);
+        const cudaError_t e = cudaGetLastError();
+        return e == cudaSuccess ? FDTD_OK : (int)e;
+    }
+};
 
-// The batch kernel's shared-memory opt-in on the current device (it holds
-// for that device only): made on the first use there.
-template <bool COMPACT, bool R16 = false>
-int batch_opt_in()
+int batch_fused_ctas(bool compact, int nclasses, bool r16)
 {
-    auto kernel = batch_step_kernel<TY_SEL, S_SEL, COMPACT, R16>;
-    static PerDeviceOnce<> smem_opt_in;
-    int dev = 0;
-    const cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess)
-        return (int)e;
-    const int so = smem_opt_in.run(dev, [&] {
-        return (int)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         batch_smem<COMPACT, R16>(FDTD_MAX_CLASSES));
-    });
-    return so < 0 ? FDTD_ERR_INVALID : so;
-}
-
-template <bool COMPACT, bool R16 = false>
-int batch_ctas_impl(int nclasses)
-{
-    auto kernel = batch_step_kernel<TY_SEL, S_SEL, COMPACT, R16>;
-    batch_opt_in<COMPACT, R16>();
-    int dev = 0, sms = 0, per_sm = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, FTX * TY_SEL, batch_smem<COMPACT, R16>(nclasses));
-    return sms * (per_sm > 0 ? per_sm : 1);
-}
-
-int batch_persistent_ctas(bool compact, int nclasses, bool r16)
-{
-    if (r16)
-        return batch_ctas_impl<true, true>(nclasses);
-    return compact ? batch_ctas_impl<true>(nclasses) : batch_ctas_impl<false>(nclasses);
+    return r16 ? BatchStep<true, true>::ctas(nclasses)
+               : (compact ? BatchStep<true>::ctas(nclasses) : BatchStep<false>::ctas(nclasses));
 }
 
 int launch_batch_step(const BatchLaunch &b, cudaStream_t s)
 {
     if (b.max_classes < 1 || b.max_classes > FDTD_MAX_CLASSES)
         return FDTD_ERR_INVALID;
+    const int st = b.strip     ? launch_batch_strip(b, s)
+                   : b.r16     ? BatchStep<true, true>::launch(b, s)
+                   : b.compact ? BatchStep<true>::launch(b, s)
+                               : BatchStep<false>::launch(b, s);
+    if (st != FDTD_OK)
+        return st;
     cudaError_t e = cudaSuccess;
-    if (b.strip) {
-        const int st = launch_batch_strip(b, s);
-        if (st != FDTD_OK)
-            return st;
-    } else {
-    const int oi = b.r16 ? batch_opt_in<true, true>() : (b.compact ? batch_opt_in<true>() : batch_opt_in<false>());
-    if (oi != FDTD_OK)
-        return oi;
-    if (b.r16)
-        batch_step_kernel<TY_SEL, S_SEL, true, true>
-            <<<b.persistent_ctas, dim3(FTX, TY_SEL), batch_smem<true, true>(b.max_classes), s>>>(
-                b.descs, b.nsolves, b.total_units, b.work_counter);
-    else if (b.compact)
-        batch_step_kernel<TY_SEL, S_SEL, true>
-            <<<b.persistent_ctas, dim3(FTX, TY_SEL), batch_smem<true>(b.max_classes), s>>>(
-                b.descs, b.nsolves, b.total_units, b.work_counter);
-    else
-        batch_step_kernel<TY_SEL, S_SEL, false>
-            <<<b.persistent_ctas, dim3(FTX, TY_SEL), batch_smem<false>(b.max_classes), s>>>(
-                b.descs, b.nsolves, b.total_units, b.work_counter);
-    e = cudaGetLastError();
-    }
-    if (e == cudaSuccess && b.nmur_blocks > 0) {
+    if (b.nmur_blocks > 0) {
         batch_mur_kernel<<<b.nmur_blocks, 256, 0, s>>>(b.descs, b.mur_blocks);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) {
-        batch_advance_kernel<<<(b.nsolves + 255) / 256, 256, 0, s>>>(b.descs, b.nsolves, b.work_counter);
+        batch_advance_kernel<<<(b.nsolves + 255) / 256, 256, 0, s>>>(b.descs, b.nsolves);
         e = cudaGetLastError();
     }
     return e == cudaSuccess ? FDTD_OK : (int)e;

@@ -10,8 +10,6 @@
 
 namespace fdtd {
 
-int strip_zchunk(int nz);
-
 namespace strip {
 namespace {
 
@@ -88,7 +86,7 @@ int solve_zchunk(int nx, int ny, int nz, int nclasses)
     constexpr int RY = Shape<SHAPE>::RY, W = Shape<SHAPE>::W;
     using G = StripGeo<RY, W, R16>;
     int dev = 0;
-    if (std::getenv("FDTD_STRIP_ZCHUNK") || nclasses < 1 || nclasses > FDTD_MAX_CLASSES ||
+    if (strip_zchunk_fixed() || nclasses < 1 || nclasses > FDTD_MAX_CLASSES ||
         cudaGetDevice(&dev) != cudaSuccess || opt_in<SHAPE, R16>() != 0)
         return strip_zchunk(nz);
     static PerDeviceValue<FDTD_MAX_CLASSES + 1> resident;
@@ -216,18 +214,23 @@ int strip_solve_zchunk(int nx, int ny, int nz, bool r16, int nclasses)
     }
 }
 
-int strip_zchunk(int nz)
+// The z chunk limit of the default launches: FDTD_STRIP_ZCHUNK in the
+// environment (2-64 planes) overrides the build's; read wherever the launch
+// and the masks are made.
+int strip_zchunk_max()
 {
-    // FDTD_STRIP_ZCHUNK in the environment (2-64 planes) overrides the
-    // build's limit; read wherever the launch and the masks are made
     int limit = FDTD_STRIP_ZCHUNK;
     if (const char *v = std::getenv("FDTD_STRIP_ZCHUNK")) {
         const int n = std::atoi(v);
         if (n >= 2 && n <= 64)
             limit = n;
     }
-    return zchunk_limited(nz, limit);
+    return limit;
 }
+
+bool strip_zchunk_fixed() { return std::getenv("FDTD_STRIP_ZCHUNK") != nullptr; }
+
+int strip_zchunk(int nz) { return zchunk_limited(nz, strip_zchunk_max()); }
 
 std::vector<unsigned char> strip_plane_flags(const uint8_t *mat, int nx, int ny, int nz, int pitch, const float *specs,
                                              int nclasses)
