@@ -243,6 +243,11 @@ def serve(requests: list[Request], budget_bytes: int, chunk: int = 25, snapshot_
 
     try:
         while pending or queue or active or chunks or snaps or finishing:
+            # keep at most `inflight` chunks queued: wait for the oldest before
+            # looking for arrivals, so that a request that arrives meanwhile
+            # joins the next chunk
+            while active and len(chunks) >= inflight:
+                batch.done(chunks.popleft(), wait=True)
             now = clock() - t0
             while pending and pending[0].arrival <= now:
                 queue.append(pending.popleft())
@@ -289,8 +294,7 @@ def serve(requests: list[Request], budget_bytes: int, chunk: int = 25, snapshot_
                 active_cells += cells
                 admitted += 1
             if active:
-                # keep at most `inflight` chunks queued: wait for the oldest
-                while len(chunks) >= inflight:
+                while len(chunks) >= inflight:  # of solves that ended since
                     batch.done(chunks.popleft(), wait=True)
                 batch.run(chunk)
                 finished = []
