@@ -282,7 +282,7 @@ int rebuild(fdtd_batch *b)
             std::vector<std::array<int, 2>> grids;
             for (auto *v : b->solves)
                 grids.push_back({((v->nx + 31) / 32) * ((v->ny + ty - 1) / ty), v->nz});
-            zmax = balanced_batch_limit(grids, zmax, ctas, strip ? 0.5 : 1.25);
+            zmax = balanced_batch_limit(grids, zmax, ctas);
         }
     }
     for (size_t i = 0; i < b->solves.size(); i++) {

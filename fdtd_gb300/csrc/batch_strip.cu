@@ -20,10 +20,9 @@ namespace {
 // hardware in unit order like the single-solve kernel's grid): the unit's
 // record, its solve's constants in shared memory, then the unit.
 template <int RY, int W, int S, bool R16, int MINB>
-__global__ void __launch_bounds__(32 * W, MINB) batch_strip_kernel(const BatchDesc *__restrict__ descs,
+__global__ void __launch_bounds__(32 * W + 32, MINB) batch_strip_kernel(const BatchDesc *__restrict__ descs,
                                                                   const BatchUnit *__restrict__ units)
 {
-    using G = StripGeo<RY, W, R16>;
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ StripConsts s_c;
     const StripSmem sm = strip_smem<RY, W, S, R16>(smem_raw);
@@ -31,16 +30,14 @@ __global__ void __launch_bounds__(32 * W, MINB) batch_strip_kernel(const BatchDe
     const int n = *rec.counter;
     if (n >= rec.steps_target)  // the solve is done (uniform over the CTA)
         return;
-    strip_init_bars<S>(sm);
+    strip_init_bars<W, S>(sm);
     const BatchDesc &d = descs[rec.solve];
     const int par = n & 1;
     if (threadIdx.x == 0)
         strip_consts(s_c, d.c[par]);
-    strip_load_coef(d.c[par], sm.coef, G::NTH);
+    strip_load_coef(d.c[par], sm.coef, 32 * W + 32);
     __syncthreads();
-    strip_unit<RY, W, S, R16>(s_c, d.smaps[par], rec.zchunk, rec.bx, rec.by, rec.bz, rec.memless, sm, 0u, false);
-    if (threadIdx.x == G::STORE_TID)
-        bulk_wait_all();
+    strip_unit<RY, W, S, R16>(s_c, d.smaps[par], rec.zchunk, rec.bx, rec.by, rec.bz, rec.memless, sm, false);
 }
 
 template <int SHAPE, bool R16>
@@ -69,7 +66,7 @@ struct BatchKernel {
         int dev = 0, sms = 0, per_sm = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, 32 * W, smem(nclasses));
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, 32 * W + 32, smem(nclasses));
         return sms * (per_sm > 0 ? per_sm : 1);
     }
     static int launch(const BatchLaunch &b, cudaStream_t s)
@@ -77,7 +74,7 @@ struct BatchKernel {
         const int st = opt_in();
         if (st != FDTD_OK)
             return st;
-        fn<<<b.total_units, 32 * W, smem(b.max_classes), s>>>(b.descs, b.units);
+        fn<<<b.total_units, 32 * W + 32, smem(b.max_classes), s>>>(b.descs, b.units);
         const cudaError_t e = cudaGetLastError();
         return e == cudaSuccess ? FDTD_OK : (int)e;
     }

@@ -224,12 +224,11 @@ int fused_tile_height();
 int zchunk_limited(int nz, int max_planes);  // nz in equal chunks of at most max_planes planes
 // z chunk of one solve's launch: equal chunks of at most max_planes planes,
 // shorter ones where columns (column tiles) x chunks would leave the device's
-// `resident` CTAs idle in the first wave or nearly empty in the last; start:
-// what a CTA costs before its first plane, in planes.
-int balanced_zchunk(int nz, int max_planes, long long columns, int resident, double start);
+// `resident` CTAs idle in the first wave or nearly empty in the last.
+int balanced_zchunk(int nz, int max_planes, long long columns, int resident);
 // z chunk limit of a batch's default launch, for its solves' (column tiles,
 // planes): the form's limit, or a shorter one where that leaves the device idle.
-int balanced_batch_limit(const std::vector<std::array<int, 2>> &grids, int max_planes, int resident, double start);
+int balanced_batch_limit(const std::vector<std::array<int, 2>> &grids, int max_planes, int resident);
 int fused_zchunk_max();
 int compact_zchunk_max();
 int strip_zchunk_max();

@@ -783,7 +783,7 @@ int launch_fused_impl(FusedArgs &a, int zmax, const FusedMaps &maps, cudaStream_
     static PerDeviceValue<FDTD_MAX_CLASSES + 1> resident;
     const int r = resident.get(dev, a.c.nclasses, [&] { return resident_ctas(kernel, FTX * TY_SEL, smem); });
     const int tiles_x = (a.c.nx + FTX - 1) / FTX, tiles_y = (a.c.ny + TY_SEL - 1) / TY_SEL;
-    a.zchunk = balanced_zchunk(a.c.nz, zmax, (long long)tiles_x * tiles_y, r, 1.25);
+    a.zchunk = balanced_zchunk(a.c.nz, zmax, (long long)tiles_x * tiles_y, r);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(tiles_x, tiles_y, (a.c.nz + a.zchunk - 1) / a.zchunk);
     cfg.blockDim = dim3(FTX, TY_SEL);
@@ -807,23 +807,27 @@ int zchunk_limited(int nz, int max_planes)
     return (nz + chunks - 1) / chunks;
 }
 
-// The default chunk serves grids of many waves of CTAs.  Small and middle
+// The longest chunk serves grids of many waves of CTAs.  Small and middle
 // grids are chunked by whole waves: a grid of 64^3 in 64-plane chunks has 16
 // CTAs for 152 SMs and takes as long as one CTA needs for 66 planes.  With W
-// = ceil(CTAs / resident) waves, W (chunk + start) orders the measured step
-// times of ten grids from 64^3 to 512 x 512 x 400 to within 4 % of the best
-// of 13 chunk lengths (D form, us per step, 64-plane chunks against this
-// choice: 64^3 85.6 -> 10.2, 128^3 109.6 -> 41.0, 224 x 208 x 176 188 -> 138,
-// 256 x 239 x 160 186 -> 165; the compact strip kernel, 24-plane chunks:
-// 64^3 44.0 -> 10.3, 128^3 53.9 -> 34.1, 256 x 239 x 160 128.9 -> 118.6).
-// Beyond six waves the CTAs have drifted apart, no wave ends as one, and the
-// default chunk is as good or better (512 x 512 x 400: 1568 us with 58
+// = ceil(CTAs / resident) waves, W (chunk + 1.5) picks, among the chunk lengths
+// measured on twelve grids from 64^3 to 1024 x 1024 x 128, one within 4 % of the
+// fastest in the D form, 2 % in the compact form (16-bit R: 4 %, but for one grid
+// of 1.03 waves that runs as one: 12 %).  us per step in 64-plane chunks (strip
+// kernel: 24) and as chosen: D form 64^3 85.6 and 10.2, 128^3 109.6 and 41.0,
+// 224 x 208 x 176 188 and 138, 256 x 239 x 160 186 and 165; compact form 64^3
+// 34.2 and 9.5, 128^3 47.9 and 31.8, 256 x 239 x 160 121.5 and 106.
+// Beyond eight waves the CTAs have drifted apart, no wave ends as one, and the
+// longest chunk is as good or better (D form, 512 x 512 x 400: 1568 us with 58
 // planes, 1579 with 24).
-int balanced_zchunk(int nz, int max_planes, long long columns, int resident, double start)
+constexpr double CTA_START = 1.5;   // what a CTA costs before its first plane, in planes
+constexpr long long MOST_WAVES = 8;
+
+int balanced_zchunk(int nz, int max_planes, long long columns, int resident)
 {
     const int longest = zchunk_limited(nz, max_planes);
     auto chunks_of = [&](int c) { return (long long)((nz + c - 1) / c); };
-    if (resident < 1 || columns * chunks_of(longest) > 6LL * resident)
+    if (resident < 1 || columns * chunks_of(longest) > MOST_WAVES * resident)
         return longest;
     int best = longest;
     double best_cost = 0.0;
@@ -831,9 +835,9 @@ int balanced_zchunk(int nz, int max_planes, long long columns, int resident, dou
         const long long ctas = columns * chunks_of(c);
         if (c != zchunk_limited(nz, c))
             continue;  // the same number of chunks as a shorter, more even one
-        if (ctas > 6LL * resident)
+        if (ctas > MOST_WAVES * resident)
             break;
-        const double cost = (double)((ctas + resident - 1) / resident) * (c + start);
+        const double cost = (double)((ctas + resident - 1) / resident) * (c + CTA_START);
         if (c == longest || cost < best_cost) {
             best = c;
             best_cost = cost;
@@ -850,7 +854,7 @@ int balanced_zchunk(int nz, int max_planes, long long columns, int resident, dou
 // 204 x 145 x 208 192 and 140; compact form 119 and 112, 16-bit R 128 and
 // 122, its 3 small solves 49 and 25.  Limits below 8 were no better there (24,
 // 154): those steps are bound by their three launches.
-int balanced_batch_limit(const std::vector<std::array<int, 2>> &grids, int max_planes, int resident, double start)
+int balanced_batch_limit(const std::vector<std::array<int, 2>> &grids, int max_planes, int resident)
 {
     const int limits[] = {max_planes, 48, 32, 24, 16, 8};
     int best = max_planes;
@@ -864,10 +868,10 @@ int balanced_batch_limit(const std::vector<std::array<int, 2>> &grids, int max_p
             const int c = zchunk_limited(g[1], limit);
             const long long n = (long long)g[0] * ((g[1] + c - 1) / c);
             ctas += n;
-            planes += (double)n * (c + start);
-            longest = std::max(longest, c + start);
+            planes += (double)n * (c + CTA_START);
+            longest = std::max(longest, c + CTA_START);
         }
-        if (resident < 1 || (best_cost < 0.0 && ctas > 6LL * resident))
+        if (resident < 1 || (best_cost < 0.0 && ctas > MOST_WAVES * resident))
             return max_planes;
         const double cost = std::max(planes / resident + 0.5 * longest, longest);
         if (best_cost < 0.0 || cost < best_cost) {

@@ -15,7 +15,7 @@ namespace {
 
 // One solve: CTA (bx, by, bz) processes one unit.
 template <int RY, int W, int S, bool R16>
-__global__ void __launch_bounds__(32 * W) strip_step_kernel(const __grid_constant__ StripArgs a,
+__global__ void __launch_bounds__(32 * W + 32) strip_step_kernel(const __grid_constant__ StripArgs a,
                                                             const __grid_constant__ StripMaps maps)
 {
     using G = StripGeo<RY, W, R16>;
@@ -24,7 +24,7 @@ __global__ void __launch_bounds__(32 * W) strip_step_kernel(const __grid_constan
     const NativeConsts &c = a.c;
     const int x0 = blockIdx.x * SX, y0 = blockIdx.y * G::TY, bz = blockIdx.z;
     const int zc0 = bz * a.zchunk, zc1 = min(c.nz, zc0 + a.zchunk);
-    strip_init_bars<S>(sm);
+    strip_init_bars<W, S>(sm);
     strip_load_coef(c, sm.coef, G::NTH);
     if (c.overlap_prev) {
         // Launched while the previous step's Mur kernel may still run (it
@@ -39,23 +39,21 @@ __global__ void __launch_bounds__(32 * W) strip_step_kernel(const __grid_constan
     }
     __syncthreads();
     bool stall = false;
-    if (c.stall_once && blockIdx.x == 0 && blockIdx.y == 0 && bz == 0 && threadIdx.x == 0)
+    if (c.stall_once && blockIdx.x == 0 && blockIdx.y == 0 && bz == 0 && threadIdx.x == G::CELL_THREADS)
         stall = atomicExch(c.stall_once, 0) != 0;
     const unsigned long long memless =
         c.memless ? c.memless[((size_t)bz * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x] : 0ull;
-    strip_unit<RY, W, S, R16>(c, maps, a.zchunk, blockIdx.x, blockIdx.y, bz, memless, sm, 0u, stall);
-    if (threadIdx.x == G::STORE_TID)
-        bulk_wait_all();
+    strip_unit<RY, W, S, R16>(c, maps, a.zchunk, blockIdx.x, blockIdx.y, bz, memless, sm, stall);
 }
 
 // ------------------------------------------------------------------ host side
 
-// z chunks of at most 24 planes, for both storage forms: on the
-// 512 x 512 x 400 phantom within 0.5 % of the fastest limit in every sweep
-// (12, 16, 20, 22, 23, 25, 27, 29, 32, 48 tried; in the latest, 23 and 29
-// ran 0.4 % and 0.2 % faster, 25 0.7 % and 20 1.2 % slower)
+// z chunks of at most 40 planes: us per step on the 512 x 512 x 400 phantom at
+// 24 / 31 / 40 / 45 / 58 planes 997 / 994 / 994 / 998 / 996 with 32-bit R and
+// 940 / 925 / 922 / 919 / 914 with 16-bit R; beyond 40 the grids of a few waves
+// lose (304 x 245 x 187: 153 at 27 planes, 165 at 47)
 #ifndef FDTD_STRIP_ZCHUNK
-#define FDTD_STRIP_ZCHUNK 24
+#define FDTD_STRIP_ZCHUNK 40
 #endif
 static_assert(FDTD_STRIP_ZCHUNK >= 2 && FDTD_STRIP_ZCHUNK <= 64, "a unit's memoryless-plane mask has 64 bits");
 
@@ -94,7 +92,7 @@ int solve_zchunk(int nx, int ny, int nz, int nclasses)
         return resident_ctas(strip_step_kernel<RY, W, S_SEL, R16>, G::NTH, strip_smem_bytes<RY, W, S_SEL, R16>(nclasses));
     });
     const long long columns = (long long)((nx + SX - 1) / SX) * ((ny + G::TY - 1) / G::TY);
-    return balanced_zchunk(nz, FDTD_STRIP_ZCHUNK, columns, r, 0.5);
+    return balanced_zchunk(nz, FDTD_STRIP_ZCHUNK, columns, r);
 }
 
 template <int SHAPE, bool R16>

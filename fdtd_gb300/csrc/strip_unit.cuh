@@ -1,6 +1,6 @@
 // strip_unit.cuh -- device side of the compact forms' strip kernels (one
 // work unit of the step), shared by the single-solve kernels
-// (step_strip.cu) and the persistent batched kernels (batch_strip.cu).
+// (step_strip.cu) and the batched kernels (batch_strip.cu).
 //
 // Same update as the compact path of step_fused.cu (H, D increment and
 // sources, Debye E and the recursion variable R, the x-face Mur updates),
@@ -17,9 +17,16 @@
 //   (E^n with a one-cell halo, H^{n-1/2} with a low x / low y halo, the tile's
 //   R, class bytes and, with 16-bit R, the rows' scale words).  Outputs go
 //   the same way: each thread writes its results into dense shared-memory
-//   tiles, and one thread stores the plane's H^{n+1/2},
-//   E^{n+1}, R^{n+1} (and scale words) with TMA stores.  No thread computes a
-//   global address per cell.
+//   tiles, over the boxes its plane was read from, and the plane's H^{n+1/2},
+//   E^{n+1}, R^{n+1} (and scale words) leave by TMA stores.  No thread
+//   computes a global address per cell.
+// * A warp of its own moves the planes: it waits until the other warps have
+//   consumed a plane, stores its tiles, waits until the stores have read them
+//   and refills the stage.  With thread 0 of the cell warps doing this, every
+//   plane of a CTA waited for its own stores: 1.9 us per plane of a lone CTA
+//   against 1.4 (64^3, 32-bit R).  us per step before and after: 512 x 512 x
+//   400 1018 and 992 (16-bit R 930 and 925), 150 x 134 x 170 52 and 48 (53 and
+//   50), 20 batched solves of 48-256 cells per axis 454 and 432 (480 and 440).
 // * Tiles whose cells, halo included, all lie inside the update ranges of
 //   every component, away from the x faces and from sources, take a path
 //   without per-cell range tests (CTA-uniform choice, per plane for the
@@ -46,7 +53,8 @@ constexpr int SX = 32;  // tile width in x: one warp's lanes
 
 template <int RY, int W, bool R16>
 struct StripGeo {
-    static constexpr int TY = RY * W, NTH = 32 * W;
+    static constexpr int TY = RY * W;
+    static constexpr int CELL_THREADS = 32 * W, NTH = CELL_THREADS + 32;  // the cell warps, then the moving warp
     static_assert(TY % 4 == 0 && TY <= 32, "tile rows: a multiple of 4 (scale-word boxes) and one lane per row");
     static constexpr int EW = SX + 8, EH = TY + 2;  // E^n box: x0-4 .. x0+35, y0-1 .. y0+TY
     static constexpr int HW = SX + 4, HH = TY + 1;  // H box: x0-4 .. x0+31, y0-1 .. y0+TY-1
@@ -67,24 +75,23 @@ struct StripGeo {
     static constexpr unsigned TX_FULL = 3u * E_BYTES + 3u * H_BYTES + 3u * R_BYTES + X_BYTES + M_BYTES;
     static constexpr unsigned TX_PRO = 3u * E_BYTES + 3u * H_BYTES;
     static constexpr unsigned TX_EPI = 3u * E_BYTES;
-    // the output tiles (dense 32 x TY): H^{n+1/2}, E^{n+1}, R^{n+1}, scale words
+    // The output tiles (dense 32 x TY) live in the plane's own ring stage:
+    // H^{n+1/2} and E^{n+1} over its E^n and H boxes (consumed by the H pass),
+    // R^{n+1} and the scale words in place (each cell's by the thread that
+    // read it).  They cost no shared memory; the stage's refill waits for its
+    // stores to have read them.
     static constexpr int T_BYTES = SX * TY * 4;
-    static constexpr int O_H = 0, O_E = 3 * T_BYTES, O_R = 6 * T_BYTES;
-    static constexpr int O_X = O_R + 3 * pad128(R_BYTES);
-    // Where the output tiles live: in the plane's own ring stage, over its
-    // E^n and H boxes (consumed by the H pass), when they fit below the
-    // stage's R tiles; else in an area of their own.  In the stage they cost
-    // no shared memory (one more CTA per SM), but the stage's refill waits
-    // for its stores to have read them.
-    static constexpr bool IN_STAGE = O_X + X_BYTES <= OFF_R;
-    static constexpr int OUT = IN_STAGE ? 0 : pad128(O_X + X_BYTES);
-    // the thread that issues the TMA stores: thread 0, which also issues the
-    // loads, when a stage's refill waits for its stores; else lane 0 of warp 1
-    static constexpr int STORE_TID = (W > 1 && !IN_STAGE) ? 32 : 0;
-    // H^{n+1/2} hz, hy of every row with the x0-1 column in front ([2][TY][33]),
-    // and hz, hx of the row above each warp's first row ([2][W][32]; row
-    // y0-1 for warp 0)
-    static constexpr int XC = 2 * TY * (SX + 1), XR = 2 * W * SX;
+    static constexpr int O_H = 0, O_E = 3 * T_BYTES;
+    static_assert(6 * T_BYTES <= OFF_R, "H and E output tiles fit over the boxes");
+    // H exchange of one plane: hz, hx of the row above each warp's first row
+    // ([2][W][32]; row y0-1 for warp 0), and hz, hy of the x0-1 column
+    // ([2][TY]).  Two sets, taken in turn by plane: a warp writes a plane's
+    // set again two planes later, behind a barrier that every warp reaches
+    // after reading it.
+    static constexpr int XR = 2 * W * SX, XC = 2 * TY, XSET = XR + XC;
+    // S barriers, then the give-up word
+    template <int S>
+    static constexpr int BAR_BYTES = (2 * S * 8 + 4 + 15) & ~15;
 };
 
 // Strip shapes: (cells per thread in y, warps per CTA).  0-2 use 8-row tiles
@@ -115,7 +122,7 @@ template <int RY, int W, int S, bool R16>
 constexpr int strip_smem_bytes(int nclasses)
 {
     using G = StripGeo<RY, W, R16>;
-    return 128 + S * G::STAGE + G::OUT + 4 * (G::XC + G::XR) + ((S * 8 + 15) & ~15) + nclasses * 32;
+    return 128 + S * G::STAGE + 4 * 2 * G::XSET + G::template BAR_BYTES<S> + nclasses * 32;
 }
 
 struct StripArgs {
@@ -143,13 +150,8 @@ __device__ __forceinline__ void fence_async_shared() { asm volatile("fence.proxy
 
 // One thread arms the stage's barrier and issues the plane's boxes; no_r:
 // the tile-plane holds no Debye memory, its R (and scale words) are not
-// loaded.  With arm_only (the stall test hook) nothing is issued.  part:
-// ISSUE_ALL, or the plane in two parts on one barrier -- ISSUE_HALO arms it
-// for the whole plane and issues the E^n and H boxes (the H pass's inputs),
-// ISSUE_TILE later issues the classes, R, scale words and x-face Mur
-// factors (the E pass's).
-enum StripIssuePart { ISSUE_ALL = 0, ISSUE_HALO = 1, ISSUE_TILE = 2 };
-
+// loaded.  With arm_only (the stall test hook) nothing is issued.
+//
 // A face tile's Mur factors: rows y0 .. of plane 0 of its x face (the near
 // one when a tile of a grid at most 32 cells wide holds both; the far face's
 // lanes then read theirs from global memory), nullptr in other tiles; plane z
@@ -162,25 +164,19 @@ struct StripFaces {
 
 template <int RY, int W, bool R16>
 __device__ __forceinline__ void strip_issue(const StripMaps &maps, const StripFaces &f, unsigned char *stage,
-                                            uint32_t bar, int kind, int x0, int y0, int z, bool arm_only, bool no_r,
-                                            int part = ISSUE_ALL)
+                                            uint32_t bar, int kind, int x0, int y0, int z, bool arm_only, bool no_r)
 {
     using G = StripGeo<RY, W, R16>;
-    if (part != ISSUE_TILE) {
-        const unsigned full = (no_r ? G::TX_FULL - 3u * G::R_BYTES - G::X_BYTES : G::TX_FULL) + (f.src ? f.bytes : 0u);
-        mbar_expect_tx(bar, kind == PLANE_FULL ? full : (kind == PLANE_PRO ? G::TX_PRO : G::TX_EPI));
-        if (arm_only)
-            return;
-        for (int c = 0; c < 3; c++)
-            tma_load_3d(smem_addr(stage + G::OFF_E + c * pad128(G::E_BYTES)), &maps.m[c], x0 - 4, y0 - 1, z, bar);
-        if (kind == PLANE_EPI)
-            return;
-        for (int c = 0; c < 3; c++)
-            tma_load_3d(smem_addr(stage + G::OFF_H + c * pad128(G::H_BYTES)), &maps.m[3 + c], x0 - 4, y0 - 1, z,
-                        bar);
-        if (part == ISSUE_HALO)
-            return;
-    }
+    const unsigned full = (no_r ? G::TX_FULL - 3u * G::R_BYTES - G::X_BYTES : G::TX_FULL) + (f.src ? f.bytes : 0u);
+    mbar_expect_tx(bar, kind == PLANE_FULL ? full : (kind == PLANE_PRO ? G::TX_PRO : G::TX_EPI));
+    if (arm_only)
+        return;
+    for (int c = 0; c < 3; c++)
+        tma_load_3d(smem_addr(stage + G::OFF_E + c * pad128(G::E_BYTES)), &maps.m[c], x0 - 4, y0 - 1, z, bar);
+    if (kind == PLANE_EPI)
+        return;
+    for (int c = 0; c < 3; c++)
+        tma_load_3d(smem_addr(stage + G::OFF_H + c * pad128(G::H_BYTES)), &maps.m[3 + c], x0 - 4, y0 - 1, z, bar);
     if (kind != PLANE_FULL)
         return;
     tma_load_3d(smem_addr(stage + G::OFF_M), &maps.m[9], x0, y0, z, bar);
@@ -251,15 +247,13 @@ __device__ __forceinline__ bool strip_has_source(const C &c, int x0, int y0, int
     return any;
 }
 
-// A CTA's shared memory: S ring stages, the output tiles, the H exchange
-// rows, S barriers, the class table.  The store of a plane's output tiles
-// must have read them before the next plane writes them: the storing thread
-// waits for that before the next plane's first barrier, so the store has a
-// whole H pass to drain.
+// A CTA's shared memory: S ring stages, the two H exchange sets, the S
+// barriers, the give-up word, the class table.
 struct StripSmem {
-    unsigned char *stages, *outs;
-    float *hnx, *xrw;
-    uint64_t *bars;
+    unsigned char *stages;
+    float *xch;
+    uint64_t *full, *consumed;
+    int *stop;
     DebyeCoef *coef;
 };
 
@@ -269,20 +263,23 @@ __device__ __forceinline__ StripSmem strip_smem(unsigned char *smem_raw)
     using G = StripGeo<RY, W, R16>;
     StripSmem m;
     m.stages = smem_raw + ((128 - (smem_addr(smem_raw) & 127)) & 127);
-    m.outs = m.stages + S * G::STAGE;
-    m.hnx = reinterpret_cast<float *>(m.outs + G::OUT);       // [2][TY][33]
-    m.xrw = m.hnx + G::XC;                                     // [2][W][32]
-    m.bars = reinterpret_cast<uint64_t *>(m.xrw + G::XR);
-    m.coef = reinterpret_cast<DebyeCoef *>(reinterpret_cast<unsigned char *>(m.bars) + ((S * 8 + 15) & ~15));
+    m.xch = reinterpret_cast<float *>(m.stages + S * G::STAGE);
+    m.full = reinterpret_cast<uint64_t *>(m.xch + 2 * G::XSET);
+    m.consumed = m.full + S;
+    m.stop = reinterpret_cast<int *>(m.consumed + S);
+    m.coef = reinterpret_cast<DebyeCoef *>(reinterpret_cast<unsigned char *>(m.full) + G::template BAR_BYTES<S>);
     return m;
 }
 
-template <int S>
+template <int W, int S>
 __device__ __forceinline__ void strip_init_bars(const StripSmem &m)
 {
     if (threadIdx.x == 0) {
-        for (int s = 0; s < S; s++)
-            mbar_init(smem_addr(&m.bars[s]), 1);
+        for (int s = 0; s < S; s++) {
+            mbar_init(smem_addr(&m.full[s]), 1);
+            mbar_init(smem_addr(&m.consumed[s]), W);
+        }
+        *m.stop = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
 }
@@ -296,34 +293,123 @@ __device__ __forceinline__ void strip_load_coef(const C &c, DebyeCoef *coef, int
         dst[i] = src[i];
 }
 
-// One work unit: column tile (bx, by), z chunk bz of one solve.  The ring's
-// stages and barrier phases continue from earlier units of the same CTA (g0
-// planes staged before).  memless: bit j set when plane zc0 + j of the tile
-// holds no Debye memory.  stall (thread 0 only): leave the second plane's
-// copies unissued (test hook).  Returns false when a bounded wait gave up
-// (the error flag is raised; the CTA must stop).
+// The planes of a unit as the moving warp and the cell warps see them: the
+// unit's first plane p0, its planes (prologue and epilogue included) and the
+// ring's stages and barrier phases.
+template <int RY, int W, int S, bool R16>
+struct StripPlanes {
+    using G = StripGeo<RY, W, R16>;
+    const StripSmem &sm;
+    int zc0, zc1, p0, nplanes;
+    unsigned long long memless;  // bit j: plane zc0 + j of the tile holds no Debye memory
+    __device__ __forceinline__ StripPlanes(const StripSmem &m, int nz, int zchunk, int bz, unsigned long long ml)
+        : sm(m), zc0(bz * zchunk), zc1(min(nz, bz * zchunk + zchunk)), p0(max(zc0 - 1, 0)),
+          nplanes(min(zc1, nz - 1) - p0 + 1), memless(ml)
+    {
+    }
+    __device__ __forceinline__ unsigned char *stage(int k) const { return sm.stages + (k % S) * G::STAGE; }
+    __device__ __forceinline__ uint32_t full(int k) const { return smem_addr(&sm.full[k % S]); }
+    __device__ __forceinline__ uint32_t consumed(int k) const { return smem_addr(&sm.consumed[k % S]); }
+    __device__ __forceinline__ uint32_t parity(int k) const { return (uint32_t)((k / S) & 1); }
+    __device__ __forceinline__ bool no_r(int z) const { return z >= zc0 && ((memless >> (z - zc0)) & 1ull) != 0; }
+};
+
+constexpr int BAR_CELLS = 1;  // named barrier of the cell warps alone
+
+__device__ __forceinline__ void mbar_arrive(uint32_t bar)
+{
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+
+// The moving warp's one lane at work: run() fills the ring, then plane by
+// plane waits until the cell warps have consumed the plane, stores the tiles
+// they have left in its stage and refills the stage.  Its waits are bounded;
+// when one gives up, or a cell warp's did (the stop word), the copies in
+// flight land (bounded) and the unit ends.  stall: leave the second plane's
+// copies unissued (test hook).
+template <int RY, int W, int S, bool R16>
+struct StripMove {
+    using G = StripGeo<RY, W, R16>;
+    const StripMaps &maps;
+    const StripPlanes<RY, W, S, R16> &u;
+    StripFaces faces;
+    int x0, y0;
+    __device__ __forceinline__ void issue(int k, bool arm_only) const
+    {
+        const int z = u.p0 + k;
+        strip_issue<RY, W, R16>(maps, faces, u.stage(k), u.full(k), plane_kind(z, u.zc0, u.zc1), x0, y0, z, arm_only,
+                                u.no_r(z));
+    }
+    __device__ __forceinline__ void store(int k) const
+    {
+        const int z = u.p0 + k;
+        const uint32_t ob = smem_addr(u.stage(k));
+        const bool no_r = u.no_r(z);
+        for (int comp = 0; comp < 3; comp++) {
+            tma_store_3d(&maps.m[11 + comp], ob + G::O_H + comp * G::T_BYTES, x0, y0, z);
+            tma_store_3d(&maps.m[14 + comp], ob + G::O_E + comp * G::T_BYTES, x0, y0, z);
+            if (!no_r)
+                tma_store_3d(&maps.m[6 + comp], ob + G::OFF_R + comp * pad128(G::R_BYTES), x0, y0, z);
+        }
+        if (R16 && !no_r)
+            tma_store_3d(&maps.m[10], ob + G::OFF_X, y0, x0 / SX, z);
+        bulk_commit();
+    }
+    __device__ __forceinline__ void run(bool stall) const
+    {
+        for (int k = 0; k < S && k < u.nplanes; k++)
+            issue(k, stall && k == 1);
+        for (int k = 0; u.p0 + k < u.zc1; k++) {
+            if (!mbar_wait(u.consumed(k), u.parity(k)) || *static_cast<volatile int *>(u.sm.stop)) {
+                for (int j = k; j < u.nplanes && j < k + S; j++)
+                    mbar_wait(u.full(j), u.parity(j));
+                break;
+            }
+            if (u.p0 + k >= u.zc0)
+                store(k);
+            if (k + S < u.nplanes) {
+                bulk_wait_read<0>();  // the refill overwrites the tiles
+                issue(k + S, false);
+            }
+        }
+        bulk_wait_all();
+    }
+};
+
+// Barrier of the cell warps alone; true in every thread if any passes true.
+template <int THREADS>
+__device__ __forceinline__ bool cells_barrier_or(bool v)
+{
+    uint32_t r;
+    asm volatile(
+        "{\n .reg .pred p, q;\n setp.ne.u32 p, %1, 0;\n barrier.cta.red.or.pred q, %3, %2, p;\n"
+        " selp.u32 %0, 1, 0, q;\n}\n"
+        : "=r"(r)
+        : "r"((uint32_t)v), "n"(THREADS), "n"(BAR_CELLS)
+        : "memory");
+    return __any_sync(0xffffffffu, r != 0);  // a vote: known as uniform over the warp
+}
+
+// One work unit: column tile (bx, by), z chunk bz of one solve.  memless: bit
+// j set when plane zc0 + j of the tile holds no Debye memory.  stall: the
+// test hook of StripMove.  When a bounded wait gives up the error flag is
+// raised and the unit ends.
 template <int RY, int W, int S, bool R16, class C>
-__device__ __forceinline__ bool strip_unit(const C &c, const StripMaps &maps, int zchunk, int bx, int by,
-                                           int bz, unsigned long long memless, const StripSmem &sm, unsigned g0,
-                                           bool stall)
+__device__ __forceinline__ void strip_unit(const C &c, const StripMaps &maps, int zchunk, int bx, int by,
+                                           int bz, unsigned long long memless, const StripSmem &sm, bool stall)
 {
     using G = StripGeo<RY, W, R16>;
     constexpr int TY = G::TY;
-    float *hnx = sm.hnx, *xrw = sm.xrw;
-    const DebyeCoef *coef = sm.coef;
     const int nx = c.nx, ny = c.ny, nz = c.nz;
-    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31;
+    // by a shuffle: the compiler then knows the warp index as uniform over the
+    // warp, and keeps the plane loop's addresses in uniform registers behind the
+    // moving warp's branch (without it the 16-bit form ran 6 % slower)
+    const int w = __shfl_sync(0xffffffffu, tid >> 5, 0);
     const int x0 = bx * SX, y0 = by * TY;
-    const int x = x0 + lane, ry0 = w * RY;  // first row of this thread's strip, relative to y0
-    const int zc0 = bz * zchunk, zc1 = min(nz, zc0 + zchunk);
-    const int p0 = max(zc0 - 1, 0), plast = min(zc1, nz - 1);
-    const int nplanes = plast - p0 + 1;
-    const bool unit_src = strip_has_source(c, x0, y0, TY, zc0, zc1);
+    const StripPlanes<RY, W, S, R16> u(sm, nz, zchunk, bz, memless);
+    const int zc0 = u.zc0, zc1 = u.zc1, p0 = u.p0, nplanes = u.nplanes;
 
-    auto stage = [&](int k) { return sm.stages + ((g0 + k) % S) * G::STAGE; };
-    auto bar = [&](int k) { return smem_addr(&sm.bars[(g0 + k) % S]); };
-    auto parity = [&](int k) { return (uint32_t)(((g0 + k) / S) & 1); };
-    auto no_r = [&](int z) { return z >= zc0 && ((memless >> (z - zc0)) & 1ull) != 0; };
     // x-face Mur updates (updateMurBoundary ey/ez x faces,
     // fdtd_calculations.cu:280-340) in the tiles that hold x = 0 or nx-1;
     // their per-cell factors arrive with the plane's boxes
@@ -332,16 +418,21 @@ __device__ __forceinline__ bool strip_unit(const C &c, const StripMaps &maps, in
     const bool face_far_cta = (mur_bits & 2) && x0 <= nx - 1 && nx - 1 < x0 + SX;
     const bool face_cta = face_near || face_far_cta;
     const bool faces_both = face_near && face_far_cta;
-    StripFaces faces{nullptr, (size_t)ny, 0u};
-    if (face_cta) {
-        faces.bytes = (uint32_t)min(TY, ny - y0) * 16u;
-        faces.src = face_near ? c.mur_x + y0 : c.mur_x + (size_t)nz * ny + y0;
+    if (w == W) {
+        if (lane == 0) {
+            StripMove<RY, W, S, R16> move{maps, u, StripFaces{nullptr, (size_t)ny, 0u}, x0, y0};
+            if (face_cta) {
+                move.faces.bytes = (uint32_t)min(TY, ny - y0) * 16u;
+                move.faces.src = face_near ? c.mur_x + y0 : c.mur_x + (size_t)nz * ny + y0;
+            }
+            move.run(stall);
+        }
+        return;
     }
-    if (tid == 0)
-        for (int k = 0; k < S && k < nplanes; k++)
-            strip_issue<RY, W, R16>(maps, faces, stage(k), bar(k), plane_kind(p0 + k, zc0, zc1), x0, y0, p0 + k,
-                                    stall && k == 1, no_r(p0 + k));
 
+    const DebyeCoef *coef = sm.coef;
+    const int x = x0 + lane, ry0 = w * RY;  // first row of this thread's strip, relative to y0
+    const bool unit_src = strip_has_source(c, x0, y0, TY, zc0, zc1);
     float jz_now = 0.0f;
     if (unit_src) {
         const int n = c.step_counter ? *c.step_counter : c.step;
@@ -385,29 +476,36 @@ __device__ __forceinline__ bool strip_unit(const C &c, const StripMaps &maps, in
     for (int r = 0; r < RY; r++)
         hxm[r] = hym[r] = 0.0f;
 
-    auto give_up = [&](int k) {
+    // this warp is done with the plane in ring stage `slot` (its writes to the
+    // stage are visible to the TMA stores)
+    auto consumed = [&](int slot) {
+        fence_async_shared();
+        __syncwarp();
+        if (lane == 0)
+            mbar_arrive(smem_addr(&sm.consumed[slot]));
+    };
+    auto give_up = [&](int slot) {
         if (tid == 0) {
             atomicExch(c.err, 1);
-            for (int j = k; j < nplanes && j < k + S; j++)
-                mbar_wait(bar(j), parity(j));
+            *static_cast<volatile int *>(sm.stop) = 1;
         }
-        if (tid == G::STORE_TID)
-            bulk_wait_all();
-        __syncthreads();
+        consumed(slot);
     };
-
-    for (int k = 0; k < nplanes; k++) {
+    int slot = 0, next = 1;   // ring stages of planes k and k + 1 (S > 1)
+    uint32_t phase_next = 0;  // barrier phase of plane k + 1
+    for (int k = 0; p0 + k < zc1; k++, slot = next, next = next + 1 == S ? 0 : next + 1, phase_next ^= next == 0) {
         const int z = p0 + k;
-        if (z >= zc1)
-            break;
         bool ok = true;
         if (k == 0)
-            ok = mbar_wait(bar(0), parity(0));
+            ok = mbar_wait(smem_addr(&sm.full[0]), 0);
         if (ok && k + 1 < nplanes)
-            ok = mbar_wait(bar(k + 1), parity(k + 1));
-        const float *EA = reinterpret_cast<const float *>(stage(k) + G::OFF_E);
-        const float *EB = reinterpret_cast<const float *>(stage(k + 1) + G::OFF_E);
-        const float *HA = reinterpret_cast<const float *>(stage(k) + G::OFF_H);
+            ok = mbar_wait(smem_addr(&sm.full[next]), phase_next);
+        unsigned char *stage = sm.stages + slot * G::STAGE;
+        const float *EA = reinterpret_cast<const float *>(stage + G::OFF_E);
+        const float *EB = reinterpret_cast<const float *>(sm.stages + next * G::STAGE + G::OFF_E);
+        const float *HA = reinterpret_cast<const float *>(stage + G::OFF_H);
+        // this plane's H exchange set
+        float *xr = sm.xch + (k & 1) * G::XSET, *xc = xr + G::XR;
         constexpr int ES = pad128(G::E_BYTES) / 4, HS = pad128(G::H_BYTES) / 4;
         auto ea = [&](int comp, int r, int cc) { return EA[comp * ES + r * G::EW + cc]; };
         auto eb = [&](int comp, int r, int cc) { return EB[comp * ES + r * G::EW + cc]; };
@@ -458,19 +556,15 @@ __device__ __forceinline__ bool strip_unit(const C &c, const StripMaps &maps, in
                 hxm[r] = hxn[r];
                 hym[r] = hyn[r];
             }
-            if (__syncthreads_or(!ok)) {
-                give_up(k);
-                return false;
+            if (cells_barrier_or<G::CELL_THREADS>(!ok)) {
+                give_up(slot);
+                return;
             }
+            consumed(slot);
         } else {
-#pragma unroll
-            for (int r = 0; r < RY; r++) {
-                hnx[(ry0 + r) * (SX + 1) + lane + 1] = hzn[r];
-                hnx[(TY + ry0 + r) * (SX + 1) + lane + 1] = hyn[r];
-            }
             if (w + 1 < W) {
-                xrw[(w + 1) * SX + lane] = hzn[RY - 1];
-                xrw[(W + w + 1) * SX + lane] = hxn[RY - 1];
+                xr[(w + 1) * SX + lane] = hzn[RY - 1];
+                xr[(W + w + 1) * SX + lane] = hxn[RY - 1];
             }
             if (w == 0) {  // row y0 - 1: hx, hz (box row 0)
                 const float ex_ = ea(0, 0, ec), ey_ = ea(1, 0, ec), ez_ = ea(2, 0, ec);
@@ -486,8 +580,8 @@ __device__ __forceinline__ bool strip_unit(const C &c, const StripMaps &maps, in
                 } else {
                     vx = vz = 0.0f;
                 }
-                xrw[lane] = vz;
-                xrw[W * SX + lane] = vx;
+                xr[lane] = vz;
+                xr[W * SX + lane] = vx;
             }
             if (w == W - 1 && lane < TY) {  // column x0 - 1: hy, hz of row y0 + lane (box column 3)
                 const int er = lane + 1, cc = 3, yy = y0 + lane;
@@ -504,75 +598,68 @@ __device__ __forceinline__ bool strip_unit(const C &c, const StripMaps &maps, in
                 } else {
                     vy = vz = 0.0f;
                 }
-                hnx[lane * (SX + 1)] = vz;
-                hnx[(TY + lane) * (SX + 1)] = vy;
+                xc[lane] = vz;
+                xc[TY + lane] = vy;
             }
-            // the CTA decides here whether a wait gave up (nothing has
+            // the cell warps decide here whether a wait gave up (nothing has
             // reached global memory from this plane yet)
-            // outputs in their own area: the tiles this plane writes were
-            // stored one plane ago, and that store has read them by now
-            // (checked before the barrier)
-            if (!G::IN_STAGE && tid == G::STORE_TID)
-                bulk_wait_read<0>();
-            if (__syncthreads_or(!ok)) {
-                give_up(k);
-                return false;
-            }
-            // outputs in their own area: the H pass has consumed this
-            // stage's E^n and H boxes, refill them with plane k + S now, half
-            // a plane before the rest
-            if (!G::IN_STAGE && tid == 0 && k + S < nplanes) {
-                fence_async_shared();
-                const int zn = p0 + k + S;
-                strip_issue<RY, W, R16>(maps, faces, stage(k + S), bar(k + S), plane_kind(zn, zc0, zc1), x0, y0, zn,
-                                        false, no_r(zn), ISSUE_HALO);
+            if (cells_barrier_or<G::CELL_THREADS>(!ok)) {
+                give_up(slot);
+                return;
             }
 
             // ---- D increment, sources, E^{n+1} and R^{n+1} on the strip
-            const bool plane_no_r = no_r(z);  // uniform: R is +0 on every cell of the tile-plane
-            unsigned char *O = G::IN_STAGE ? stage(k) : sm.outs;
-            float *OH = reinterpret_cast<float *>(O + G::O_H);
-            float *OE = reinterpret_cast<float *>(O + G::O_E);
-            const unsigned char *M = stage(k) + G::OFF_M;
+            const bool plane_no_r = u.no_r(z);  // uniform: R is +0 on every cell of the tile-plane
+            float *OH = reinterpret_cast<float *>(stage + G::O_H);
+            float *OE = reinterpret_cast<float *>(stage + G::O_E);
+            const unsigned char *M = stage + G::OFF_M;
             constexpr int TS = SX * TY;  // elements of one dense tile
+            // every operand of the strip first, every result last: the stores may
+            // alias the loads, so the compiler keeps their order
+            float hz_xm[RY], hy_xm[RY], r0[RY], r1[RY], r2[RY];
+            DebyeCoef kcs[RY];
+            const float hz_row = xr[w * SX + lane], hx_row = xr[(W + w) * SX + lane];
 #pragma unroll
             for (int r = 0; r < RY; r++) {
-                const int row = ry0 + r, t = row * SX + lane, y = y0 + row;
-                const float hz_xm = hnx[row * (SX + 1) + lane], hy_xm = hnx[(TY + row) * (SX + 1) + lane];
-                const float hz_ym = r ? hzn[r - 1] : xrw[w * SX + lane];
-                const float hx_ym = r ? hxn[r - 1] : xrw[(W + w) * SX + lane];
-                const DebyeCoef kc = coef[min((int)M[t], cls_max)];
-                const float k12 = cm_k12(kc);
-                float r0, r1, r2;
-                float sc = 0.0f;
-                unsigned short q0 = 0, q1 = 0, q2 = 0;
+                const int row = ry0 + r, t = row * SX + lane;
+                const float hz_up = __shfl_up_sync(0xffffffffu, hzn[r], 1);
+                const float hy_up = __shfl_up_sync(0xffffffffu, hyn[r], 1);
+                hz_xm[r] = lane ? hz_up : xc[row];
+                hy_xm[r] = lane ? hy_up : xc[TY + row];
+                kcs[r] = coef[min((int)M[t], cls_max)];
                 if (plane_no_r) {
-                    r0 = r1 = r2 = 0.0f;
+                    r0[r] = r1[r] = r2[r] = 0.0f;
                 } else if constexpr (R16) {
-                    const unsigned short *RT = reinterpret_cast<const unsigned short *>(stage(k) + G::OFF_R);
+                    const unsigned short *RT = reinterpret_cast<const unsigned short *>(stage + G::OFF_R);
                     constexpr int RS = pad128(G::R_BYTES) / 2;
-                    q0 = RT[t];
-                    q1 = RT[RS + t];
-                    q2 = RT[2 * RS + t];
-                    sc = cm_r16_scale(reinterpret_cast<const uint32_t *>(stage(k) + G::OFF_X)[row]);
-                    r0 = cm_r16_r(q0, sc, kc.a, ex[r]);
-                    r1 = cm_r16_r(q1, sc, kc.a, ey[r]);
-                    r2 = cm_r16_r(q2, sc, kc.a, ez[r]);
+                    const float sc = cm_r16_scale(reinterpret_cast<const uint32_t *>(stage + G::OFF_X)[row]);
+                    r0[r] = cm_r16_r(RT[t], sc, kcs[r].a, ex[r]);
+                    r1[r] = cm_r16_r(RT[RS + t], sc, kcs[r].a, ey[r]);
+                    r2[r] = cm_r16_r(RT[2 * RS + t], sc, kcs[r].a, ez[r]);
                 } else {
-                    const float *RT = reinterpret_cast<const float *>(stage(k) + G::OFF_R);
+                    const float *RT = reinterpret_cast<const float *>(stage + G::OFF_R);
                     constexpr int RS = pad128(G::R_BYTES) / 4;
-                    r0 = RT[t];
-                    r1 = RT[RS + t];
-                    r2 = RT[2 * RS + t];
+                    r0[r] = RT[t];
+                    r1[r] = RT[RS + t];
+                    r2[r] = RT[2 * RS + t];
                 }
+            }
+            float en[3][RY], rn[3][RY];
+#pragma unroll
+            for (int r = 0; r < RY; r++) {
+                const int row = ry0 + r, y = y0 + row;
+                const float hz_ym = r ? hzn[r - 1] : hz_row;
+                const float hx_ym = r ? hxn[r - 1] : hx_row;
+                const DebyeCoef &kc = kcs[r];
+                const float k12 = cm_k12(kc);
                 float en0, en1, en2, rn0, rn1, rn2;
                 if (fast) {
                     const float g0 = cm_dinc(tcy, hzn[r], hz_ym, tcz, hyn[r], hym[r]);
-                    const float g1 = cm_dinc(tcz, hxn[r], hxm[r], tcx, hzn[r], hz_xm);
-                    const float g2 = cm_dinc(tcx, hyn[r], hy_xm, tcy, hxn[r], hx_ym);
-                    en0 = cm_e_next(kc, k12, ex[r], g0, r0);
-                    en1 = cm_e_next(kc, k12, ey[r], g1, r1);
-                    en2 = cm_e_next(kc, k12, ez[r], g2, r2);
+                    const float g1 = cm_dinc(tcz, hxn[r], hxm[r], tcx, hzn[r], hz_xm[r]);
+                    const float g2 = cm_dinc(tcx, hyn[r], hy_xm[r], tcy, hxn[r], hx_ym);
+                    en0 = cm_e_next(kc, k12, ex[r], g0, r0[r]);
+                    en1 = cm_e_next(kc, k12, ey[r], g1, r1[r]);
+                    en2 = cm_e_next(kc, k12, ez[r], g2, r2[r]);
                     rn0 = cm_r_next(kc, ex[r], g0);
                     rn1 = cm_r_next(kc, ey[r], g1);
                     rn2 = cm_r_next(kc, ez[r], g2);
@@ -585,20 +672,20 @@ __device__ __forceinline__ bool strip_unit(const C &c, const StripMaps &maps, in
                     const bool ex_on = has(r, M_E0) && zmid;  // also the range of g0
                     const float g0 = ex_on ? cm_dinc(tcy, hzn[r], hz_ym, tcz, hyn[r], hym[r]) : 0.0f;
                     const float g1 =
-                        has(r, M_E1) && zmid ? cm_dinc(tcz, hxn[r], hxm[r], tcx, hzn[r], hz_xm) : 0.0f;
+                        has(r, M_E1) && zmid ? cm_dinc(tcz, hxn[r], hxm[r], tcx, hzn[r], hz_xm[r]) : 0.0f;
                     bool src = false;
                     if (unit_src)
                         for (int s = 0; s < c.nsources; s++)
                             src |= c.sources[3 * s + 2] == z && c.sources[3 * s] == x && c.sources[3 * s + 1] == y;
-                    const float d2 = cm_dinc(tcx, hyn[r], hy_xm, tcy, hxn[r], hx_ym);
+                    const float d2 = cm_dinc(tcx, hyn[r], hy_xm[r], tcy, hxn[r], hx_ym);
                     const float g2 = has(r, M_DOM) && ((has(r, M_E2) && zlo) || src)
                                          ? (src ? __fsub_rn(d2, jz_now) : d2)
                                          : 0.0f;
                     const bool eyz_on = has(r, M_EYZ) && z >= 1;
                     // not updated: E keeps E^n, R keeps R^n (16-bit R: residual 0)
-                    const float u0 = cm_e_next(kc, k12, ex[r], g0, r0);
-                    const float u1 = cm_e_next(kc, k12, ey[r], g1, r1);
-                    const float u2 = cm_e_next(kc, k12, ez[r], g2, r2);
+                    const float u0 = cm_e_next(kc, k12, ex[r], g0, r0[r]);
+                    const float u1 = cm_e_next(kc, k12, ey[r], g1, r1[r]);
+                    const float u2 = cm_e_next(kc, k12, ez[r], g2, r2[r]);
                     float s0 = cm_r_next(kc, ex[r], g0), s1 = cm_r_next(kc, ey[r], g1), s2 = cm_r_next(kc, ez[r], g2);
                     if constexpr (R16) {
                         s0 = cm_r16_rho(kc.a, u0, s0);
@@ -608,9 +695,9 @@ __device__ __forceinline__ bool strip_unit(const C &c, const StripMaps &maps, in
                     en0 = ex_on ? u0 : ex[r];
                     en1 = eyz_on ? u1 : ey[r];
                     en2 = eyz_on ? u2 : ez[r];
-                    rn0 = ex_on ? s0 : (R16 ? 0.0f : r0);
-                    rn1 = eyz_on ? s1 : (R16 ? 0.0f : r1);
-                    rn2 = eyz_on ? s2 : (R16 ? 0.0f : r2);
+                    rn0 = ex_on ? s0 : (R16 ? 0.0f : r0[r]);
+                    rn1 = eyz_on ? s1 : (R16 ? 0.0f : r1[r]);
+                    rn2 = eyz_on ? s2 : (R16 ? 0.0f : r2[r]);
                     if (face_cta) {  // uniform over the CTA: every lane takes part in the shuffles
                         const unsigned all = 0xffffffffu;
                         const float ey_hi = __shfl_down_sync(all, en1, 1), ez_hi = __shfl_down_sync(all, en2, 1);
@@ -619,7 +706,7 @@ __device__ __forceinline__ bool strip_unit(const C &c, const StripMaps &maps, in
                             const float4 mf =
                                 faces_both && face_far
                                     ? c.mur_x[((size_t)nz + z) * ny + y]
-                                    : reinterpret_cast<const float4 *>(stage(k) + G::OFF_F)[row];
+                                    : reinterpret_cast<const float4 *>(stage + G::OFF_F)[row];
                             auto mur = [&](float tn, float sn, float sf) {
                                 return __fmul_rn(mf.x, __fsub_rn(__fadd_rn(__fmul_rn(mf.y, tn), __fmul_rn(mf.z, sn)),
                                                                  __fmul_rn(mf.w, sf)));
@@ -635,71 +722,49 @@ __device__ __forceinline__ bool strip_unit(const C &c, const StripMaps &maps, in
                         }
                     }
                 }
+                en[0][r] = en0;
+                en[1][r] = en1;
+                en[2][r] = en2;
+                rn[0][r] = rn0;
+                rn[1][r] = rn1;
+                rn[2][r] = rn2;
+            }
+#pragma unroll
+            for (int r = 0; r < RY; r++) {
+                const int row = ry0 + r, t = row * SX + lane, y = y0 + row;
                 OH[t] = hxn[r];
                 OH[TS + t] = hyn[r];
                 OH[2 * TS + t] = hzn[r];
-                OE[t] = en0;
-                OE[TS + t] = en1;
-                OE[2 * TS + t] = en2;
+                OE[t] = en[0][r];
+                OE[TS + t] = en[1][r];
+                OE[2 * TS + t] = en[2][r];
                 if (plane_no_r) {
                     // R stays +0: nothing to store
                 } else if constexpr (R16) {
                     // one warp is one row segment: every cell of it is
                     // rewritten with the segment's new scale
                     unsigned short h0, h1, h2;
-                    const uint32_t b = cm_r16_encode(rn0, rn1, rn2, h0, h1, h2);
-                    unsigned short *OR = reinterpret_cast<unsigned short *>(O + G::O_R);
+                    const uint32_t b = cm_r16_encode(rn[0][r], rn[1][r], rn[2][r], h0, h1, h2);
+                    unsigned short *OR = reinterpret_cast<unsigned short *>(stage + G::OFF_R);
                     constexpr int RS = pad128(G::R_BYTES) / 2;
                     OR[t] = h0;
                     OR[RS + t] = h1;
                     OR[2 * RS + t] = h2;
                     if (lane == 0)
-                        reinterpret_cast<uint32_t *>(O + G::O_X)[row] = y < ny ? b : 0u;
+                        reinterpret_cast<uint32_t *>(stage + G::OFF_X)[row] = y < ny ? b : 0u;
                 } else {
-                    float *OR = reinterpret_cast<float *>(O + G::O_R);
+                    float *OR = reinterpret_cast<float *>(stage + G::OFF_R);
                     constexpr int RS = pad128(G::R_BYTES) / 4;
-                    OR[t] = rn0;
-                    OR[RS + t] = rn1;
-                    OR[2 * RS + t] = rn2;
+                    OR[t] = rn[0][r];
+                    OR[RS + t] = rn[1][r];
+                    OR[2 * RS + t] = rn[2][r];
                 }
                 hxm[r] = hxn[r];
                 hym[r] = hyn[r];
             }
-            fence_async_shared();
-            __syncthreads();  // stage k consumed, output tiles written
-            if (tid == G::STORE_TID) {
-                const uint32_t ob = smem_addr(O);
-                for (int comp = 0; comp < 3; comp++) {
-                    tma_store_3d(&maps.m[11 + comp], ob + G::O_H + comp * G::T_BYTES, x0, y0, z);
-                    tma_store_3d(&maps.m[14 + comp], ob + G::O_E + comp * G::T_BYTES, x0, y0, z);
-                    if (!plane_no_r)
-                        tma_store_3d(&maps.m[6 + comp], ob + G::O_R + comp * pad128(G::R_BYTES), x0, y0, z);
-                }
-                if (R16 && !plane_no_r)
-                    tma_store_3d(&maps.m[10], ob + G::O_X, y0, x0 / SX, z);
-                bulk_commit();
-                if (G::IN_STAGE)  // the refill below overwrites the tiles
-                    bulk_wait_read<0>();
-            }
-        }
-        // refill the stage of plane k with plane k + S: all of it after a
-        // prologue plane or with the outputs in the stage, else its classes,
-        // R and scale words (the boxes went after the H pass)
-        if (tid == 0 && k + S < nplanes) {
-            fence_async_shared();
-            const int zn = p0 + k + S;
-            strip_issue<RY, W, R16>(maps, faces, stage(k + S), bar(k + S), plane_kind(zn, zc0, zc1), x0, y0, zn, false,
-                                    no_r(zn), (z < zc0 || G::IN_STAGE) ? ISSUE_ALL : ISSUE_TILE);
+            consumed(slot);
         }
     }
-    return true;
-}
-
-// Planes a unit stages (its ring advance).
-__host__ __device__ inline int strip_unit_planes(int nz, int zchunk, int bz)
-{
-    const int zc0 = bz * zchunk, zc1 = min(nz, zc0 + zchunk);
-    return min(zc1, nz - 1) - max(zc0 - 1, 0) + 1;
 }
 
 }  // namespace strip
