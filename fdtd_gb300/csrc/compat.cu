@@ -2,8 +2,12 @@
 //
 // Same argument lists and per-component index ranges as the reference's five
 // kernels, over the reference's float material arrays and three-slot state.
-// The grids differ: 32 x 8 thread tiles instead of 128 x 1 rows, sources as
-// one warp instead of a full grid, Mur over the face cells only.
+// The grids differ: 32 x 8 thread tiles (of several z planes for H and D)
+// instead of 128 x 1 rows, sources as one warp instead of a full grid, Mur over
+// the face cells only.  The kernels are programmatic dependents of the stream's
+// previous launch: one after another on a small grid they took 4.2-5.4 us each,
+// so 2.7-4.
+#include <algorithm>
 #include <array>
 #include <atomic>
 
@@ -38,35 +42,30 @@ int current_device_checked(int *dev)
     return FDTD_OK;
 }
 
-int launch_status()
-{
-    const cudaError_t e = cudaGetLastError();
-    return e == cudaSuccess ? FDTD_OK : (int)e;
-}
-
 constexpr int TX = 32, TY = 8;
+
+// z planes per thread of the H and D kernels, bound by HBM (36 bytes per cell).
+// With one plane per thread, each component loaded, updated and stored in
+// turn, they ran 114 and 117 us on 256 x 256 x 200 (4.1 and 4.0 TB/s): few loads
+// in flight, and E or H of the neighbouring plane read again through L2.  With
+// all loads first and 1 / 2 / 4 / 8 planes per thread: H 83 / 81 / 79 / 84 us, D 86
+// / 83 / 82 / 90.
+constexpr int H_PLANES = 4, D_PLANES = 4;
 
 __global__ void __launch_bounds__(TX *TY) compat_h_kernel(float *__restrict__ hx, float *__restrict__ hy,
                                                          float *__restrict__ hz, const float *__restrict__ ex,
                                                          const float *__restrict__ ey, const float *__restrict__ ez)
 {
+    pdl_begin();
     const int nx = c_sym.nx, ny = c_sym.ny, nz = c_sym.nz;
-    const int x = blockIdx.x * TX + threadIdx.x, y = blockIdx.y * TY + threadIdx.y, z = blockIdx.z;
-    if (x >= nx || y >= ny)
+    const int x = blockIdx.x * TX + threadIdx.x, y = blockIdx.y * TY + threadIdx.y;
+    if (x >= nx - 1 || y >= ny - 1)
         return;
     const float dt = c_sym.dt, mu0 = c_sym.mu0;
     const float kx = dt / (mu0 * c_sym.dx), ky = dt / (mu0 * c_sym.dy), kz = dt / (mu0 * c_sym.dz);
-    const size_t i = cell_index(x, y, z, nx, ny);
-    const size_t sx = 1, sy = nx, sz = (size_t)nx * ny;
-    // hx: x 1..nx-2, y 0..ny-2, z 0..nz-2; both terms scaled by dy (:48-52)
-    if (x >= 1 && x < nx - 1 && y < ny - 1 && z < nz - 1)
-        hx[i] = hx[i] - ky * (ez[i + sy] - ez[i]) + ky * (ey[i + sz] - ey[i]);
-    // hy: x 0..nx-2, y 1..ny-2, z 0..nz-2 (:60-64)
-    if (x < nx - 1 && y >= 1 && y < ny - 1 && z < nz - 1)
-        hy[i] = hy[i] - kz * (ex[i + sz] - ex[i]) + kx * (ez[i + sx] - ez[i]);
-    // hz: x 0..nx-2, y 0..ny-2, z 1..nz-2 (:71-75)
-    if (x < nx - 1 && y < ny - 1 && z >= 1 && z < nz - 1)
-        hz[i] = hz[i] - kx * (ey[i + sx] - ey[i]) + ky * (ex[i + sy] - ex[i]);
+    const float *const in[3] = {hx, hy, hz};
+    float *const out[3] = {hx, hy, hz};
+    h_column<H_PLANES>(x, y, blockIdx.z * H_PLANES, nx, ny, nz, nx, kx, ky, kz, ex, ey, ez, in, out);
 }
 
 __global__ void __launch_bounds__(TX *TY) compat_d_kernel(float *__restrict__ dxT, float *__restrict__ dyT,
@@ -75,19 +74,56 @@ __global__ void __launch_bounds__(TX *TY) compat_d_kernel(float *__restrict__ dx
                                                          const float *__restrict__ hx, const float *__restrict__ hy,
                                                          const float *__restrict__ hz)
 {
+    pdl_begin();
+    constexpr int K = D_PLANES;
     const int nx = c_sym.nx, ny = c_sym.ny, nz = c_sym.nz;
-    const int x = blockIdx.x * TX + threadIdx.x, y = blockIdx.y * TY + threadIdx.y, z = blockIdx.z;
-    if (x >= nx || y >= ny)
-        return;
+    const int x = blockIdx.x * TX + threadIdx.x, y = blockIdx.y * TY + threadIdx.y, z0 = blockIdx.z * K;
+    if (x >= nx - 1 || y >= ny - 1)
+        return;  // no D component is updated at x = nx-1, y = ny-1 or z = nz-1
+    const int n = min(K, nz - 1 - z0);
     const float tx = c_sym.dt / c_sym.dx, ty = c_sym.dt / c_sym.dy, tz = c_sym.dt / c_sym.dz;
-    const size_t i = cell_index(x, y, z, nx, ny);
-    const size_t sx = 1, sy = nx, sz = (size_t)nx * ny;
-    if (x < nx - 1 && y >= 1 && y < ny - 1 && z >= 1 && z < nz - 1)
-        dxT[i] = dxS[i] + ty * (hz[i] - hz[i - sy]) - tz * (hy[i] - hy[i - sz]);
-    if (x >= 1 && x < nx - 1 && y < ny - 1 && z >= 1 && z < nz - 1)
-        dyT[i] = dyS[i] + tz * (hx[i] - hx[i - sz]) - tx * (hz[i] - hz[i - sx]);
-    if (x >= 1 && x < nx - 1 && y >= 1 && y < ny - 1 && z < nz - 1)
-        dzT[i] = dzS[i] + tx * (hy[i] - hy[i - sx]) - ty * (hx[i] - hx[i - sy]);
+    const size_t i = cell_index(x, y, z0, nx, ny), sy = nx, sz = (size_t)nx * ny;
+    const bool xi = x >= 1, yi = y >= 1;
+    // every load before the first store; H x, y of a plane are read once for
+    // the cells above and below it
+    float a[K + 1], b[K + 1], c[K], ay[K], bx[K], cx[K], cy[K], d[3][K];
+    a[0] = b[0] = 0.0f;
+    if (z0 >= 1) {
+        a[0] = hx[i - sz];
+        b[0] = hy[i - sz];
+    }
+#pragma unroll
+    for (int k = 0; k < K; k++)
+        if (k < n) {
+            const size_t j = i + k * sz;
+            a[k + 1] = hx[j];
+            b[k + 1] = hy[j];
+            c[k] = hz[j];
+            if (yi) {
+                ay[k] = hx[j - sy];
+                cy[k] = hz[j - sy];
+                d[0][k] = dxS[j];
+            }
+            if (xi) {
+                bx[k] = hy[j - 1];
+                cx[k] = hz[j - 1];
+                d[1][k] = dyS[j];
+            }
+            if (xi && yi)
+                d[2][k] = dzS[j];
+        }
+#pragma unroll
+    for (int k = 0; k < K; k++)
+        if (k < n) {
+            const size_t j = i + k * sz;
+            const bool zi = z0 + k >= 1;
+            if (yi && zi)
+                dxT[j] = d[0][k] + ty * (c[k] - cy[k]) - tz * (b[k + 1] - b[k]);
+            if (xi && zi)
+                dyT[j] = d[1][k] + tz * (a[k + 1] - a[k]) - tx * (c[k] - cx[k]);
+            if (xi && yi)
+                dzT[j] = d[2][k] + tx * (b[k + 1] - bx[k]) - ty * (a[k + 1] - ay[k]);
+        }
 }
 
 struct ETriplet {
@@ -100,6 +136,7 @@ __global__ void __launch_bounds__(TX *TY) compat_e_kernel(ETriplet a, const floa
                                                          const float *__restrict__ eps_s,
                                                          const float *__restrict__ tau_d)
 {
+    pdl_begin();
     const int nx = c_sym.nx, ny = c_sym.ny, nz = c_sym.nz;
     const int x = blockIdx.x * TX + threadIdx.x, y = blockIdx.y * TY + threadIdx.y, z = blockIdx.z;
     if (x >= nx || y >= ny)
@@ -110,18 +147,32 @@ __global__ void __launch_bounds__(TX *TY) compat_e_kernel(ETriplet a, const floa
     if (!ex_on && !eyz_on)
         return;
     const size_t i = cell_index(x, y, z, nx, ny);
-    const DebyeCoef k = cell_coef(c_sym.dt, c_sym.eps0, sigma[i], eps_s[i], eps_i[i], tau_d[i], FDTD_SCHEME_REFERENCE);
+    // all 19 loads before the first store: with each component loaded, updated
+    // and stored in turn the kernel ran 184 us on 256 x 256 x 200 (6.3 TB/s on its
+    // 88 bytes per cell), so 162 (7.1 TB/s); two or four planes per thread gave
+    // nothing more
+    const float s = sigma[i], es = eps_s[i], ei = eps_i[i], tau = tau_d[i];
+    float v[3][5];
 #pragma unroll
-    for (int c = 0; c < 3; c++) {
-        if (c == 0 ? !ex_on : !eyz_on)
-            continue;
-        a.t[c][i] = debye_update(k, a.e0[c][i], a.e1[c][i], a.d0[c][i], a.d1[c][i], a.d2[c][i]);
-    }
+    for (int c = 0; c < 3; c++)
+        if (c == 0 ? ex_on : eyz_on) {
+            v[c][0] = a.e0[c][i];
+            v[c][1] = a.e1[c][i];
+            v[c][2] = a.d0[c][i];
+            v[c][3] = a.d1[c][i];
+            v[c][4] = a.d2[c][i];
+        }
+    const DebyeCoef k = cell_coef(c_sym.dt, c_sym.eps0, s, es, ei, tau, FDTD_SCHEME_REFERENCE);
+#pragma unroll
+    for (int c = 0; c < 3; c++)
+        if (c == 0 ? ex_on : eyz_on)
+            a.t[c][i] = debye_update(k, v[c][0], v[c][1], v[c][2], v[c][3], v[c][4]);
 }
 
 __global__ void compat_sources_kernel(float *__restrict__ dzT, const float *__restrict__ dzS,
                                       const float *__restrict__ hx, const float *__restrict__ hy, int iter)
 {
+    pdl_begin();
     const int s = threadIdx.x;
     if (s >= c_sym.nsources)
         return;
@@ -138,17 +189,20 @@ struct MurArgs {
     MurSlabs rp;
 };
 
-__global__ void __launch_bounds__(256) compat_mur_kernel(MurArgs a)
+// Face set blockIdx.z; x runs along its faster in-face axis, each thread takes
+// MUR_ROWS rows of the other, gridDim.y apart, loads before stores.
+constexpr int MUR_THREADS = 128, MUR_ROWS = 4;
+
+__global__ void __launch_bounds__(MUR_THREADS) compat_mur_kernel(MurArgs a)
 {
+    pdl_begin();
     const int nx = c_sym.nx, ny = c_sym.ny, nz = c_sym.nz;
-    const int f = blockIdx.y;
+    const int f = blockIdx.z;
     const MurFace m = mur_face(f, nx, ny, nz);
-    const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= (long long)m.len_u * m.len_v)
-        return;
-    const int iu = (int)(idx % m.len_u), iv = (int)(idx / m.len_u);
-    mur_apply(f, iu, iv, nx, ny, nz, nx, c_sym.dt, c_sym.dx, c_sym.dy, c_sym.dz, c_sym.mu0 * c_sym.eps0, a.rp, a.t[0],
-              a.t[1], a.t[2], a.s[0], a.s[1], a.s[2], false);
+    const int iu = blockIdx.x * MUR_THREADS + threadIdx.x;
+    for (int iv = blockIdx.y; iv < m.len_v; iv += MUR_ROWS * gridDim.y)
+        mur_apply_k<MUR_ROWS>(f, iu, iv, gridDim.y, m.len_v, nx, ny, nz, nx, c_sym.dt, c_sym.dx, c_sym.dy, c_sym.dz,
+                              c_sym.mu0 * c_sym.eps0, a.rp, a.t[0], a.t[1], a.t[2], a.s[0], a.s[1], a.s[2], false);
 }
 
 int prologue(SymbolBlock *sym)
@@ -163,7 +217,11 @@ int prologue(SymbolBlock *sym)
     return FDTD_OK;
 }
 
-dim3 cell_grid(const SymbolBlock &s) { return dim3((s.nx + TX - 1) / TX, (s.ny + TY - 1) / TY, s.nz); }
+// The cells in columns of `planes` z planes.
+dim3 cell_grid(const SymbolBlock &s, int planes)
+{
+    return dim3((s.nx + TX - 1) / TX, (s.ny + TY - 1) / TY, (s.nz + planes - 1) / planes);
+}
 
 }  // namespace
 }  // namespace fdtd
@@ -216,8 +274,8 @@ int fdtd_update_h(float *hx, float *hy, float *hz, const float *exSource, const 
         return st;
     if (!hx || !hy || !hz || !exSource || !eySource || !ezSource)
         return FDTD_ERR_INVALID;
-    compat_h_kernel<<<cell_grid(s), dim3(TX, TY), 0, stream>>>(hx, hy, hz, exSource, eySource, ezSource);
-    return launch_status();
+    return launch_pdl(compat_h_kernel, cell_grid(s, H_PLANES), dim3(TX, TY), stream, hx, hy, hz, exSource, eySource,
+                      ezSource);
 }
 
 int fdtd_update_d(float *dxTarget, float *dyTarget, float *dzTarget, const float *dxSource, const float *dySource,
@@ -229,9 +287,8 @@ int fdtd_update_d(float *dxTarget, float *dyTarget, float *dzTarget, const float
         return st;
     if (!dxTarget || !dyTarget || !dzTarget || !dxSource || !dySource || !dzSource || !hx || !hy || !hz)
         return FDTD_ERR_INVALID;
-    compat_d_kernel<<<cell_grid(s), dim3(TX, TY), 0, stream>>>(dxTarget, dyTarget, dzTarget, dxSource, dySource,
-                                                              dzSource, hx, hy, hz);
-    return launch_status();
+    return launch_pdl(compat_d_kernel, cell_grid(s, D_PLANES), dim3(TX, TY), stream, dxTarget, dyTarget, dzTarget,
+                      dxSource, dySource, dzSource, hx, hy, hz);
 }
 
 int fdtd_update_e(float *exTarget, float *eyTarget, float *ezTarget, const float *exSource0, const float *eySource0,
@@ -256,8 +313,7 @@ int fdtd_update_e(float *exTarget, float *eyTarget, float *ezTarget, const float
             return FDTD_ERR_INVALID;
     if (!sigma || !epsI || !epsS || !tauD)
         return FDTD_ERR_INVALID;
-    compat_e_kernel<<<cell_grid(s), dim3(TX, TY), 0, stream>>>(a, sigma, epsI, epsS, tauD);
-    return launch_status();
+    return launch_pdl(compat_e_kernel, cell_grid(s, 1), dim3(TX, TY), stream, a, sigma, epsI, epsS, tauD);
 }
 
 int fdtd_update_sources(float *dzTarget, const float *dzSource, const float *hx, const float *hy, int currIteration,
@@ -271,8 +327,7 @@ int fdtd_update_sources(float *dzTarget, const float *dzSource, const float *hx,
         return FDTD_ERR_INVALID;
     if (s.nsources == 0)
         return FDTD_OK;
-    compat_sources_kernel<<<1, 32, 0, stream>>>(dzTarget, dzSource, hx, hy, currIteration);
-    return launch_status();
+    return launch_pdl(compat_sources_kernel, dim3(1), dim3(32), stream, dzTarget, dzSource, hx, hy, currIteration);
 }
 
 int fdtd_update_mur(float *exTarget, float *eyTarget, float *ezTarget, const float *exSource, const float *eySource,
@@ -289,13 +344,15 @@ int fdtd_update_mur(float *exTarget, float *eyTarget, float *ezTarget, const flo
             return FDTD_ERR_INVALID;
     if (!rpx0 || !rpy0 || !rpz0 || !rpxEnd || !rpyEnd || !rpzEnd)
         return FDTD_ERR_INVALID;
-    long long most = 0;
+    int most_u = 1, most_v = 1;
     for (int f = 0; f < 12; f++) {
         const MurFace m = mur_face(f, s.nx, s.ny, s.nz);
-        most = std::max(most, (long long)m.len_u * m.len_v);
+        most_u = std::max(most_u, m.len_u);
+        most_v = std::max(most_v, m.len_v);
     }
-    compat_mur_kernel<<<dim3((unsigned)((most + 255) / 256), 12), 256, 0, stream>>>(a);
-    return launch_status();
+    const int rows = (most_v + MUR_ROWS - 1) / MUR_ROWS;
+    const dim3 grid((unsigned)((most_u + MUR_THREADS - 1) / MUR_THREADS), (unsigned)std::min(rows, 65535), 12);
+    return launch_pdl(compat_mur_kernel, grid, dim3(MUR_THREADS), stream, a);
 }
 
 }  // extern "C"

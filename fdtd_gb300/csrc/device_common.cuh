@@ -12,6 +12,79 @@ __host__ __device__ inline size_t cell_index(int x, int y, int z, int nx, int ny
     return ((size_t)z * (size_t)ny + (size_t)y) * (size_t)nx + (size_t)x;
 }
 
+// Programmatic dependent launch: lets the next launch's blocks be placed while
+// this grid finishes, and (before any access to memory) waits for the previous
+// grid to complete.  A stream's order is kept: every kernel launched this way
+// waits before it reads or writes.
+__device__ __forceinline__ void pdl_begin()
+{
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+// Launches kernel so that its blocks may be placed before the stream's
+// previous grid completes; the kernel must call pdl_begin() first.
+template <class... P, class... A>
+int launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t stream, A &&...args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+    return e == cudaSuccess ? FDTD_OK : (int)e;
+}
+
+// updateHField (fdtd_calculations.cu:32-77) for the cells (x, y, z0 .. z0+K-1),
+// x < nx-1, y < ny-1: every load before the first store, and E^n x, y of a
+// plane read once for the cells below and above it.  out may be in.
+template <int K>
+__device__ __forceinline__ void h_column(int x, int y, int z0, int nx, int ny, int nz, int pitch, float kx, float ky,
+                                         float kz, const float *ex, const float *ey, const float *ez,
+                                         const float *const in[3], float *const out[3])
+{
+    const int n = min(K, nz - 1 - z0);  // no component is updated at z = nz-1
+    const size_t i = cell_index(x, y, z0, pitch, ny), sy = pitch, sz = (size_t)pitch * ny;
+    const bool xi = x >= 1, yi = y >= 1;
+    float a[K + 1], b[K + 1], c[K], ay[K], bx[K], cx[K], cy[K], h[3][K];
+#pragma unroll
+    for (int k = 0; k <= K; k++)
+        if (k <= n) {
+            a[k] = ex[i + k * sz];
+            b[k] = ey[i + k * sz];
+        }
+#pragma unroll
+    for (int k = 0; k < K; k++)
+        if (k < n) {
+            const size_t j = i + k * sz;
+            c[k] = ez[j];
+            cy[k] = ez[j + sy];
+            cx[k] = ez[j + 1];
+            ay[k] = ex[j + sy];
+            bx[k] = ey[j + 1];
+            h[0][k] = in[0][j];
+            h[1][k] = in[1][j];
+            h[2][k] = in[2][j];
+        }
+#pragma unroll
+    for (int k = 0; k < K; k++)
+        if (k < n) {
+            const size_t j = i + k * sz;
+            // hx: both terms scaled by dy (fdtd_calculations.cu:48-52)
+            if (xi)
+                out[0][j] = h[0][k] - ky * (cy[k] - c[k]) + ky * (b[k + 1] - b[k]);
+            if (yi)
+                out[1][j] = h[1][k] - kz * (a[k + 1] - a[k]) + kx * (cx[k] - c[k]);
+            if (z0 + k >= 1)
+                out[2][j] = h[2][k] - kx * (bx[k] - b[k]) + ky * (ay[k] - a[k]);
+        }
+}
+
 // Debye E update of one component (fdtd_calculations.cu:150-156): E^{n+1} =
 // c (d E^n - a E^{n-1} + k1 D^{n+1} - k2 D^n + k3 D^{n-1}), the D terms in
 // the difference form of DebyeCoef.
