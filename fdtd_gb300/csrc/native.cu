@@ -159,25 +159,18 @@ __device__ __forceinline__ DebyeCoef load_coef(const DebyeCoef *__restrict__ tab
 }
 
 // updateHField (fdtd_calculations.cu:32-77) with separate in and out buffers
-// (they may alias).
+// (they may alias), H_PLANES z planes per thread, bound by HBM (36 bytes per
+// cell): 82 us on 250 x 239 x 160 with one plane per thread and each component
+// loaded, updated and stored in turn, 61 so (5.6 TB/s); two planes: 62.
+constexpr int H_PLANES = 4;
+
 __global__ void __launch_bounds__(TX *TY) native_h_kernel(NativeConsts c)
 {
-    const int nx = c.nx, ny = c.ny, nz = c.nz;
-    const int x = blockIdx.x * TX + threadIdx.x, y = blockIdx.y * TY + threadIdx.y, z = blockIdx.z;
-    if (x >= nx - 1 || y >= ny - 1 || z >= nz - 1)
+    const int x = blockIdx.x * TX + threadIdx.x, y = blockIdx.y * TY + threadIdx.y;
+    if (x >= c.nx - 1 || y >= c.ny - 1)
         return;  // no H component is updated at x = nx-1, y = ny-1 or z = nz-1
-    const size_t i = cell_index(x, y, z, c.pitch, ny);
-    const size_t sx = 1, sy = c.pitch, sz = (size_t)c.pitch * ny;
-    const float *__restrict__ ex = c.e_cur[0];
-    const float *__restrict__ ey = c.e_cur[1];
-    const float *__restrict__ ez = c.e_cur[2];
-    const float ex0 = ex[i], ey0 = ey[i], ez0 = ez[i];
-    if (x >= 1)
-        c.h_out[0][i] = c.h_in[0][i] - c.ky * (ez[i + sy] - ez0) + c.ky * (ey[i + sz] - ey0);
-    if (y >= 1)
-        c.h_out[1][i] = c.h_in[1][i] - c.kz * (ex[i + sz] - ex0) + c.kx * (ez[i + sx] - ez0);
-    if (z >= 1)
-        c.h_out[2][i] = c.h_in[2][i] - c.kx * (ey[i + sx] - ey0) + c.ky * (ex[i + sy] - ex0);
+    h_column<H_PLANES>(x, y, blockIdx.z * H_PLANES, c.nx, c.ny, c.nz, c.pitch, c.kx, c.ky, c.kz, c.e_cur[0], c.e_cur[1],
+                       c.e_cur[2], c.h_in, c.h_out);
 }
 
 __device__ __forceinline__ int source_sample_index(const NativeConsts &c, int n)
@@ -186,7 +179,9 @@ __device__ __forceinline__ int source_sample_index(const NativeConsts &c, int n)
 }
 
 // updateDField + updateSources + updateEField for one cell (fdtd_calculations.cu
-// :80-122, :187-213, :125-184).  H^{n+1/2} is read from h_out.
+// :80-122, :187-213, :125-184).  H^{n+1/2} is read from h_out.  Bound by HBM (85
+// bytes per cell): with the Mur launch 178 us on 250 x 239 x 160 with loads and
+// stores mixed, 140 with every load first.
 __global__ void __launch_bounds__(TX *TY) native_de_kernel(NativeConsts c)
 {
     const int nx = c.nx, ny = c.ny, nz = c.nz;
@@ -194,7 +189,7 @@ __global__ void __launch_bounds__(TX *TY) native_de_kernel(NativeConsts c)
     if (x >= nx || y >= ny)
         return;
     const size_t i = cell_index(x, y, z, c.pitch, ny);
-    const size_t sx = 1, sy = c.pitch, sz = (size_t)c.pitch * ny;
+    const size_t sy = c.pitch, sz = (size_t)c.pitch * ny;
     const float *__restrict__ hx = c.h_out[0];
     const float *__restrict__ hy = c.h_out[1];
     const float *__restrict__ hz = c.h_out[2];
@@ -219,19 +214,44 @@ __global__ void __launch_bounds__(TX *TY) native_de_kernel(NativeConsts c)
     if (!ex_on && !eyz_on && !dx_on && !dy_on && !dz_on && !is_src)
         return;
 
-    float dn[3], dp[3], dnew[3];
+    // every load before the first store
+    const bool d_on = dx_on || dy_on || dz_on || is_src, h_xm = x >= 1, h_ym = y >= 1, h_zm = z >= 1;
+    float dn[3], dp[3], dnew[3], e0[3], e1[3];
+    float hx0 = 0, hy0 = 0, hz0 = 0, hx_y = 0, hx_z = 0, hy_x = 0, hy_z = 0, hz_x = 0, hz_y = 0;
 #pragma unroll
     for (int k = 0; k < 3; k++) {
         dn[k] = c.d_cur[k][i];
         dp[k] = c.d_prev[k][i];
         dnew[k] = dp[k];  // untouched cells keep the slot's value
+        if (k == 0 ? ex_on : eyz_on) {
+            e0[k] = c.e_cur[k][i];
+            e1[k] = c.e_prev[k][i];
+        }
     }
+    if (d_on) {
+        hx0 = hx[i];
+        hy0 = hy[i];
+        hz0 = hz[i];
+        if (h_xm) {
+            hy_x = hy[i - 1];
+            hz_x = hz[i - 1];
+        }
+        if (h_ym) {
+            hx_y = hx[i - sy];
+            hz_y = hz[i - sy];
+        }
+        if (h_zm) {
+            hx_z = hx[i - sz];
+            hy_z = hy[i - sz];
+        }
+    }
+    const int cls = (ex_on || eyz_on) ? c.mat[i] : 0;
     if (dx_on)
-        dnew[0] = dn[0] + c.ty * (hz[i] - hz[i - sy]) - c.tz * (hy[i] - hy[i - sz]);
+        dnew[0] = dn[0] + c.ty * (hz0 - hz_y) - c.tz * (hy0 - hy_z);
     if (dy_on)
-        dnew[1] = dn[1] + c.tz * (hx[i] - hx[i - sz]) - c.tx * (hz[i] - hz[i - sx]);
+        dnew[1] = dn[1] + c.tz * (hx0 - hx_z) - c.tx * (hz0 - hz_x);
     if (dz_on || is_src) {
-        dnew[2] = dn[2] + c.tx * (hy[i] - hy[i - sx]) - c.ty * (hx[i] - hx[i - sy]);
+        dnew[2] = dn[2] + c.tx * (hy0 - hy_x) - c.ty * (hx0 - hx_y);
         if (is_src) {
             const int n = c.step_counter ? *c.step_counter : c.step;
             const int j = source_sample_index(c, n);
@@ -239,20 +259,14 @@ __global__ void __launch_bounds__(TX *TY) native_de_kernel(NativeConsts c)
         }
         dz_on = true;
     }
+    const DebyeCoef k = load_coef(c.coef, cls);
     if (dx_on) c.d_prev[0][i] = dnew[0];
     if (dy_on) c.d_prev[1][i] = dnew[1];
     if (dz_on) c.d_prev[2][i] = dnew[2];
-
-    if (ex_on || eyz_on) {
-        const DebyeCoef k = load_coef(c.coef, c.mat[i]);
 #pragma unroll
-        for (int m = 0; m < 3; m++) {
-            if (m == 0 ? !ex_on : !eyz_on)
-                continue;
-            const float e0 = c.e_cur[m][i], e1 = c.e_prev[m][i];
-            c.e_prev[m][i] = debye_update(k, e0, e1, dnew[m], dn[m], dp[m]);
-        }
-    }
+    for (int m = 0; m < 3; m++)
+        if (m == 0 ? ex_on : eyz_on)
+            c.e_prev[m][i] = debye_update(k, e0[m], e1[m], dnew[m], dn[m], dp[m]);
 }
 
 // updateMurBoundary over the face cells of the native state: blockIdx.z is
@@ -340,7 +354,7 @@ bool fields_ok(const fdtd_native_fields *f, bool need_h_out)
 
 int launch_h(const NativeConsts &c, cudaStream_t s)
 {
-    const dim3 grid((c.nx + TX - 1) / TX, (c.ny + TY - 1) / TY, c.nz);
+    const dim3 grid((c.nx + TX - 1) / TX, (c.ny + TY - 1) / TY, (c.nz + H_PLANES - 1) / H_PLANES);
     native_h_kernel<<<grid, dim3(TX, TY), 0, s>>>(c);
     return launch_status();
 }
