@@ -244,6 +244,21 @@ __global__ void __launch_bounds__(TX *TY) native_de_kernel(NativeConsts c)
             hx_z = hx[i - sz];
             hy_z = hy[i - sz];
         }
+        if (is_src && c.h_edges_in) {  // a source on an upper face reads H cells outside the update ranges
+            const bool zr = z < nz - 1;
+            if (!(xi && zr)) {
+                hx_y = h_ym ? c.h_in[0][i - sy] : 0.0f;
+                hx0 = c.h_in[0][i];
+            } else if (y == ny - 1) {
+                hx0 = c.h_in[0][i];
+            }
+            if (!(yi && zr)) {
+                hy_x = h_xm ? c.h_in[1][i - 1] : 0.0f;
+                hy0 = c.h_in[1][i];
+            } else if (x == nx - 1) {
+                hy0 = c.h_in[1][i];
+            }
+        }
     }
     const int cls = (ex_on || eyz_on) ? c.mat[i] : 0;
     if (dx_on)

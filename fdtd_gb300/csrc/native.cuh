@@ -82,6 +82,9 @@ struct NativeConsts {
     // mur_value rounds it
     float mur_k[6][4];
     int mur_uniform;
+    // the D half step reads H cells that no H half step ever writes from h_in
+    // (a single-pass step: only h_in is sure to hold them)
+    int h_edges_in;
 };
 
 NativeConsts make_consts(const fdtd_plan *p, const fdtd_native_fields *f, int n);
@@ -146,6 +149,9 @@ int step_kernels(int kernel_kind, const NativeConsts &c, StepKernel *out, int ma
 // H, D, sources and E of one step in the single-pass kernel (the Mur faces
 // follow in launch_mur).
 int launch_h_de_fused(const NativeConsts &c, cudaStream_t s);
+// Whether a kernel kind's step on these arrays applies the x-face Mur updates
+// itself (NativeConsts::fuse_mur_x): not where it runs the two-pass kernels.
+bool step_fuses_mur_x(int kernel_kind, const NativeConsts &c);
 
 // Tensor maps of one single-pass launch: E^n (3), H_old (3), D^n (3),
 // D^{n-1} (3), E^{n-1} (3), material classes (1).  Compact form: R (3)

@@ -638,7 +638,7 @@ int fdtd_solver_profile(fdtd_solver *s, int nsteps, float *avg_ms, int max_kerne
         const int n = s->steps;
         NativeConsts c = solver_consts(s, n);
         c.step_counter = s->counter;
-        c.fuse_mur_x = s->kernel != FDTD_KERNEL_TWO_PASS;  // as launch_step sets it
+        c.fuse_mur_x = step_fuses_mur_x(s->kernel, c) ? 1 : 0;  // as launch_step sets it
         cudaEvent_t *e = &ev[(size_t)k * (nk + 1)];
         st = cu(cudaEventRecord(e[0], s->stream));
         for (int j = 0; j < nk && st == FDTD_OK; j++) {

@@ -1009,7 +1009,16 @@ int launch_h_de_fused(const NativeConsts &c, cudaStream_t s)
     FusedMaps maps;
     if (encode_step_maps(c, false, &maps))
         return launch_fused_impl<true, false>(a, FDTD_ZCHUNK, maps, s);
-    return launch_fused_impl<false, false>(a, FDTD_ZCHUNK, maps, s);
+    // Arrays that TMA cannot address (a caller's dense rows that are not a
+    // multiple of 16 cells, bases off 16 bytes) take the two-pass kernels: 121
+    // bytes per cell-update instead of 97, but plain coalesced loads.  us per
+    // step with the z-marching kernel fed by 4-byte cp.async, so, and with a
+    // single-pass kernel reading straight from global memory (tried, not
+    // kept): 250 x 239 x 160 324 / 202 / 191, 123 x 131 x 90 76 / 35 / 40, 498
+    // x 300 x 200 - / 604 / 575.
+    a.c.h_edges_in = 1;
+    const int st = launch_h(a.c, s);
+    return st == FDTD_OK ? launch_de(a.c, s) : st;
 }
 
 // The compact forms run the strip kernel (step_strip.cu) wherever its TMA
@@ -1051,10 +1060,15 @@ int launch_h_e_compact16(const NativeConsts &c, cudaStream_t s)
     return launch_fused_impl<false, true, true>(a, FDTD_COMPACT_ZCHUNK, maps, s);
 }
 
+bool step_fuses_mur_x(int kernel_kind, const NativeConsts &c)
+{
+    return kernel_kind != FDTD_KERNEL_TWO_PASS && (kernel_kind != FDTD_KERNEL_SINGLE_PASS || fused_uses_tma(c));
+}
+
 int launch_step(const NativeConsts &c0, cudaStream_t s)
 {
     NativeConsts c = c0;
-    c.fuse_mur_x = 1;
+    c.fuse_mur_x = step_fuses_mur_x(FDTD_KERNEL_SINGLE_PASS, c) ? 1 : 0;
     int st = launch_h_de_fused(c, s);
     if (st == FDTD_OK)
         st = launch_mur(c, s);
