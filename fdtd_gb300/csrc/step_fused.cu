@@ -638,6 +638,7 @@ __global__ void __launch_bounds__(FTX *TY) fused_step_kernel(const __grid_consta
     uint64_t *bars;
     fused_cta_setup<S, TMA, GeoOf<TY, COMPACT, R16>>(smem, &coef, &bars);
     load_coef(a.c, coef, FTX * TY);
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // the Mur kernel may be placed (it waits)
     const int bz = blockIdx.z;
     if (a.c.overlap_prev) {
         // Launched while the previous step's Mur kernel may still run.  That
@@ -817,6 +818,10 @@ int zchunk_limited(int nz, int max_planes)
 // kernel: 24) and as chosen: D form 64^3 85.6 and 10.2, 128^3 109.6 and 41.0,
 // 224 x 208 x 176 188 and 138, 256 x 239 x 160 186 and 165; compact form 64^3
 // 34.2 and 9.5, 128^3 47.9 and 31.8, 256 x 239 x 160 121.5 and 106.
+// Chunks that fill the last wave to its last CTA are not counted on (one CTA in
+// 128 is left free): with the Mur kernel's blocks between two steps such a fit
+// took a wave more (D form, 224 x 208 x 176, 5.99 waves: 152 us; the next
+// choice 140).
 // Beyond eight waves the CTAs have drifted apart, no wave ends as one, and the
 // longest chunk is as good or better (D form, 512 x 512 x 400: 1568 us with 58
 // planes, 1579 with 24).
@@ -825,6 +830,7 @@ constexpr long long MOST_WAVES = 8;
 
 int balanced_zchunk(int nz, int max_planes, long long columns, int resident)
 {
+    resident -= resident / 128;
     const int longest = zchunk_limited(nz, max_planes);
     auto chunks_of = [&](int c) { return (long long)((nz + c - 1) / c); };
     if (resident < 1 || columns * chunks_of(longest) > MOST_WAVES * resident)

@@ -26,6 +26,7 @@ __global__ void __launch_bounds__(32 * W + 32) strip_step_kernel(const __grid_co
     const int zc0 = bz * a.zchunk, zc1 = min(c.nz, zc0 + a.zchunk);
     strip_init_bars<W, S>(sm);
     strip_load_coef(c, sm.coef, G::NTH);
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // the Mur kernel may be placed (it waits)
     if (c.overlap_prev) {
         // Launched while the previous step's Mur kernel may still run (it
         // writes E at the faces and reads E at faces and their neighbours in
