@@ -434,12 +434,13 @@ class Solver:
     def dft(self, comp: int) -> np.ndarray:
         """Complex (nplanes, ny, nx) accumulator of E component comp."""
         shape = (self._dft_np, self.params.ny, self.params.nx)
-        re = np.zeros(shape, np.float64)
-        im = np.zeros(shape, np.float64)
+        # one buffer for either half: fresh pages, most of the cost of a read, are touched once
+        out, half = np.empty(shape, np.complex128), np.empty(shape, np.float64)
         P = C.POINTER(C.c_double)
-        check(lib().fdtd_solver_get_dft(self.handle, comp, re.ctypes.data_as(P), im.ctypes.data_as(P)),
-              "fdtd_solver_get_dft")
-        return re + 1j * im
+        for part, ptrs in ((out.real, (half.ctypes.data_as(P), None)), (out.imag, (None, half.ctypes.data_as(P)))):
+            check(lib().fdtd_solver_get_dft(self.handle, comp, *ptrs), "fdtd_solver_get_dft")
+            part[...] = half
+        return out
 
     def peak_sar(self, rho=None) -> tuple[float, int]:
         peak = C.c_double()
