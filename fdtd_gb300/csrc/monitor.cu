@@ -47,8 +47,13 @@ struct MonitorArgs {
     double *acc;               // re x,y,z then im x,y,z (count each)
 };
 
+// Lets the next step's kernel start beside it: that kernel reads the E this one
+// reads and writes the other slot, and its blocks at the faces wait for this
+// grid, so the step after it finds this one done.
 __global__ void __launch_bounds__(256) monitor_kernel(MonitorArgs a)
 {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int m = *a.counter;
     if (blockIdx.x == 0 && (int)threadIdx.x < a.nprobes) {
         const int k = m - a.probe_start - 1;
@@ -72,13 +77,37 @@ __global__ void __launch_bounds__(256) monitor_kernel(MonitorArgs a)
     }
     __syncthreads();
     const double c = cs[0], s = cs[1];
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < a.count; i += (size_t)gridDim.x * blockDim.x) {
-        const size_t j = a.base + row_element(i, a.nx, a.pitch);
+    // Bound by HBM: 12 bytes of E read and 48 of sums read and written per cell.
+    // All loads of a cell before its first store, and its row found by counting
+    // on instead of by a division: a pass added 162 us to a step on 224 x 208 x
+    // 176, so 145 (217 x 253 x 181: 214 and 179).  The FP64 pipe is 85 % busy with
+    // the sums and the conversions of E; converting by integer operations instead
+    // ran slower (153 us against 145 for the kernel alone).
+    const size_t stride = (size_t)gridDim.x * blockDim.x, first = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const size_t rows = stride / a.nx;
+    const unsigned xs = (unsigned)(stride - rows * a.nx);
+    size_t row = first / a.nx;
+    unsigned x = (unsigned)(first - row * a.nx);
+    for (size_t i = first; i < a.count; i += stride) {
+        const size_t j = a.base + row * a.pitch + x;
+        float e[3];
+        double re[3], im[3];
 #pragma unroll
         for (int comp = 0; comp < 3; comp++) {
-            const double e = a.e[comp][j];
-            a.acc[comp * a.count + i] += e * c;
-            a.acc[(3 + comp) * a.count + i] += e * s;
+            e[comp] = a.e[comp][j];
+            re[comp] = a.acc[comp * a.count + i];
+            im[comp] = a.acc[(3 + comp) * a.count + i];
+        }
+#pragma unroll
+        for (int comp = 0; comp < 3; comp++) {
+            a.acc[comp * a.count + i] = re[comp] + (double)e[comp] * c;
+            a.acc[(3 + comp) * a.count + i] = im[comp] + (double)e[comp] * s;
+        }
+        row += rows;
+        x += xs;
+        if (x >= a.nx) {
+            x -= a.nx;
+            row++;
         }
     }
 }
@@ -131,7 +160,12 @@ __global__ void __launch_bounds__(256) sar_kernel(SarArgs a)
     }
 }
 
-int monitor_blocks() { return 152 * 8; }
+int sar_blocks() { return 152 * 8; }
+
+// Blocks of a DFT pass: us per step with a pass after every step at 3 / 5 / 6 / 8
+// blocks per SM 241 / 238 / 257 / 249 (224 x 208 x 176, compact form; 94 without)
+// and 307 / 295 / 329 / 307 (217 x 253 x 181; 117).
+int dft_blocks() { return 152 * 5; }
 
 // Slot of the latest / previous E and D after `count` completed steps.
 int latest_slot(int count) { return count > 0 ? ((count - 1) & 1) : 0; }
@@ -164,7 +198,13 @@ int launch_monitor(fdtd_solver *s, int n)
     a.nx = s->nx;
     a.pitch = s->pitch;
     a.acc = s->d_dft;
-    monitor_kernel<<<s->dft_on ? monitor_blocks() : 1, 256, 0, s->stream>>>(a);
+    // Probes alone: one block, placed while the Mur kernel runs.  The many
+    // blocks of a DFT pass are launched plainly: placed early they lost more of
+    // the step that follows them (268 us per step instead of 249, 8 blocks per
+    // SM on 224 x 208 x 176) than the launch costs.
+    if (!s->dft_on)
+        return launch_pdl(monitor_kernel, dim3(1), dim3(256), s->stream, a);
+    monitor_kernel<<<dft_blocks(), 256, 0, s->stream>>>(a);
     return cu(cudaGetLastError());
 }
 
@@ -293,7 +333,7 @@ int fdtd_solver_peak_sar(fdtd_solver *s, const float *rho, double *peak, long lo
         a.sigma[k] = s->specs[4 * k];
         a.inv_2rho[k] = 0.5f / r;
     }
-    const int nb = monitor_blocks();
+    const int nb = sar_blocks();
     double *bm = nullptr;
     st = cu(cudaMalloc(&bm, (sizeof(double) + sizeof(long long)) * nb));
     if (st != FDTD_OK)

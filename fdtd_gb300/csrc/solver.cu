@@ -92,8 +92,8 @@ int enqueue_step(fdtd_solver *s, int n)
     NativeConsts c = solver_consts(s, n);
     c.step_counter = s->counter;
     // in a graph the step's first kernel follows the previous step's Mur
-    // kernel unless a monitor kernel runs between them
-    c.overlap_prev = s->nprobes == 0 && !s->dft_on;
+    // kernel, or a monitor kernel that ran behind it
+    c.overlap_prev = 1;
     int st;
     if (s->kernel == FDTD_KERNEL_SINGLE_PASS) {
         st = launch_step(c, s->stream);
