@@ -158,21 +158,31 @@ __device__ __forceinline__ size_t r16_word(const NativeConsts &c, int z, int bx,
     return ((size_t)z * r16_segments(c.nx) + bx) * r16_rows(c.ny) + y;
 }
 
-// One work unit: the column tile (bx, by) and z chunk bz of one solve.  The
-// stage ring and its barriers continue from earlier units of the same CTA:
-// g0 counts the planes this CTA has staged before.  Returns false when a
-// bounded wait gave up (the error flag is set; the CTA must stop).  stall
-// (read by thread 0 only): leave the second plane's copies unissued.
-template <int TY, int S, bool TMA, bool COMPACT = false, bool R16 = false>
-__device__ __forceinline__ bool fused_unit(const NativeConsts &c, const FusedMaps &maps, int zchunk, int bx, int by,
+// MOVER (TMA only): the planes are moved by a warp of its own behind the TY cell
+// warps; else thread 0 refills a stage behind the barrier at its plane's end.
+// The batched D form runs with a moving warp (20 solves of 48-256 cells per axis
+// 668 us per step without, 632 with; of 24-128 150 and 135); the single solve
+// without (512 x 512 x 400: 1559 us, with 1598; 224 x 208 x 176: 139, 141; why a
+// grid that fills the device with equal CTAs loses is not established).
+template <int TY, bool MOVER>
+__host__ __device__ constexpr int fused_threads() { return FTX * (TY + (MOVER ? 1 : 0)); }
+
+// One work unit: the column tile (bx, by) and z chunk bz of one solve.  When a
+// bounded wait gives up the error flag is set and the unit ends.  stall (read
+// by the issuing thread only): leave the second plane's copies unissued.
+template <int TY, int S, bool TMA, bool MOVER, bool COMPACT, bool R16>
+__device__ __forceinline__ void fused_unit(const NativeConsts &c, const FusedMaps &maps, int zchunk, int bx, int by,
                                            int bz, unsigned char *smem, const DebyeCoef *coef, uint64_t *bars,
-                                           unsigned g0, bool stall = false)
+                                           bool stall = false)
 {
     static_assert(COMPACT || !R16, "16-bit R is a compact-form layout");
+    static_assert(TMA || !MOVER, "a moving warp issues TMA loads");
     constexpr int NT = COMPACT ? 3 : 9, TB = R16 ? 2 : 4, XB = R16 ? TY * 4 : 0;
     using G = Geo<TY, NT, TB, XB>;
     const int nx = c.nx, ny = c.ny, nz = c.nz;
-    const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * FTX + tx;
+    // the row by a shuffle: known as uniform over the warp (see strip_unit.cuh)
+    const int tx = threadIdx.x, ty = MOVER ? __shfl_sync(0xffffffffu, (int)threadIdx.y, 0) : (int)threadIdx.y;
+    const int tid = ty * FTX + tx;
     const int x0 = bx * FTX, y0 = by * TY;
     const int x = x0 + tx, y = y0 + ty;
     const int zc0 = bz * zchunk, zc1 = min(nz, zc0 + zchunk);
@@ -180,12 +190,41 @@ __device__ __forceinline__ bool fused_unit(const NativeConsts &c, const FusedMap
     const int nplanes = plast - p0 + 1;
 
     float *hn = reinterpret_cast<float *>(smem + S * G::STAGE);
-    auto stage = [&](int k) { return smem + ((g0 + k) % S) * G::STAGE; };
-    auto bar = [&](int k) { return smem_addr(&bars[(g0 + k) % S]); };
-    auto parity = [&](int k) { return ((g0 + k) / S) & 1u; };
+    auto stage = [&](int k) { return smem + (k % S) * G::STAGE; };
+    auto bar = [&](int k) { return smem_addr(&bars[k % S]); };
+    auto parity = [&](int k) { return (uint32_t)((k / S) & 1); };
+    // with a moving warp: S barriers on which the cell warps give a stage back, and the stop word
+    auto consumed_bar = [&](int k) { return smem_addr(&bars[S + k % S]); };
+    volatile int *stop = reinterpret_cast<volatile int *>(&bars[2 * S]);
+
+    if constexpr (MOVER) {
+        if (ty == TY) {
+            if (tx == 0) {
+                auto issue = [&](int k, bool arm_only) {
+                    const int z = p0 + k;
+                    issue_plane_tma<TY, NT, TB, XB>(maps, stage(k), bar(k), plane_kind(z, zc0, zc1), x0, y0, z, arm_only);
+                };
+                for (int k = 0; k < S && k < nplanes; k++)
+                    issue(k, stall && k == 1);
+                for (int k = 0; p0 + k < zc1; k++) {
+                    if (!mbar_wait(consumed_bar(k), parity(k)) || *stop) {
+                        // a bounded wait gave up: the copies in flight land (bounded)
+                        for (int j = k; j < nplanes && j < k + S; j++)
+                            mbar_wait(bar(j), parity(j));
+                        break;
+                    }
+                    if (k + S < nplanes) {
+                        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                        issue(k + S, false);
+                    }
+                }
+            }
+            return;
+        }
+    }
 
     // prologue: fill the ring
-    for (int k = 0; k < S; k++) {
+    for (int k = 0; k < S && !MOVER; k++) {
         if (k < nplanes) {
             const int z = p0 + k;
             if (TMA) {
@@ -249,41 +288,65 @@ __device__ __forceinline__ bool fused_unit(const NativeConsts &c, const FusedMap
         mat_next = c.mat[(size_t)zc0 * plane + col];
 
     // a bounded wait gave up: raise the error flag, let the copies in flight
-    // land (bounded) and leave; called by every thread after one CTA-wide
-    // decision, so no thread is left at a barrier
-    auto give_up = [&](int k) {
-        if (tid == 0) {
-            atomicExch(c.err, 1);
-            for (int j = k; j < nplanes && j < k + S; j++)
-                mbar_wait(bar(j), parity(j));
-        }
-        __syncthreads();
+    // land (bounded; the moving warp does, once told) and leave; called by every
+    // cell thread after one decision of all of them, so no thread is left at a
+    // barrier
+    auto consumed = [&](int slot) {  // this warp is done with the plane in ring stage `slot`
+        __syncwarp();
+        if (tx == 0)
+            mbar_arrive(smem_addr(&bars[S + slot]));
     };
-    for (int k = 0; k < nplanes; k++) {
+    auto give_up = [&](int k) {
+        if (tid == 0)
+            atomicExch(c.err, 1);
+        if constexpr (MOVER) {
+            if (tid == 0)
+                *stop = 1;
+            consumed(k);
+        } else {
+            if (tid == 0)
+                for (int j = k; j < nplanes && j < k + S; j++)
+                    mbar_wait(bar(j), parity(j));
+            __syncthreads();
+        }
+    };
+    auto any = [&](bool v) {
+        if constexpr (MOVER)
+            return cells_barrier_or<FTX * TY>(v);
+        else
+            return __syncthreads_or(v) != 0;
+    };
+    int slot = 0, next = 1;   // ring stages of planes k and k + 1 (S > 1)
+    uint32_t phase_next = 0;  // barrier phase of plane k + 1
+    for (int k = 0; p0 + k < zc1; k++, slot = next, next = next + 1 == S ? 0 : next + 1, phase_next ^= next == 0) {
         const int z = p0 + k;
-        if (z >= zc1)
-            break;
+        unsigned char *stage_k = smem + slot * G::STAGE;
+        unsigned char *stage_n = smem + next * G::STAGE;
         // planes k and k+1 resident
         bool ok = true;
         if (TMA) {
             if (k == 0)
                 ok = mbar_wait(bar(0), parity(0));
             if (ok && k + 1 < nplanes)
-                ok = mbar_wait(bar(k + 1), parity(k + 1));
+                ok = mbar_wait(smem_addr(&bars[next]), phase_next);
             // the CTA decides at its next barrier (below): until then it only
             // reads shared memory
         } else {
             cp_async_wait<S - 2>();
             __syncthreads();
         }
-        const float *EA = reinterpret_cast<const float *>(stage(k) + G::OFF_E);
-        const float *EB = reinterpret_cast<const float *>(stage(k + 1) + G::OFF_E);
-        const float *HA = reinterpret_cast<const float *>(stage(k) + G::OFF_H);
+        const float *EA = reinterpret_cast<const float *>(stage_k + G::OFF_E);
+        const float *EB = reinterpret_cast<const float *>(stage_n + G::OFF_E);
+        const float *HA = reinterpret_cast<const float *>(stage_k + G::OFF_H);
         constexpr int ES = pad128(G::E_BYTES) / 4, HS = pad128(G::H_BYTES) / 4, TS = pad128(G::T_BYTES) / 4;
         auto ea = [&](int comp, int r, int cc) { return EA[comp * ES + r * G::EW + cc]; };
         auto eb = [&](int comp, int r, int cc) { return EB[comp * ES + r * G::EW + cc]; };
         auto ha = [&](int comp, int r, int cc) { return HA[comp * HS + r * G::HW + cc]; };
-        auto hnr = [&](int comp, int r, int cc) -> float & { return hn[(comp * G::HNH + r) * G::HNW + cc]; };
+        // with a moving warp two sets, taken in turn: a warp writes a plane's set
+        // again two planes later, behind a barrier that every warp reaches after
+        // reading it
+        float *hnk = MOVER ? hn + (k & 1) * (G::HN_BYTES / 4) : hn;
+        auto hnr = [&](int comp, int r, int cc) -> float & { return hnk[(comp * G::HNH + r) * G::HNW + cc]; };
 
         const bool zlo = z < nz - 1, zmid = z >= 1 && z < nz - 1;
         // ---- H^{n+1/2} at plane z, own cell (fdtd_calculations.cu:43-76)
@@ -343,9 +406,9 @@ __device__ __forceinline__ bool fused_unit(const NativeConsts &c, const FusedMap
                 hnr(2, 0, tx + 1) = v;
             }
             if (TMA) {
-                if (__syncthreads_or(!ok)) {
-                    give_up(k);
-                    return false;
+                if (any(!ok)) {
+                    give_up(MOVER ? slot : k);
+                    return;
                 }
             } else {
                 __syncthreads();
@@ -362,12 +425,12 @@ __device__ __forceinline__ bool fused_unit(const NativeConsts &c, const FusedMap
                 uint32_t w;
                 if constexpr (R16) {
                     if (TMA) {
-                        const unsigned short *T = reinterpret_cast<const unsigned short *>(stage(k) + G::OFF_T);
+                        const unsigned short *T = reinterpret_cast<const unsigned short *>(stage_k + G::OFF_T);
                         constexpr int TS16 = pad128(G::T_BYTES) / 2;
                         q0 = T[t];
                         q1 = T[TS16 + t];
                         q2 = T[2 * TS16 + t];
-                        w = reinterpret_cast<const uint32_t *>(stage(k) + G::OFF_X)[ty];
+                        w = reinterpret_cast<const uint32_t *>(stage_k + G::OFF_X)[ty];
                     } else {
                         q0 = reinterpret_cast<const unsigned short *>(c.d_cur[0])[i];
                         q1 = reinterpret_cast<const unsigned short *>(c.d_cur[1])[i];
@@ -375,14 +438,14 @@ __device__ __forceinline__ bool fused_unit(const NativeConsts &c, const FusedMap
                         w = c.r_exp[r16_word(c, z, bx, y)];
                     }
                 } else {
-                    const float *T = reinterpret_cast<const float *>(stage(k) + G::OFF_T);
+                    const float *T = reinterpret_cast<const float *>(stage_k + G::OFF_T);
                     r0 = T[0 * TS + t];
                     r1 = T[1 * TS + t];
                     r2 = T[2 * TS + t];
                 }
                 uint8_t cls;
                 if (TMA) {
-                    cls = (stage(k) + G::OFF_M)[t];
+                    cls = (stage_k + G::OFF_M)[t];
                 } else {
                     cls = mat_next;
                     if (z + 1 < zc1)
@@ -479,14 +542,14 @@ __device__ __forceinline__ bool fused_unit(const NativeConsts &c, const FusedMap
             } else {
             if (in_dom) {
                 const size_t i = (size_t)z * plane + col;
-                const float *T = reinterpret_cast<const float *>(stage(k) + G::OFF_T);
+                const float *T = reinterpret_cast<const float *>(stage_k + G::OFF_T);
                 const int t = ty * FTX + tx;
                 const float dn0 = T[0 * TS + t], dn1 = T[1 * TS + t], dn2 = T[2 * TS + t];
                 const float dp0 = T[3 * TS + t], dp1 = T[4 * TS + t], dp2 = T[5 * TS + t];
                 const float ep0 = T[6 * TS + t], ep1 = T[7 * TS + t], ep2 = T[8 * TS + t];
                 uint8_t cls;
                 if (TMA) {
-                    cls = (stage(k) + G::OFF_M)[t];
+                    cls = (stage_k + G::OFF_M)[t];
                 } else {
                     cls = mat_next;
                     if (z + 1 < zc1)
@@ -565,12 +628,16 @@ __device__ __forceinline__ bool fused_unit(const NativeConsts &c, const FusedMap
             hym = hyn;
         }
         if (TMA && z < zc0) {  // the chunk prologue plane has no other decision point
-            if (__syncthreads_or(!ok)) {
-                give_up(k);
-                return false;
+            if (any(!ok)) {
+                give_up(MOVER ? slot : k);
+                return;
             }
-        } else {
+        } else if (!MOVER) {
             __syncthreads();  // stage k and hn fully consumed
+        }
+        if constexpr (MOVER) {
+            consumed(slot);
+            continue;
         }
         // refill the stage of plane k with plane k + S
         const int kn = k + S;
@@ -590,30 +657,34 @@ __device__ __forceinline__ bool fused_unit(const NativeConsts &c, const FusedMap
     }
     if (!TMA)
         cp_async_wait<0>();
-    return true;
 }
 
-// Shared-memory layout of a CTA: S stages, the H^{n+1/2} plane, S barriers,
-// then the class table (the launch sizes it for the solve's classes, so a
+// Shared-memory layout of a CTA: S stages, the H^{n+1/2} plane, S full and S
+// consumed barriers and the stop word, then the class table (the launch sizes it for the solve's classes, so a
 // small table leaves room for more resident CTAs).
 template <int S>
-__host__ __device__ constexpr int bars_bytes() { return (S * 8 + 15) & ~15; }
+__host__ __device__ constexpr int bars_bytes() { return (2 * S * 8 + 4 + 15) & ~15; }
 
+// hn sets: two with a moving warp, else one
 template <int S, class G>
-__host__ __device__ constexpr int fused_smem_bytes(int nclasses)
+__host__ __device__ constexpr int fused_smem_bytes(int nclasses, bool mover)
 {
-    return 128 + S * G::STAGE + G::HN_BYTES + bars_bytes<S>() + nclasses * (int)sizeof(DebyeCoef);
+    return 128 + S * G::STAGE + (mover ? 2 : 1) * G::HN_BYTES + bars_bytes<S>() + nclasses * (int)sizeof(DebyeCoef);
 }
 
-template <int S, bool TMA, class G>
+template <int TY, int S, bool TMA, bool MOVER, class G>
 __device__ __forceinline__ void fused_cta_setup(unsigned char *smem, DebyeCoef **coef, uint64_t **bars)
 {
-    *bars = reinterpret_cast<uint64_t *>(smem + S * G::STAGE + G::HN_BYTES);
-    *coef = reinterpret_cast<DebyeCoef *>(smem + S * G::STAGE + G::HN_BYTES + bars_bytes<S>());
+    unsigned char *b = smem + S * G::STAGE + (MOVER ? 2 : 1) * G::HN_BYTES;
+    *bars = reinterpret_cast<uint64_t *>(b);
+    *coef = reinterpret_cast<DebyeCoef *>(b + bars_bytes<S>());
     const int tid = threadIdx.y * FTX + threadIdx.x;
     if (TMA && tid == 0) {
-        for (int s = 0; s < S; s++)
+        for (int s = 0; s < S; s++) {
             mbar_init(smem_addr(&(*bars)[s]), 1);
+            mbar_init(smem_addr(&(*bars)[S + s]), TY);
+        }
+        *reinterpret_cast<int *>(&(*bars)[2 * S]) = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
 }
@@ -636,7 +707,7 @@ __global__ void __launch_bounds__(FTX *TY) fused_step_kernel(const __grid_consta
     unsigned char *smem = smem_raw + ((128 - (smem_addr(smem_raw) & 127)) & 127);
     DebyeCoef *coef;
     uint64_t *bars;
-    fused_cta_setup<S, TMA, GeoOf<TY, COMPACT, R16>>(smem, &coef, &bars);
+    fused_cta_setup<TY, S, TMA, false, GeoOf<TY, COMPACT, R16>>(smem, &coef, &bars);
     load_coef(a.c, coef, FTX * TY);
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // the Mur kernel may be placed (it waits)
     const int bz = blockIdx.z;
@@ -660,8 +731,7 @@ __global__ void __launch_bounds__(FTX *TY) fused_step_kernel(const __grid_consta
     if (TMA && a.c.stall_once && blockIdx.x == 0 && blockIdx.y == 0 && bz == 0 && threadIdx.x == 0 &&
         threadIdx.y == 0)
         stall = atomicExch(a.c.stall_once, 0) != 0;
-    fused_unit<TY, S, TMA, COMPACT, R16>(a.c, maps, a.zchunk, blockIdx.x, blockIdx.y, bz, smem, coef, bars, 0u,
-                                         stall);
+    fused_unit<TY, S, TMA, false, COMPACT, R16>(a.c, maps, a.zchunk, blockIdx.x, blockIdx.y, bz, smem, coef, bars, stall);
 }
 
 // Many solves: one CTA per work unit (the grid is the batch's work list); the
@@ -674,7 +744,7 @@ __global__ void __launch_bounds__(FTX *TY) fused_step_kernel(const __grid_consta
 // persistent form: the 64-solve workload ran 4.8 % faster than with 5; with
 // 16-bit R 11 % faster than with 3 or 5).
 template <int TY, int S, bool COMPACT, bool R16 = false>
-__global__ void __launch_bounds__(FTX *TY, COMPACT ? 4 : 3) batch_step_kernel(const BatchDesc *__restrict__ descs,
+__global__ void __launch_bounds__((fused_threads<TY, !COMPACT>()), COMPACT ? 4 : 3) batch_step_kernel(const BatchDesc *__restrict__ descs,
                                                                              const BatchUnit *__restrict__ units)
 {
     extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -686,21 +756,22 @@ __global__ void __launch_bounds__(FTX *TY, COMPACT ? 4 : 3) batch_step_kernel(co
         return;
     DebyeCoef *coef;
     uint64_t *bars;
-    fused_cta_setup<S, true, GeoOf<TY, COMPACT, R16>>(smem, &coef, &bars);
+    fused_cta_setup<TY, S, true, !COMPACT, GeoOf<TY, COMPACT, R16>>(smem, &coef, &bars);
+    constexpr int NTH = fused_threads<TY, !COMPACT>();
     const int tid = threadIdx.y * FTX + threadIdx.x;
     const BatchDesc &d = descs[rec.solve];
     const int par = n & 1;
     {
         const int *src = reinterpret_cast<const int *>(&d.c[par]);
         int *dst = reinterpret_cast<int *>(&s_c);
-        for (int i = tid; i < (int)(sizeof(NativeConsts) / 4); i += FTX * TY)
+        for (int i = tid; i < (int)(sizeof(NativeConsts) / 4); i += NTH)
             dst[i] = src[i];
     }
-    load_coef(d.c[par], coef, FTX * TY);
+    load_coef(d.c[par], coef, NTH);
     __syncthreads();
     const int local = (int)blockIdx.x - d.unit_begin, per_z = d.tiles_x * d.tiles_y, rem = local % per_z;
-    fused_unit<TY, S, true, COMPACT, R16>(s_c, d.maps[par], d.zchunk, rem % d.tiles_x, rem / d.tiles_x, local / per_z,
-                                          smem, coef, bars, 0u);
+    fused_unit<TY, S, true, !COMPACT, COMPACT, R16>(s_c, d.maps[par], d.zchunk, rem % d.tiles_x, rem / d.tiles_x, local / per_z,
+                                          smem, coef, bars);
 }
 
 __global__ void __launch_bounds__(256) batch_mur_kernel(const BatchDesc *__restrict__ descs,
@@ -776,11 +847,11 @@ int launch_fused_impl(FusedArgs &a, int zmax, const FusedMaps &maps, cudaStream_
         return (int)de;
     const int so = smem_opt_in.run(dev, [&] {
         return (int)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         fused_smem_bytes<S_SEL, G>(FDTD_MAX_CLASSES));
+                                         fused_smem_bytes<S_SEL, G>(FDTD_MAX_CLASSES, false));
     });
     if (so != 0)
         return so < 0 ? FDTD_ERR_INVALID : so;
-    const int smem = fused_smem_bytes<S_SEL, G>(a.c.nclasses);
+    const int smem = fused_smem_bytes<S_SEL, G>(a.c.nclasses, false);
     static PerDeviceValue<FDTD_MAX_CLASSES + 1> resident;
     const int r = resident.get(dev, a.c.nclasses, [&] { return resident_ctas(kernel, FTX * TY_SEL, smem); });
     const int tiles_x = (a.c.nx + FTX - 1) / FTX, tiles_y = (a.c.ny + TY_SEL - 1) / TY_SEL;
@@ -955,7 +1026,11 @@ int fused_tile_height() { return TY_SEL; }
 template <bool COMPACT, bool R16 = false>
 struct BatchStep {
     static constexpr auto fn = batch_step_kernel<TY_SEL, S_SEL, COMPACT, R16>;
-    static int smem(int nclasses) { return fused_smem_bytes<S_SEL, GeoOf<TY_SEL, COMPACT, R16>>(nclasses); }
+    static constexpr int NTH = fused_threads<TY_SEL, !COMPACT>();
+    static int smem(int nclasses)
+    {
+        return fused_smem_bytes<S_SEL, GeoOf<TY_SEL, COMPACT, R16>>(nclasses, !COMPACT);
+    }
     static int opt_in()
     {
         static PerDeviceOnce<> once;
@@ -968,13 +1043,13 @@ struct BatchStep {
         });
         return so < 0 ? FDTD_ERR_INVALID : so;
     }
-    static int ctas(int nclasses) { return opt_in() == FDTD_OK ? resident_ctas(fn, FTX * TY_SEL, smem(nclasses)) : 0; }
+    static int ctas(int nclasses) { return opt_in() == FDTD_OK ? resident_ctas(fn, NTH, smem(nclasses)) : 0; }
     static int launch(const BatchLaunch &b, cudaStream_t s)
     {
         const int st = opt_in();
         if (st != FDTD_OK)
             return st;
-        fn<<<b.total_units, dim3(FTX, TY_SEL), smem(b.max_classes), s>>>(b.descs, b.units);
+        fn<<<b.total_units, dim3(FTX, NTH / FTX), smem(b.max_classes), s>>>(b.descs, b.units);
         const cudaError_t e = cudaGetLastError();
         return e == cudaSuccess ? FDTD_OK : (int)e;
     }

@@ -314,13 +314,6 @@ struct StripPlanes {
     __device__ __forceinline__ bool no_r(int z) const { return z >= zc0 && ((memless >> (z - zc0)) & 1ull) != 0; }
 };
 
-constexpr int BAR_CELLS = 1;  // named barrier of the cell warps alone
-
-__device__ __forceinline__ void mbar_arrive(uint32_t bar)
-{
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-
 // The moving warp's one lane at work: run() fills the ring, then plane by
 // plane waits until the cell warps have consumed the plane, stores the tiles
 // they have left in its stage and refills the stage.  Its waits are bounded;
@@ -375,20 +368,6 @@ struct StripMove {
         bulk_wait_all();
     }
 };
-
-// Barrier of the cell warps alone; true in every thread if any passes true.
-template <int THREADS>
-__device__ __forceinline__ bool cells_barrier_or(bool v)
-{
-    uint32_t r;
-    asm volatile(
-        "{\n .reg .pred p, q;\n setp.ne.u32 p, %1, 0;\n barrier.cta.red.or.pred q, %3, %2, p;\n"
-        " selp.u32 %0, 1, 0, q;\n}\n"
-        : "=r"(r)
-        : "r"((uint32_t)v), "n"(THREADS), "n"(BAR_CELLS)
-        : "memory");
-    return __any_sync(0xffffffffu, r != 0);  // a vote: known as uniform over the warp
-}
 
 // One work unit: column tile (bx, by), z chunk bz of one solve.  memless: bit
 // j set when plane zc0 + j of the tile holds no Debye memory.  stall: the

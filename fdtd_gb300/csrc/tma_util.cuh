@@ -73,6 +73,27 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity)
     return false;
 }
 
+constexpr int BAR_CELLS = 1;  // named barrier of the cell warps alone
+
+__device__ __forceinline__ void mbar_arrive(uint32_t bar)
+{
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+
+// Barrier of the cell warps alone; true in every thread if any passes true.
+template <int THREADS>
+__device__ __forceinline__ bool cells_barrier_or(bool v)
+{
+    uint32_t r;
+    asm volatile(
+        "{\n .reg .pred p, q;\n setp.ne.u32 p, %1, 0;\n barrier.cta.red.or.pred q, %3, %2, p;\n"
+        " selp.u32 %0, 1, 0, q;\n}\n"
+        : "=r"(r)
+        : "r"((uint32_t)v), "n"(THREADS), "n"(BAR_CELLS)
+        : "memory");
+    return __any_sync(0xffffffffu, r != 0);  // a vote: known as uniform over the warp
+}
+
 __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap *map, int x, int y, int z, uint32_t bar)
 {
     asm volatile(
