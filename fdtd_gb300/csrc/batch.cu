@@ -291,7 +291,10 @@ int rebuild(fdtd_batch *b)
         std::memset(&d, 0, sizeof d);
         for (int par = 0; par < 2; par++) {
             d.c[par] = solve_consts(v, par, b->d_work + BATCH_ERR_WORD);
-            d.c[par].fuse_mur_x = strip ? 1 : 0;  // the strip kernel applies the x-face Mur updates
+            // the step kernel applies the x-face Mur updates (D form, 20 solves of
+            // 48-256 cells per axis: 605 us per step, 631 with the strided faces
+            // in the Mur launch; of 24-128: 131 and 136)
+            d.c[par].fuse_mur_x = 1;
             if (strip ? !strip::encode_strip_maps(d.c[par], b->r16, ty, &d.smaps[par])
                       : !encode_step_maps(d.c[par], b->compact, &d.maps[par], b->r16))
                 return FDTD_ERR_INVALID;
