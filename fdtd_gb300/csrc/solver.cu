@@ -434,29 +434,33 @@ int fdtd_solver_create(const fdtd_solver_config *cfg, fdtd_solver **out)
         s->specs.assign(cfg->specs, cfg->specs + 4 * (size_t)ncls);
         s->material_hash = mhash;  // checkpoints must come from the same class volume
     }
+    unsigned long long memless_cells = 0;
     if (st == FDTD_OK && stores_no_d(cfg->kernel)) {
         // tile-planes without Debye memory: the strip kernel skips their R
-        const std::vector<unsigned char> flags =
-            strip_plane_flags(cfg->material, p->nx, p->ny, p->nz, p->nx, cfg->specs, ncls);
-        s->memless_rows = strip_shape_rows(strip_single_shape(cfg->kernel == FDTD_KERNEL_COMPACT_R16));
-        const int zchunk = strip_solve_zchunk(p->nx, p->ny, p->nz, r16, ncls);
-        s->memless_zchunk = zchunk;
-        std::vector<unsigned long long> masks((size_t)((p->nz + zchunk - 1) / zchunk) *
-                                              ((p->ny + s->memless_rows - 1) / s->memless_rows) * ((p->nx + 31) / 32));
-        s->memless_fraction =
-            strip_unit_masks(flags, p->nx, p->ny, p->nz, s->memless_rows, zchunk, masks.data());
-        if (s->memless_fraction > 0.0) {
-            st = cu(cudaMalloc(&s->d_memless, masks.size() * sizeof(unsigned long long)));
-            if (st == FDTD_OK)
-                st = cu(cudaMemcpyAsync(s->d_memless, masks.data(), masks.size() * sizeof(unsigned long long),
-                                        cudaMemcpyHostToDevice, s->stream));
-        }
+        s->memless_rows = strip_shape_rows(strip_single_shape(r16));
+        s->memless_zchunk = strip_solve_zchunk(p->nx, p->ny, p->nz, r16, ncls);
+        const size_t units = (size_t)((p->nz + s->memless_zchunk - 1) / s->memless_zchunk) *
+                             ((p->ny + s->memless_rows - 1) / s->memless_rows) * ((p->nx + 31) / 32);
+        st = cu(cudaMalloc(&s->d_memless, (units + 1) * sizeof(unsigned long long)));
+        if (st == FDTD_OK)
+            st = cu(cudaMemsetAsync(s->d_memless + units, 0, sizeof(unsigned long long), s->stream));
+        if (st == FDTD_OK)
+            st = strip_unit_masks_device(s->mat, p->nx, p->ny, p->nz, s->pitch, cfg->specs, ncls, s->memless_rows,
+                                         s->memless_zchunk, s->d_memless, s->d_memless + units, s->stream);
+        if (st == FDTD_OK)
+            st = cu(cudaMemcpyAsync(&memless_cells, s->d_memless + units, sizeof memless_cells, cudaMemcpyDeviceToHost,
+                                    s->stream));
     }
     if (st == FDTD_OK)
         st = cu(cudaStreamSynchronize(s->stream));
     if (st != FDTD_OK) {
         fdtd_solver_destroy(s);
         return st;
+    }
+    s->memless_fraction = (double)memless_cells / (double)n;
+    if (s->d_memless && memless_cells == 0) {
+        cudaFree(s->d_memless);
+        s->d_memless = nullptr;
     }
     s->writer = std::thread(writer_main, s);
     *out = s;

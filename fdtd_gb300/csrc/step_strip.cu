@@ -282,6 +282,60 @@ double strip_unit_masks(const std::vector<unsigned char> &flags, int nx, int ny,
     return cells / ((double)nx * ny * nz);
 }
 
+namespace strip {
+namespace {
+
+// One bit per class: no relaxation (tau = 0).
+struct ClassBits {
+    uint32_t w[FDTD_MAX_CLASSES / 32];
+};
+
+// strip_unit_masks on the device: block (bx, by, bz) of 256 threads makes the
+// mask of its unit, and the cells on its memoryless planes are added up.
+__global__ void __launch_bounds__(256) unit_masks_kernel(const uint8_t *__restrict__ mat, int nx, int ny, int nz,
+                                                         int pitch, int ty, int zchunk, ClassBits bits,
+                                                         unsigned long long *__restrict__ masks,
+                                                         unsigned long long *__restrict__ cells)
+{
+    const int x0 = blockIdx.x * SX, y0 = blockIdx.y * ty, zc0 = blockIdx.z * zchunk, zc1 = min(nz, zc0 + zchunk);
+    const int x = x0 + threadIdx.x % SX;
+    __shared__ uint32_t table[FDTD_MAX_CLASSES / 32];
+    if (threadIdx.x < FDTD_MAX_CLASSES / 32)
+        table[threadIdx.x] = bits.w[threadIdx.x];
+    __syncthreads();
+    unsigned long long m = 0;
+    for (int z = zc0; z < zc1; z++) {
+        bool ok = true;
+        for (int y = y0 + threadIdx.x / SX; y < min(ny, y0 + ty); y += 256 / SX)
+            if (x < nx) {
+                const int cls = mat[((size_t)z * ny + y) * pitch + x];
+                ok &= ((table[cls >> 5] >> (cls & 31)) & 1u) != 0;
+            }
+        if (__syncthreads_and(ok))
+            m |= 1ull << (z - zc0);
+    }
+    if (threadIdx.x == 0) {
+        masks[((size_t)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x] = m;
+        atomicAdd(cells, (unsigned long long)__popcll(m) * (min(nx, x0 + SX) - x0) * (min(ny, y0 + ty) - y0));
+    }
+}
+
+}  // namespace
+}  // namespace strip
+
+int strip_unit_masks_device(const uint8_t *mat, int nx, int ny, int nz, int pitch, const float *specs, int nclasses,
+                            int ty, int zchunk, unsigned long long *masks, unsigned long long *cells, cudaStream_t s)
+{
+    strip::ClassBits bits{};
+    for (int k = 0; k < nclasses && k < FDTD_MAX_CLASSES; k++)
+        if (specs[4 * k + 3] == 0.0f)
+            bits.w[k >> 5] |= 1u << (k & 31);
+    const dim3 grid((nx + strip::SX - 1) / strip::SX, (ny + ty - 1) / ty, (nz + zchunk - 1) / zchunk);
+    strip::unit_masks_kernel<<<grid, 256, 0, s>>>(mat, nx, ny, nz, pitch, ty, zchunk, bits, masks, cells);
+    const cudaError_t e = cudaGetLastError();
+    return e == cudaSuccess ? FDTD_OK : (int)e;
+}
+
 bool strip_usable(const NativeConsts &c, bool r16)
 {
     StripMaps maps;
