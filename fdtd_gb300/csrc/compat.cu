@@ -2,7 +2,7 @@
 //
 // Same argument lists and per-component index ranges as the reference's five
 // kernels, over the reference's float material arrays and three-slot state.
-// The grids differ: 32 x 8 thread tiles (of several z planes for H and D)
+// The grids differ: 64 x 2 thread tiles (of several z planes for H and D)
 // instead of 128 x 1 rows, sources as one warp instead of a full grid, Mur over
 // the face cells only.  The kernels are programmatic dependents of the stream's
 // previous launch: one after another on a small grid they took 4.2-5.4 us each,
@@ -42,7 +42,10 @@ int current_device_checked(int *dev)
     return FDTD_OK;
 }
 
-constexpr int TX = 32, TY = 8;
+// Thread tile: long rows share their 32-byte sectors and E and H neighbours within
+// a block (five launchers on 256 x 256 x 200: 343 us with 32 x 8, 338 with 64 x 2, 335
+// with 256 x 1, which leaves most threads of a narrow grid idle)
+constexpr int TX = 64, TY = 2;
 
 // z planes per thread of the H and D kernels, bound by HBM (36 bytes per cell).
 // With one plane per thread, each component loaded, updated and stored in
@@ -58,14 +61,15 @@ __global__ void __launch_bounds__(TX *TY) compat_h_kernel(float *__restrict__ hx
 {
     pdl_begin();
     const int nx = c_sym.nx, ny = c_sym.ny, nz = c_sym.nz;
-    const int x = blockIdx.x * TX + threadIdx.x, y = blockIdx.y * TY + threadIdx.y;
+    const TileXY t(nx, TX, TY);
+    const int x = t.x0 + threadIdx.x, y = t.y0 + threadIdx.y;
     if (x >= nx - 1 || y >= ny - 1)
         return;
     const float dt = c_sym.dt, mu0 = c_sym.mu0;
     const float kx = dt / (mu0 * c_sym.dx), ky = dt / (mu0 * c_sym.dy), kz = dt / (mu0 * c_sym.dz);
     const float *const in[3] = {hx, hy, hz};
     float *const out[3] = {hx, hy, hz};
-    h_column<H_PLANES>(x, y, blockIdx.z * H_PLANES, nx, ny, nz, nx, kx, ky, kz, ex, ey, ez, in, out);
+    h_column<H_PLANES>(x, y, blockIdx.y * H_PLANES, nx, ny, nz, nx, kx, ky, kz, ex, ey, ez, in, out);
 }
 
 __global__ void __launch_bounds__(TX *TY) compat_d_kernel(float *__restrict__ dxT, float *__restrict__ dyT,
@@ -77,7 +81,8 @@ __global__ void __launch_bounds__(TX *TY) compat_d_kernel(float *__restrict__ dx
     pdl_begin();
     constexpr int K = D_PLANES;
     const int nx = c_sym.nx, ny = c_sym.ny, nz = c_sym.nz;
-    const int x = blockIdx.x * TX + threadIdx.x, y = blockIdx.y * TY + threadIdx.y, z0 = blockIdx.z * K;
+    const TileXY t(nx, TX, TY);
+    const int x = t.x0 + threadIdx.x, y = t.y0 + threadIdx.y, z0 = blockIdx.y * K;
     if (x >= nx - 1 || y >= ny - 1)
         return;  // no D component is updated at x = nx-1, y = ny-1 or z = nz-1
     const int n = min(K, nz - 1 - z0);
@@ -138,7 +143,8 @@ __global__ void __launch_bounds__(TX *TY) compat_e_kernel(ETriplet a, const floa
 {
     pdl_begin();
     const int nx = c_sym.nx, ny = c_sym.ny, nz = c_sym.nz;
-    const int x = blockIdx.x * TX + threadIdx.x, y = blockIdx.y * TY + threadIdx.y, z = blockIdx.z;
+    const TileXY t(nx, TX, TY);
+    const int x = t.x0 + threadIdx.x, y = t.y0 + threadIdx.y, z = blockIdx.y;
     if (x >= nx || y >= ny)
         return;
     // ex: x 0..nx-2, y 1..ny-2, z 1..nz-2; ey, ez: x 1..nx-1, y 0..ny-1, z 1..nz-1 (:147-175)
@@ -218,10 +224,7 @@ int prologue(SymbolBlock *sym)
 }
 
 // The cells in columns of `planes` z planes.
-dim3 cell_grid(const SymbolBlock &s, int planes)
-{
-    return dim3((s.nx + TX - 1) / TX, (s.ny + TY - 1) / TY, (s.nz + planes - 1) / planes);
-}
+dim3 cell_grid(const SymbolBlock &s, int planes) { return tile_grid(s.nx, s.ny, s.nz, TX, TY, planes); }
 
 }  // namespace
 }  // namespace fdtd

@@ -12,6 +12,23 @@ __host__ __device__ inline size_t cell_index(int x, int y, int z, int nx, int ny
     return ((size_t)z * (size_t)ny + (size_t)y) * (size_t)nx + (size_t)x;
 }
 
+// Tile of a block in a grid of (tiles in x * tiles in y, z) blocks, x fastest:
+// flat, as gridDim.y's limit of 65535 is too low for tiles of a few rows.
+struct TileXY {
+    int x0, y0;
+    __device__ __forceinline__ TileXY(int nx, int tx, int ty)
+    {
+        const unsigned tiles = (unsigned)(nx + tx - 1) / tx, by = blockIdx.x / tiles;
+        x0 = (int)(blockIdx.x - by * tiles) * tx;
+        y0 = (int)by * ty;
+    }
+};
+
+inline dim3 tile_grid(int nx, int ny, int nz, int tx, int ty, int tz)
+{
+    return dim3((unsigned)((nx + tx - 1) / tx) * (unsigned)((ny + ty - 1) / ty), (unsigned)((nz + tz - 1) / tz));
+}
+
 // Programmatic dependent launch: lets the next launch's blocks be placed while
 // this grid finishes, and (before any access to memory) waits for the previous
 // grid to complete.  A stream's order is kept: every kernel launched this way

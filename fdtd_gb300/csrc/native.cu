@@ -162,14 +162,18 @@ __device__ __forceinline__ DebyeCoef load_coef(const DebyeCoef *__restrict__ tab
 // (they may alias), H_PLANES z planes per thread, bound by HBM (36 bytes per
 // cell): 82 us on 250 x 239 x 160 with one plane per thread and each component
 // loaded, updated and stored in turn, 61 so (5.6 TB/s); two planes: 62.
-constexpr int H_PLANES = 4;
+// Tiles of 64 x 2 threads: long rows share their sectors and E neighbours within
+// a block (512 x 300 x 200: 185 us with 32 x 8, 181 so; the D/E kernel gains
+// nothing from them).
+constexpr int H_PLANES = 4, HTX = 64, HTY = 2;
 
-__global__ void __launch_bounds__(TX *TY) native_h_kernel(NativeConsts c)
+__global__ void __launch_bounds__(HTX *HTY) native_h_kernel(NativeConsts c)
 {
-    const int x = blockIdx.x * TX + threadIdx.x, y = blockIdx.y * TY + threadIdx.y;
+    const TileXY t(c.nx, HTX, HTY);
+    const int x = t.x0 + threadIdx.x, y = t.y0 + threadIdx.y;
     if (x >= c.nx - 1 || y >= c.ny - 1)
         return;  // no H component is updated at x = nx-1, y = ny-1 or z = nz-1
-    h_column<H_PLANES>(x, y, blockIdx.z * H_PLANES, c.nx, c.ny, c.nz, c.pitch, c.kx, c.ky, c.kz, c.e_cur[0], c.e_cur[1],
+    h_column<H_PLANES>(x, y, blockIdx.y * H_PLANES, c.nx, c.ny, c.nz, c.pitch, c.kx, c.ky, c.kz, c.e_cur[0], c.e_cur[1],
                        c.e_cur[2], c.h_in, c.h_out);
 }
 
@@ -375,8 +379,7 @@ bool fields_ok(const fdtd_native_fields *f, bool need_h_out)
 
 int launch_h(const NativeConsts &c, cudaStream_t s)
 {
-    const dim3 grid((c.nx + TX - 1) / TX, (c.ny + TY - 1) / TY, (c.nz + H_PLANES - 1) / H_PLANES);
-    native_h_kernel<<<grid, dim3(TX, TY), 0, s>>>(c);
+    native_h_kernel<<<tile_grid(c.nx, c.ny, c.nz, HTX, HTY, H_PLANES), dim3(HTX, HTY), 0, s>>>(c);
     return launch_status();
 }
 

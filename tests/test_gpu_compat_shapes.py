@@ -1,10 +1,11 @@
 """The compat launchers at the edges of their launch shapes: planes below, at
 and just over the H and D kernels' planes per thread, rows and columns around
-one 32 x 8 tile, face rows around the Mur kernel's rows per thread, and calls
-queued back to back on one stream (each launch may be placed before the
-previous one has finished, and must still read what it wrote).  Against the
-FP32 oracle (the reference kernels' own arithmetic), 24 rotated steps, at the
-parity bar of every field."""
+one 64 x 2 tile, more rows than a grid has blocks in y, face rows around the
+Mur kernel's rows per thread, and calls queued back to back on one stream (each
+launch may be placed before the previous one has finished, and must still read
+what it wrote).  Against the FP32 oracle (the
+reference kernels' own arithmetic), 24 rotated steps, at the parity bar of
+every field."""
 from __future__ import annotations
 
 import ctypes as C
@@ -22,7 +23,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("dims", [(3, 3, 3), (31, 8, 4), (32, 9, 5), (33, 7, 6), (34, 16, 8), (65, 17, 9),
-                                  (130, 5, 13), (5, 131, 10)])
+                                  (130, 5, 13), (5, 131, 10), (63, 3, 5), (64, 4, 4), (3, 131074, 3)])
 def test_back_to_back_steps_match_the_oracle(cuda, dims):
     torch, (nx, ny, nz), steps = cuda, dims, 24
     codes, specs, rp, sources, consts, jz = random_case(*dims, seed=sum(dims), ncls=3, nsrc=2)
