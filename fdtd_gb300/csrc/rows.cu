@@ -4,11 +4,17 @@
 // address them; callers see dense volumes.  A strided copy
 // (cudaMemcpy2DAsync) moves short rows slowly, the more so the shorter they
 // are: 10 M floats to page-locked memory at 49 GB/s in rows of 61 and 115 in
-// rows of 217, against 186 for one contiguous copy; bytes to the device at
-// 15 - 58 GB/s against 590.  So the rows are packed by a kernel instead:
-// straight into page-locked memory (183 GB/s, the link's rate, from 152
-// blocks on), or through a device scratch area and contiguous copies (164
-// GB/s into pageable memory).
+// rows of 217; bytes to the device at 15 - 58 GB/s against 590.  So the rows
+// are packed by a kernel instead: straight into page-locked memory, or through
+// a device scratch area and contiguous copies (164 GB/s into pageable memory).
+//
+// Page-locked memory is written by the kernel for dense rows as well.  One
+// contiguous copy of 420 MB ran at 107 - 191 GB/s, from one buffer and one
+// moment to the next (now and then at a fifth of that); the kernel at 189 -
+// 191 every time, the link's rate, with 16-byte stores from 76 blocks on
+// (4-byte stores: 180 - 185).
+#include <cuda.h>
+
 #include <algorithm>
 
 #include "rows.h"
@@ -18,16 +24,50 @@ namespace {
 
 constexpr int PACK_THREADS = 512;
 
+unsigned blocks_for(size_t n, unsigned most)
+{
+    return (unsigned)std::min<size_t>((n + PACK_THREADS - 1) / PACK_THREADS, most);
+}
+
 // n elements of dense rows, from `first` on (an offset into the dense
-// volume): consecutive threads write consecutive elements.
+// volume).  Each thread writes four at once, on 16 bytes: dst is `skew`
+// elements above such a boundary, and the first and last group may be partial.
 __global__ void __launch_bounds__(PACK_THREADS) pack_rows_kernel(float *__restrict__ dst,
                                                                  const float *__restrict__ src, size_t first, size_t n,
-                                                                 unsigned nx, unsigned pitch)
+                                                                 unsigned nx, unsigned pitch, unsigned skew)
 {
-    for (size_t i = blockIdx.x * (size_t)PACK_THREADS + threadIdx.x; i < n; i += (size_t)gridDim.x * PACK_THREADS) {
-        const size_t row = (first + i) / nx;
-        dst[i] = src[row * pitch + (first + i - row * nx)];
+    const size_t groups = (n + skew + 3) / 4;
+    for (size_t g = blockIdx.x * (size_t)PACK_THREADS + threadIdx.x; g < groups; g += (size_t)gridDim.x * PACK_THREADS) {
+        const size_t begin = g == 0 ? 0 : 4 * g - skew, end = min(4 * g + 4 - skew, n);
+        const size_t row = (first + begin) / nx;
+        unsigned x = (unsigned)(first + begin - row * nx);
+        const float *p = src + row * pitch + x;
+        float v[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            if (begin + k < end)
+                v[k] = *p;
+            if (++x == nx) {  // on to the next row
+                x = 0;
+                p += pitch - nx;
+            }
+            p++;
+        }
+        if (end - begin == 4) {
+            *reinterpret_cast<float4 *>(dst + begin) = make_float4(v[0], v[1], v[2], v[3]);
+        } else {
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+                if (begin + k < end)
+                    dst[begin + k] = v[k];
+        }
     }
+}
+
+void launch_pack(float *dst, const float *src, size_t first, size_t n, int nx, int pitch, unsigned most, cudaStream_t s)
+{
+    const unsigned skew = (unsigned)(reinterpret_cast<uintptr_t>(dst) / sizeof(float) % 4);
+    pack_rows_kernel<<<blocks_for((n + skew + 3) / 4, most), PACK_THREADS, 0, s>>>(dst, src, first, n, nx, pitch, skew);
 }
 
 __global__ void __launch_bounds__(PACK_THREADS) unpack_bytes_kernel(uint8_t *__restrict__ dst,
@@ -40,24 +80,33 @@ __global__ void __launch_bounds__(PACK_THREADS) unpack_bytes_kernel(uint8_t *__r
     }
 }
 
-unsigned blocks_for(size_t n, unsigned most)
+// Whether a kernel may write host memory [p, p + bytes): floats on their own
+// alignment, all within one page-locked allocation (the two ends alone do not
+// tell: pages between two registered ranges need not be mapped) that the
+// device sees at the same address.  Anything else is left to the copy engine.
+bool kernel_may_write(const float *p, size_t bytes)
 {
-    return (unsigned)std::min<size_t>((n + PACK_THREADS - 1) / PACK_THREADS, most);
-}
-
-// The device address of page-locked host memory [p, p + bytes), or null.
-float *mapped_address(float *p, size_t bytes)
-{
-    cudaPointerAttributes a{}, z{};
-    if (cudaPointerGetAttributes(&a, p) != cudaSuccess ||
-        cudaPointerGetAttributes(&z, reinterpret_cast<char *>(p) + bytes - 1) != cudaSuccess) {
-        cudaGetLastError();  // not a sticky error: memory CUDA does not know
-        return nullptr;
-    }
-    if (a.type != cudaMemoryTypeHost || z.type != cudaMemoryTypeHost || !a.devicePointer || !z.devicePointer ||
-        (size_t)(static_cast<char *>(z.devicePointer) - static_cast<char *>(a.devicePointer)) != bytes - 1)
-        return nullptr;
-    return static_cast<float *>(a.devicePointer);
+    using Get = CUresult (*)(unsigned, CUpointer_attribute *, void **, CUdeviceptr);
+    static const Get get = []() -> Get {
+        void *f = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPointByVersion("cuPointerGetAttributes", &f, 12000, cudaEnableDefault, &q) !=
+                cudaSuccess ||
+            q != cudaDriverEntryPointSuccess)
+            return nullptr;
+        return reinterpret_cast<Get>(f);
+    }();
+    const uintptr_t at = reinterpret_cast<uintptr_t>(p);
+    unsigned type = 0, managed = 0;
+    CUdeviceptr dev = 0, start = 0;
+    size_t size = 0;
+    CUpointer_attribute what[] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_IS_MANAGED,
+                                  CU_POINTER_ATTRIBUTE_DEVICE_POINTER, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR,
+                                  CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+    void *to[] = {&type, &managed, &dev, &start, &size};
+    return get && at % sizeof(float) == 0 && get(5, what, to, (CUdeviceptr)at) == CUDA_SUCCESS &&
+           type == CU_MEMORYTYPE_HOST && !managed && dev == (CUdeviceptr)at && start <= dev &&
+           bytes <= size && dev - start <= size - bytes;
 }
 
 }  // namespace
@@ -68,19 +117,19 @@ cudaError_t read_rows(float *host, const float *src, size_t rows, int nx, int pi
     const size_t n = rows * (size_t)nx;
     if (n == 0)
         return cudaSuccess;
-    if (pitch == nx)
-        return cudaMemcpyAsync(host, src, sizeof(float) * n, cudaMemcpyDeviceToHost, s);
-    if (float *mapped = mapped_address(host, sizeof(float) * n)) {
-        pack_rows_kernel<<<blocks_for(n, 152), PACK_THREADS, 0, s>>>(mapped, src, 0, n, nx, pitch);
+    if (kernel_may_write(host, sizeof(float) * n)) {
+        launch_pack(host, src, 0, n, nx, pitch, 152, s);
         return cudaGetLastError();
     }
+    if (pitch == nx)
+        return cudaMemcpyAsync(host, src, sizeof(float) * n, cudaMemcpyDeviceToHost, s);
     if (!scratch || scratch_floats == 0)
         return cudaMemcpy2DAsync(host, sizeof(float) * nx, src, sizeof(float) * pitch, sizeof(float) * nx, rows,
                                  cudaMemcpyDeviceToHost, s);
     cudaError_t e = cudaSuccess;
     for (size_t o = 0; o < n && e == cudaSuccess; o += scratch_floats) {
         const size_t m = std::min(scratch_floats, n - o);
-        pack_rows_kernel<<<blocks_for(m, 152 * 4), PACK_THREADS, 0, s>>>(scratch, src, o, m, nx, pitch);
+        launch_pack(scratch, src, o, m, nx, pitch, 152 * 4, s);
         e = cudaGetLastError();
         if (e == cudaSuccess)
             e = cudaMemcpyAsync(host + o, scratch, sizeof(float) * m, cudaMemcpyDeviceToHost, s);

@@ -16,7 +16,7 @@ inline int padded_rows_pitch(int nx) { return nx < 16 ? nx : (nx + 15) & ~15; }
 // Queues on s the copy of `rows` rows of nx floats, pitch floats apart, into
 // the dense host volume.  Page-locked memory is written by a kernel, other
 // memory through scratch (device memory that work on s may use, scratch_floats
-// long; without it a strided copy).
+// long; without it a strided copy; dense rows are copied as they are).
 cudaError_t read_rows(float *host, const float *src, size_t rows, int nx, int pitch, float *scratch,
                       size_t scratch_floats, cudaStream_t s);
 

@@ -564,8 +564,6 @@ int fdtd_solver_get_field(fdtd_solver *s, int field, float *host_out)
     if (!src)
         return FDTD_ERR_INVALID;
     int st = fdtd_solver_synchronize(s);
-    if (st == FDTD_OK && s->pitch == s->nx)
-        return cu(cudaMemcpy(host_out, src, sizeof(float) * s->ncell, cudaMemcpyDeviceToHost));
     if (st == FDTD_OK)
         st = cu(read_rows(host_out, src, (size_t)s->ny * s->nz, s->nx, s->pitch, s->scratch, s->scratch_floats,
                           s->stream));

@@ -99,3 +99,27 @@ def test_read_longer_than_the_staging_area(cuda):
         b = s.field("ez", out=pinned.view(codes.shape))
         assert np.any(a[:40]) and np.any(a[-40:])
         assert np.array_equal(_bits(a), _bits(b))
+
+
+@pytest.mark.parametrize("dims", [(3, 5, 4), (4, 3, 5), (16, 9, 7), (17, 9, 6), (33, 10, 5), (64, 21, 19), (257, 67, 41)])
+def test_reads_land_on_any_alignment_and_nowhere_else(cuda, dims):
+    """Page-locked destinations at every offset from a 16-byte boundary (the
+    kernel writes 16 bytes at a time, its first and last group partly) and off
+    a float's own alignment, dense and padded rows: the values are those of a
+    pageable read, and the elements around the volume are not touched."""
+    torch, (nx, ny, nz) = cuda, dims
+    codes, specs, _, sources, consts, jz = random_case(*dims, seed=7, ncls=3, nsrc=2)
+    p = Params(make_params(dims, consts, sources, jz))
+    n, guard = nx * ny * nz, 8
+    raw = torch.zeros(4 * (n + 2 * guard) + 16, dtype=torch.uint8, pin_memory=True).numpy()
+    with fg.Solver(p, codes, specs, scheme=fg.SCHEME_CORRECTED) as s:
+        s.run(8)
+        want = s.field("ez")
+        assert np.count_nonzero(want)
+        for skew in (0, 4, 8, 12, 2):  # bytes
+            raw[:] = 0xA5
+            lo = 4 * guard + skew
+            out = raw[lo:lo + 4 * n].view(np.float32).reshape(codes.shape)
+            s.field("ez", out=out)
+            assert out.tobytes() == want.tobytes(), skew
+            assert np.all(raw[:lo] == 0xA5) and np.all(raw[lo + 4 * n:] == 0xA5), skew
