@@ -13,11 +13,12 @@
 // cell in the D form (15 floats + 1 byte read, 9 floats written), 73 in the
 // compact form (9 + 1 byte read, 9 written).
 //
-// Staging: with nx a multiple of 16 and 16-byte aligned buffers, one thread
-// issues TMA tile loads (cp.async.bulk.tensor.3d) for a whole plane into an
-// S-deep ring completed through mbarriers (every wait bounded; a timeout
-// raises the plan's error flag and the CTA stops).  Otherwise the same ring is
-// filled with 4-byte cp.async copies (zero-filled outside the grid).
+// Staging: with rows a multiple of 16 cells and 16-byte aligned buffers, one
+// thread issues TMA tile loads (cp.async.bulk.tensor.3d) for a whole plane into
+// an S-deep ring completed through mbarriers (every wait bounded; a timeout
+// raises the plan's error flag and the CTA stops).  Other compact states fill
+// the same ring with 4-byte cp.async copies (zero-filled outside the grid);
+// other D-form arrays take the two-pass kernels (launch_h_de_fused).
 //
 // Shape (32 x 8 tiles, 3 stages, one issuing thread) is the fastest of the
 // variants measured on the 512 x 512 x 400 phantom: 16-row tiles with 2
