@@ -21,12 +21,10 @@
 //   E^{n+1}, R^{n+1} (and scale words) leave by TMA stores.  No thread
 //   computes a global address per cell.
 // * A warp of its own moves the planes: it waits until the other warps have
-//   consumed a plane, stores its tiles, waits until the stores have read them
-//   and refills the stage.  With thread 0 of the cell warps doing this, every
-//   plane of a CTA waited for its own stores: 1.9 us per plane of a lone CTA
-//   against 1.4 (64^3, 32-bit R).  us per step before and after: 512 x 512 x
-//   400 1018 and 992 (16-bit R 930 and 925), 150 x 134 x 170 52 and 48 (53 and
-//   50), 20 batched solves of 48-256 cells per axis 454 and 432 (480 and 440).
+//   consumed a plane, updates the x faces in its tiles, stores the tiles, waits
+//   until the stores have read them and refills the stage.  With thread 0 of
+//   the cell warps moving the planes, every plane of a CTA waited for its own
+//   stores: 1.9 us per plane of a lone CTA against 1.4 (64^3, 32-bit R).
 // * Tiles whose cells, halo included, all lie inside the update ranges of
 //   every component, away from the x faces and from sources, take a path
 //   without per-cell range tests (CTA-uniform choice, per plane for the
@@ -82,7 +80,10 @@ struct StripGeo {
     // stores to have read them.
     static constexpr int T_BYTES = SX * TY * 4;
     static constexpr int O_H = 0, O_E = 3 * T_BYTES;
-    static_assert(6 * T_BYTES <= OFF_R, "H and E output tiles fit over the boxes");
+    // and, in x-face tiles, E^n y, z of each face cell and of its x neighbour
+    // ([face][TY] of ey, ez, neighbour's ey, ez) for the moving warp
+    static constexpr int O_F = 6 * T_BYTES;
+    static_assert(O_F + 2 * TY * 16 <= OFF_R, "the output tiles and the faces' E^n fit over the boxes");
     // H exchange of one plane: hz, hx of the row above each warp's first row
     // ([2][W][32]; row y0-1 for warp 0), and hz, hy of the x0-1 column
     // ([2][TY]).  Two sets, taken in turn by plane: a warp writes a plane's
@@ -314,12 +315,8 @@ struct StripPlanes {
     __device__ __forceinline__ bool no_r(int z) const { return z >= zc0 && ((memless >> (z - zc0)) & 1ull) != 0; }
 };
 
-// The moving warp's one lane at work: run() fills the ring, then plane by
-// plane waits until the cell warps have consumed the plane, stores the tiles
-// they have left in its stage and refills the stage.  Its waits are bounded;
-// when one gives up, or a cell warp's did (the stop word), the copies in
-// flight land (bounded) and the unit ends.  stall: leave the second plane's
-// copies unissued (test hook).
+// The moving warp's copies: a plane's boxes into its stage, a plane's tiles
+// from it.
 template <int RY, int W, int S, bool R16>
 struct StripMove {
     using G = StripGeo<RY, W, R16>;
@@ -348,26 +345,101 @@ struct StripMove {
             tma_store_3d(&maps.m[10], ob + G::OFF_X, y0, x0 / SX, z);
         bulk_commit();
     }
-    __device__ __forceinline__ void run(bool stall) const
-    {
-        for (int k = 0; k < S && k < u.nplanes; k++)
-            issue(k, stall && k == 1);
-        for (int k = 0; u.p0 + k < u.zc1; k++) {
-            if (!mbar_wait(u.consumed(k), u.parity(k)) || *static_cast<volatile int *>(u.sm.stop)) {
-                for (int j = k; j < u.nplanes && j < k + S; j++)
-                    mbar_wait(u.full(j), u.parity(j));
+};
+
+// The x faces of a unit: the moving warp applies their Mur updates to a
+// plane's E tiles before it stores them (updateMurBoundary ey/ez x faces,
+// fdtd_calculations.cu:280-340; the same rounded operations as the Mur
+// kernel).  Lane row + TY * face (0 near, 1 far) updates one face cell from the
+// neighbour's E^{n+1} in the tile and the E^n that the cell warps left beside
+// it.  In the cell warps these updates cost four shuffles, two more loads and
+// a divergent branch per row in every warp of a face tile.  us per step with
+// them there (and the moving warp's lane 0 at work alone) and so, 16-bit R: 20
+// solves of 48-256 cells per axis 437 and 411, of 24-128 109 and 99; 301 x 245 x
+// 187 154 and 143, 150 x 134 x 170 47.8 and 44.2, 512 x 512 x 400 922 and 907;
+// 32-bit R: 431 and 418, 152 and 149, 48.6 and 47.0, 992 and 994.
+struct StripXFaces {
+    const float4 *mur_x;  // Mur factors, [face][z][y]
+    int nx, ny, nz, scheme;
+    bool near, far;       // the tile holds x = 0, x = nx - 1
+};
+
+template <int RY, int W, int S, bool R16>
+__device__ __forceinline__ void strip_mur_rows(const StripMove<RY, W, S, R16> &move, const StripXFaces &f, int k, int lane)
+{
+    using G = StripGeo<RY, W, R16>;
+    constexpr int TY = G::TY, TS = SX * TY;
+    static_assert(2 * TY <= 32, "a lane per row of either face");
+    const int z = move.u.p0 + k, face = lane / TY, row = lane % TY, y = move.y0 + row;
+    if (z < 1 || z >= f.nz - 1 || face > 1 || !(face ? f.far : f.near) || y > f.ny - 2)
+        return;
+    unsigned char *stage = move.u.stage(k);
+    float *ey = reinterpret_cast<float *>(stage + G::O_E) + TS + row * SX, *ez = ey + TS;
+    const float4 e0 = reinterpret_cast<const float4 *>(stage + G::O_F)[face * TY + row];
+    const float4 mf = face && f.near ? f.mur_x[((size_t)f.nz + z) * f.ny + y]
+                                     : reinterpret_cast<const float4 *>(stage + G::OFF_F)[row];
+    const int self = face ? f.nx - 1 - move.x0 : 0, nbr = face ? self - 1 : 1;
+    auto mur = [&](float tn, float sn, float sf) {
+        return __fmul_rn(mf.x, __fsub_rn(__fadd_rn(__fmul_rn(mf.y, tn), __fmul_rn(mf.z, sn)), __fmul_rn(mf.w, sf)));
+    };
+    // ey: y 0..ny-2, z 1..nz-2; fdtd_calculations.cu:323: the far ey face
+    // reads E^n at x-1 in both terms
+    ey[self] = mur(face && f.scheme != FDTD_SCHEME_CORRECTED ? e0.z : ey[nbr], e0.z, e0.x);
+    if (y >= 1)  // ez: y 1..ny-2 (z = 0 in the Mur kernel)
+        ez[self] = mur(ez[nbr], e0.w, e0.y);
+}
+
+// The moving warp at work: fills the ring, then plane by plane waits until the
+// cell warps have consumed the plane, applies the x-face Mur updates, stores
+// the tiles the cell warps have left in its stage and refills the stage; all
+// but the updates by one elected lane.  Its waits are bounded; when one gives
+// up, or a cell warp's did (the stop word), the copies in flight land (bounded)
+// and the unit ends.  stall: leave the second plane's copies unissued (test
+// hook).
+//
+// A plane's refill waits for this warp, so its own instructions count.  The
+// warp stays together, its lane chosen by elect.sync (the compiler then keeps
+// the copies' operands in uniform registers; lane == 0 with a shuffle 1011 us
+// where this takes 994, the other lanes gone 1031), and the issuing code is
+// there once (the kernel's loops compete for the instruction cache: 930 us
+// with the first fill apart, 920 so; 512 x 512 x 400, 32-bit R and 16-bit R).
+template <int RY, int W, int S, bool R16>
+__device__ __forceinline__ void strip_run(const StripMove<RY, W, S, R16> &move, const StripXFaces &f, int lane,
+                                          bool stall)
+{
+    const auto &u = move.u;
+    const bool one = elect_one();
+    stall = __any_sync(0xffffffffu, stall);  // one lane was told
+    // the ring's first fill is the loop's first S turns
+    for (int k = -S; u.p0 + k < u.zc1; k++) {
+        if (k >= 0) {
+            bool ok = false;
+            if (one)
+                ok = mbar_wait(u.consumed(k), u.parity(k)) && !*static_cast<volatile int *>(u.sm.stop);
+            if (!__any_sync(0xffffffffu, ok)) {
+                if (one)
+                    for (int j = k; j < u.nplanes && j < k + S; j++)
+                        mbar_wait(u.full(j), u.parity(j));
                 break;
             }
-            if (u.p0 + k >= u.zc0)
-                store(k);
-            if (k + S < u.nplanes) {
-                bulk_wait_read<0>();  // the refill overwrites the tiles
-                issue(k + S, false);
+            const bool out = u.p0 + k >= u.zc0;
+            if (out && (f.near || f.far)) {
+                __syncwarp();  // every lane sees what the waiting lane was given
+                strip_mur_rows(move, f, k, lane);
+                fence_async_shared();  // the lanes' writes are visible to the stores
+                __syncwarp();
             }
+            if (one && out)
+                move.store(k);
         }
-        bulk_wait_all();
+        if (one && k + S < u.nplanes) {
+            bulk_wait_read<0>();  // the refill overwrites the tiles
+            move.issue(k + S, stall && k + S == 1);
+        }
     }
-};
+    if (one)
+        bulk_wait_all();
+}
 
 // One work unit: column tile (bx, by), z chunk bz of one solve.  memless: bit
 // j set when plane zc0 + j of the tile holds no Debye memory.  stall: the
@@ -389,23 +461,19 @@ __device__ __forceinline__ void strip_unit(const C &c, const StripMaps &maps, in
     const StripPlanes<RY, W, S, R16> u(sm, nz, zchunk, bz, memless);
     const int zc0 = u.zc0, zc1 = u.zc1, p0 = u.p0, nplanes = u.nplanes;
 
-    // x-face Mur updates (updateMurBoundary ey/ez x faces,
-    // fdtd_calculations.cu:280-340) in the tiles that hold x = 0 or nx-1;
-    // their per-cell factors arrive with the plane's boxes
+    // x-face Mur updates in the tiles that hold x = 0 or nx-1, by the moving
+    // warp; their per-cell factors arrive with the plane's boxes
     const int mur_bits = mur_x_fused_faces(c);
     const bool face_near = (mur_bits & 1) && x0 == 0;
     const bool face_far_cta = (mur_bits & 2) && x0 <= nx - 1 && nx - 1 < x0 + SX;
     const bool face_cta = face_near || face_far_cta;
-    const bool faces_both = face_near && face_far_cta;
     if (w == W) {
-        if (lane == 0) {
-            StripMove<RY, W, S, R16> move{maps, u, StripFaces{nullptr, (size_t)ny, 0u}, x0, y0};
-            if (face_cta) {
-                move.faces.bytes = (uint32_t)min(TY, ny - y0) * 16u;
-                move.faces.src = face_near ? c.mur_x + y0 : c.mur_x + (size_t)nz * ny + y0;
-            }
-            move.run(stall);
+        StripMove<RY, W, S, R16> move{maps, u, StripFaces{nullptr, (size_t)ny, 0u}, x0, y0};
+        if (face_cta) {
+            move.faces.bytes = (uint32_t)min(TY, ny - y0) * 16u;
+            move.faces.src = face_near ? c.mur_x + y0 : c.mur_x + (size_t)nz * ny + y0;
         }
+        strip_run(move, StripXFaces{c.mur_x, nx, ny, nz, c.scheme, face_near, face_far_cta}, lane, stall);
         return;
     }
 
@@ -420,8 +488,6 @@ __device__ __forceinline__ void strip_unit(const C &c, const StripMaps &maps, in
     }
     const float kx = c.kx, ky = c.ky, kz = c.kz, tcx = c.tx, tcy = c.ty, tcz = c.tz;
     const int cls_max = c.nclasses - 1;
-    const bool face_far = x == nx - 1;
-    const bool face_lane = x < nx && (((mur_bits & 1) && x == 0) || ((mur_bits & 2) && face_far));
     // every own cell and every halo cell inside the update ranges of all
     // components in x and y, no x face, no source
     const bool xy_inside = x0 >= 1 && x0 + SX - 1 <= nx - 2 && y0 >= 1 && y0 + TY - 1 <= ny - 2 && !face_cta &&
@@ -496,8 +562,6 @@ __device__ __forceinline__ void strip_unit(const C &c, const StripMaps &maps, in
         // ---- H^{n+1/2} at plane z on the strip (fdtd_calculations.cu:43-76)
         float ex[RY + 1], ey[RY], ez[RY + 1];
         float hxn[RY], hyn[RY], hzn[RY];
-        float ey_nb[RY], ez_nb[RY];  // face lanes: E^n y, z of the x-neighbour (read here: the box is
-                                     // refilled before the E pass)
 #pragma unroll
         for (int r = 0; r <= RY; r++) {
             ex[r] = ea(0, ry0 + r + 1, ec);
@@ -510,12 +574,6 @@ __device__ __forceinline__ void strip_unit(const C &c, const StripMaps &maps, in
             hxn[r] = ha(0, er, ec);
             hyn[r] = ha(1, er, ec);
             hzn[r] = ha(2, er, ec);
-            const int y = y0 + ry0 + r;
-            if (face_cta) {
-                const int cn = face_far ? ec - 1 : ec + 1;
-                ey_nb[r] = ea(1, er, cn);
-                ez_nb[r] = ea(2, er, cn);
-            }
             if (fast) {
                 hxn[r] = cm_h(hxn[r], ky, ez[r + 1], ez[r], ky, eb(1, er, ec), ey[r]);
                 hyn[r] = cm_h(hyn[r], kz, eb(0, er, ec), ex[r], kx, ea(2, er, ec + 1), ez[r]);
@@ -677,29 +735,6 @@ __device__ __forceinline__ void strip_unit(const C &c, const StripMaps &maps, in
                     rn0 = ex_on ? s0 : (R16 ? 0.0f : r0[r]);
                     rn1 = eyz_on ? s1 : (R16 ? 0.0f : r1[r]);
                     rn2 = eyz_on ? s2 : (R16 ? 0.0f : r2[r]);
-                    if (face_cta) {  // uniform over the CTA: every lane takes part in the shuffles
-                        const unsigned all = 0xffffffffu;
-                        const float ey_hi = __shfl_down_sync(all, en1, 1), ez_hi = __shfl_down_sync(all, en2, 1);
-                        const float ey_lo = __shfl_up_sync(all, en1, 1), ez_lo = __shfl_up_sync(all, en2, 1);
-                        if (face_lane && y < ny && zmid) {
-                            const float4 mf =
-                                faces_both && face_far
-                                    ? c.mur_x[((size_t)nz + z) * ny + y]
-                                    : reinterpret_cast<const float4 *>(stage + G::OFF_F)[row];
-                            auto mur = [&](float tn, float sn, float sf) {
-                                return __fmul_rn(mf.x, __fsub_rn(__fadd_rn(__fmul_rn(mf.y, tn), __fmul_rn(mf.z, sn)),
-                                                                 __fmul_rn(mf.w, sf)));
-                            };
-                            if (y <= ny - 2) {  // ey faces: y 0..ny-2, z 1..nz-2
-                                // fdtd_calculations.cu:323: the far ey face reads E^n at x-1 in both terms
-                                const float tn = face_far ? (c.scheme == FDTD_SCHEME_CORRECTED ? ey_lo : ey_nb[r])
-                                                          : ey_hi;
-                                en1 = mur(tn, ey_nb[r], ey[r]);
-                            }
-                            if (y >= 1 && y <= ny - 2)  // ez faces: y 1..ny-2 (z = 0 in the Mur kernel)
-                                en2 = mur(face_far ? ez_lo : ez_hi, ez_nb[r], ez[r]);
-                        }
-                    }
                 }
                 en[0][r] = en0;
                 en[1][r] = en1;
@@ -711,6 +746,14 @@ __device__ __forceinline__ void strip_unit(const C &c, const StripMaps &maps, in
 #pragma unroll
             for (int r = 0; r < RY; r++) {
                 const int row = ry0 + r, t = row * SX + lane, y = y0 + row;
+                if (face_cta) {  // E^n of the face cells and their neighbours, for the moving warp
+                    float2 *EF = reinterpret_cast<float2 *>(stage + G::O_F);
+                    const int to_far = nx - 1 - x;  // 0: the far face cell, 1: its neighbour
+                    if (face_near && lane < 2)
+                        EF[2 * row + lane] = make_float2(ey[r], ez[r]);
+                    if (face_far_cta && (to_far == 0 || to_far == 1))
+                        EF[2 * (TY + row) + to_far] = make_float2(ey[r], ez[r]);
+                }
                 OH[t] = hxn[r];
                 OH[TS + t] = hyn[r];
                 OH[2 * TS + t] = hzn[r];

@@ -73,6 +73,14 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity)
     return false;
 }
 
+// True in one lane of a converged warp, the same at every call.
+__device__ __forceinline__ bool elect_one()
+{
+    uint32_t r;
+    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(r));
+    return r != 0;
+}
+
 constexpr int BAR_CELLS = 1;  // named barrier of the cell warps alone
 
 __device__ __forceinline__ void mbar_arrive(uint32_t bar)
