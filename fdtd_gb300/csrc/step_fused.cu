@@ -163,7 +163,7 @@ __device__ __forceinline__ size_t r16_word(const NativeConsts &c, int z, int bx,
 // warps; else thread 0 refills a stage behind the barrier at its plane's end.
 // The batched D form runs with a moving warp (20 solves of 48-256 cells per axis
 // 668 us per step without, 632 with; of 24-128 150 and 135); the single solve
-// without (512 x 512 x 400: 1559 us, with 1598; 224 x 208 x 176: 139, 141; why a
+// without (512 x 512 x 400: 1559 us, with 1600; 224 x 208 x 176: 139, 141; why a
 // grid that fills the device with equal CTAs loses is not established).
 template <int TY, bool MOVER>
 __host__ __device__ constexpr int fused_threads() { return FTX * (TY + (MOVER ? 1 : 0)); }
@@ -181,8 +181,8 @@ __device__ __forceinline__ void fused_unit(const NativeConsts &c, const FusedMap
     constexpr int NT = COMPACT ? 3 : 9, TB = R16 ? 2 : 4, XB = R16 ? TY * 4 : 0;
     using G = Geo<TY, NT, TB, XB>;
     const int nx = c.nx, ny = c.ny, nz = c.nz;
-    // the row by a shuffle: known as uniform over the warp (see strip_unit.cuh)
-    const int tx = threadIdx.x, ty = MOVER ? __shfl_sync(0xffffffffu, (int)threadIdx.y, 0) : (int)threadIdx.y;
+    // the row by a shuffle: known as uniform over the warp
+    const int tx = threadIdx.x, ty = TMA ? __shfl_sync(0xffffffffu, (int)threadIdx.y, 0) : (int)threadIdx.y;
     const int tid = ty * FTX + tx;
     const int x0 = bx * FTX, y0 = by * TY;
     const int x = x0 + tx, y = y0 + ty;
@@ -200,24 +200,29 @@ __device__ __forceinline__ void fused_unit(const NativeConsts &c, const FusedMap
 
     if constexpr (MOVER) {
         if (ty == TY) {
-            if (tx == 0) {
-                auto issue = [&](int k, bool arm_only) {
-                    const int z = p0 + k;
-                    issue_plane_tma<TY, NT, TB, XB>(maps, stage(k), bar(k), plane_kind(z, zc0, zc1), x0, y0, z, arm_only);
-                };
-                for (int k = 0; k < S && k < nplanes; k++)
-                    issue(k, stall && k == 1);
-                for (int k = 0; p0 + k < zc1; k++) {
-                    if (!mbar_wait(consumed_bar(k), parity(k)) || *stop) {
+            // the warp stays together and one elected lane works (as in strip_unit.cuh:
+            // 604 us per step with the other lanes gone, 601 so)
+            const bool one = elect_one();
+            stall = __any_sync(0xffffffffu, stall);  // one lane was told
+            // the ring's first fill is the loop's first S turns
+            for (int k = -S; p0 + k < zc1; k++) {
+                if (k >= 0) {
+                    bool ok = false;
+                    if (one)
+                        ok = mbar_wait(consumed_bar(k), parity(k)) && !*stop;
+                    if (!__any_sync(0xffffffffu, ok)) {
                         // a bounded wait gave up: the copies in flight land (bounded)
-                        for (int j = k; j < nplanes && j < k + S; j++)
-                            mbar_wait(bar(j), parity(j));
+                        if (one)
+                            for (int j = k; j < nplanes && j < k + S; j++)
+                                mbar_wait(bar(j), parity(j));
                         break;
                     }
-                    if (k + S < nplanes) {
-                        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                        issue(k + S, false);
-                    }
+                }
+                if (one && k + S < nplanes) {
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                    const int z = p0 + k + S;
+                    issue_plane_tma<TY, NT, TB, XB>(maps, stage(k + S), bar(k + S), plane_kind(z, zc0, zc1), x0, y0, z,
+                                                    stall && k + S == 1);
                 }
             }
             return;
@@ -643,7 +648,12 @@ __device__ __forceinline__ void fused_unit(const NativeConsts &c, const FusedMap
         // refill the stage of plane k with plane k + S
         const int kn = k + S;
         if (TMA) {
-            if (tid == 0 && kn < nplanes) {
+            // one lane of warp 0, the row being uniform: the copies' operands stay in
+            // uniform registers.  us per step with tid == 0 and so, D form: 512 x 512 x
+            // 400 1559 and 1539, 217 x 253 x 181 169 and 166, 150 x 134 x 170 69.6 and
+            // 67.8; compact 1182 and 1173, 16-bit R 1271 and 1245 (512 x 512 x 400).
+            // elect.sync without the uniform row: 1628.
+            if (ty == 0 && kn < nplanes && elect_one()) {
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 const int zn = p0 + kn;
                 issue_plane_tma<TY, NT, TB, XB>(maps, stage(kn), bar(kn), plane_kind(zn, zc0, zc1), x0, y0, zn);
