@@ -118,6 +118,7 @@ NativeConsts make_consts(const fdtd_plan *p, const fdtd_native_fields *f, int n)
             c.sources[3 * s + k] = p->sources[3 * s + k];
     c.coef = p->d_coef;
     c.nclasses = p->nclasses;
+    c.class_last = FDTD_MAX_CLASSES - 1;
     c.jz = p->d_jz;
     c.njz = p->njz;
     c.rp = p->rp;
@@ -264,7 +265,7 @@ __global__ void __launch_bounds__(TX *TY) native_de_kernel(NativeConsts c)
             }
         }
     }
-    const int cls = (ex_on || eyz_on) ? c.mat[i] : 0;
+    const int cls = (ex_on || eyz_on) ? min((int)c.mat[i], c.class_last) : 0;
     if (dx_on)
         dnew[0] = dn[0] + c.ty * (hz0 - hz_y) - c.tz * (hy0 - hy_z);
     if (dy_on)

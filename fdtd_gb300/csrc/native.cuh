@@ -85,6 +85,12 @@ struct NativeConsts {
     // the D half step reads H cells that no H half step ever writes from h_in
     // (a single-pass step: only h_in is sure to hold them)
     int h_edges_in;
+    // last row of coef that a class byte selects in the two-pass D/E kernel; a
+    // larger byte takes that row, so no byte reads beyond the table.  A plan's
+    // table has all FDTD_MAX_CLASSES rows (those without a class are zero);
+    // single-pass steps limit it to the caller's classes, as the z-marching
+    // kernel does.
+    int class_last;
 };
 
 NativeConsts make_consts(const fdtd_plan *p, const fdtd_native_fields *f, int n);

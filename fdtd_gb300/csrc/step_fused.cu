@@ -1109,6 +1109,7 @@ int launch_h_de_fused(const NativeConsts &c, cudaStream_t s)
     // kept): 250 x 239 x 160 324 / 202 / 191, 123 x 131 x 90 76 / 35 / 40, 498
     // x 300 x 200 - / 604 / 575.
     a.c.h_edges_in = 1;
+    a.c.class_last = c.nclasses - 1;
     const int st = launch_h(a.c, s);
     return st == FDTD_OK ? launch_de(a.c, s) : st;
 }

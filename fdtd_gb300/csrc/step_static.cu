@@ -141,6 +141,7 @@ extern "C" int fdtd_step_static(const FdtdParams *p, const float *specs, int ncl
         c.sources[k] = p->sources[k];
     c.coef = d_coef;
     c.nclasses = nclasses;
+    c.class_last = nclasses - 1;
     c.jz = d_jz;          // one entry: the sample of step n, selected above
     c.njz = 1;
     c.step = 0;
