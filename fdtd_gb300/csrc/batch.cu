@@ -109,6 +109,8 @@ struct fdtd_batch {
     int next_id = 1;
     bool dirty = true;
     BatchDesc *d_descs = nullptr;
+    unsigned *d_seen = nullptr;  // per descriptor: which SMs have its tensor maps as last written
+    unsigned epoch = 0;          // of the descriptors' last rewrite
     size_t descs_cap = 0;
     BatchMurBlock *d_mur = nullptr;
     size_t mur_cap = 0;
@@ -335,11 +337,21 @@ int rebuild(fdtd_batch *b)
     if (st == FDTD_OK && descs.size() > b->descs_cap) {
         if (b->d_descs)
             cudaFreeAsync(b->d_descs, b->stream);
+        if (b->d_seen)
+            cudaFreeAsync(b->d_seen, b->stream);
         b->d_descs = nullptr;
+        b->d_seen = nullptr;
         const size_t cap = std::max(descs.size() * 2, size_t(16));
+        const size_t seen_bytes = sizeof(unsigned) * batch_seen_row((int)cap, 0);
         st = pool_alloc(b, reinterpret_cast<void **>(&b->d_descs), sizeof(BatchDesc) * cap, b->stream);
+        if (st == FDTD_OK)
+            st = pool_alloc(b, reinterpret_cast<void **>(&b->d_seen), seen_bytes, b->stream);
+        if (st == FDTD_OK)
+            st = cu(cudaMemsetAsync(b->d_seen, 0, seen_bytes, b->stream));
         b->descs_cap = st == FDTD_OK ? cap : 0;
     }
+    if (++b->epoch == 0)
+        b->epoch = 1;
     if (st == FDTD_OK && mur.size() > b->mur_cap) {
         if (b->d_mur)
             cudaFreeAsync(b->d_mur, b->stream);
@@ -382,7 +394,8 @@ int rebuild(fdtd_batch *b)
     if (st != FDTD_OK)
         return st;
     b->launch = BatchLaunch{b->d_descs, (int)descs.size(), units, b->d_mur, (int)mur.size(), b->compact ? 1 : 0,
-                            max_classes, b->r16 ? 1 : 0, strip ? 1 : 0, b->strip_shape, b->d_units};
+                            max_classes, b->r16 ? 1 : 0, strip ? 1 : 0, b->strip_shape, b->d_units,
+                            b->d_seen, b->epoch};
     b->strip = strip;
     drop_graphs(b);
     b->dirty = false;
@@ -520,6 +533,8 @@ int fdtd_batch_destroy(fdtd_batch *b)
         free_solve(v, s);
     if (b->d_descs)
         cudaFreeAsync(b->d_descs, s);
+    if (b->d_seen)
+        cudaFreeAsync(b->d_seen, s);
     if (b->d_mur)
         cudaFreeAsync(b->d_mur, s);
     if (b->d_units)

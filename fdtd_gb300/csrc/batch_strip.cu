@@ -21,7 +21,8 @@ namespace {
 // record, its solve's constants in shared memory, then the unit.
 template <int RY, int W, int S, bool R16, int MINB>
 __global__ void __launch_bounds__(32 * W + 32, MINB) batch_strip_kernel(const BatchDesc *__restrict__ descs,
-                                                                  const BatchUnit *__restrict__ units)
+                                                                  const BatchUnit *__restrict__ units,
+                                                                  unsigned *seen, unsigned epoch)
 {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ StripConsts s_c;
@@ -35,6 +36,8 @@ __global__ void __launch_bounds__(32 * W + 32, MINB) batch_strip_kernel(const Ba
     const int par = n & 1;
     if (threadIdx.x == 0)
         strip_consts(s_c, d.c[par]);
+    if (threadIdx.x < 32)
+        acquire_tensor_maps<STRIP_MAPS>(d.smaps[par].m, seen + batch_seen_row(rec.solve, par), epoch, threadIdx.x);
     strip_load_coef(d.c[par], sm.coef, 32 * W + 32);
     __syncthreads();
     strip_unit<RY, W, S, R16>(s_c, d.smaps[par], rec.zchunk, rec.bx, rec.by, rec.bz, rec.memless, sm, false);
@@ -74,7 +77,7 @@ struct BatchKernel {
         const int st = opt_in();
         if (st != FDTD_OK)
             return st;
-        fn<<<b.total_units, 32 * W + 32, smem(b.max_classes), s>>>(b.descs, b.units);
+        fn<<<b.total_units, 32 * W + 32, smem(b.max_classes), s>>>(b.descs, b.units, b.seen, b.epoch);
         const cudaError_t e = cudaGetLastError();
         return e == cudaSuccess ? FDTD_OK : (int)e;
     }

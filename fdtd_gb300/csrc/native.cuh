@@ -7,6 +7,7 @@
 #include <vector>
 
 #include "device_common.cuh"
+#include "tma_util.cuh"
 
 struct fdtd_plan {
     int device = 0;
@@ -163,25 +164,28 @@ bool step_fuses_mur_x(int kernel_kind, const NativeConsts &c);
 // D^{n-1} (3), E^{n-1} (3), material classes (1).  Compact form: R (3)
 // after the six halo maps, then the classes; with 16-bit R the exponent
 // words follow the classes.
+constexpr int FUSED_MAPS = 16;
 struct FusedMaps {
-    CUtensorMap m[16];
+    CUtensorMap m[FUSED_MAPS];
 };
 
 // Tensor maps of one strip-kernel launch (step_strip.cu, strip_unit.cuh):
 // E^n (0-2), H^{n-1/2} (3-5), R or its FP16 residuals (6-8, loaded and
 // stored in place), classes (9), scale words (10, 16-bit R), H^{n+1/2}
 // (11-13), E^{n+1} (14-16).
+constexpr int STRIP_MAPS = 17;
 struct StripMaps {
-    CUtensorMap m[17];
+    CUtensorMap m[STRIP_MAPS];
 };
-static_assert(sizeof(StripMaps) % 64 == 0, "tensor maps stay 64-byte aligned in arrays");
+static_assert(sizeof(FusedMaps) % 128 == 0 && sizeof(StripMaps) % 128 == 0, "tensor maps stay aligned in arrays");
 
 // One solve of a batch as the batched kernels see it (device memory).  The
 // solve's completed-step count n selects c[n & 1] / maps[n & 1] (smaps in a
 // batch run by the strip kernel); units [unit_begin, unit_begin +
 // unit_count) are its (tile x, tile y, z chunk) work items; it is skipped
-// once n reaches steps_target.
-struct alignas(64) BatchDesc {
+// once n reaches steps_target.  The maps lie on 128 bytes, the unit of
+// acquire_tensor_maps.
+struct alignas(128) BatchDesc {
     FusedMaps maps[2];
     StripMaps smaps[2];
     NativeConsts c[2];
@@ -205,6 +209,12 @@ struct alignas(16) BatchUnit {
 };
 static_assert(sizeof(BatchUnit) == 32, "two 16-byte copies per record");
 
+// First word of a solve's row in BatchLaunch::seen.
+__host__ __device__ constexpr size_t batch_seen_row(int solve, int par)
+{
+    return ((size_t)solve * 2 + par) * tma::SM_SLOTS;
+}
+
 // One face block of the batched Mur launch: solve, face set, first cell;
 // a block of 256 threads updates BATCH_MUR_CELLS consecutive cells of the set
 // (up to `limit`).
@@ -227,6 +237,8 @@ struct BatchLaunch {
     int strip;        // compact forms: run by the strip kernel of shape strip_shape
     int strip_shape;
     const BatchUnit *units;  // one record per unit
+    unsigned *seen;          // per solve and parity, SM_SLOTS words: acquire_tensor_maps
+    unsigned epoch;          // of the descriptors
 };
 
 // Tensor maps of a single-pass launch over c's buffers (false: not encodable).

@@ -756,7 +756,8 @@ __global__ void __launch_bounds__(FTX *TY) fused_step_kernel(const __grid_consta
 // 16-bit R 11 % faster than with 3 or 5).
 template <int TY, int S, bool COMPACT, bool R16 = false>
 __global__ void __launch_bounds__((fused_threads<TY, !COMPACT>()), COMPACT ? 4 : 3) batch_step_kernel(const BatchDesc *__restrict__ descs,
-                                                                             const BatchUnit *__restrict__ units)
+                                                                             const BatchUnit *__restrict__ units,
+                                                                             unsigned *seen, unsigned epoch)
 {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     unsigned char *smem = smem_raw + ((128 - (smem_addr(smem_raw) & 127)) & 127);
@@ -779,6 +780,8 @@ __global__ void __launch_bounds__((fused_threads<TY, !COMPACT>()), COMPACT ? 4 :
             dst[i] = src[i];
     }
     load_coef(d.c[par], coef, NTH);
+    if (threadIdx.y == 0)
+        acquire_tensor_maps<FUSED_MAPS>(d.maps[par].m, seen + batch_seen_row(rec.solve, par), epoch, threadIdx.x);
     __syncthreads();
     const int local = (int)blockIdx.x - d.unit_begin, per_z = d.tiles_x * d.tiles_y, rem = local % per_z;
     fused_unit<TY, S, true, !COMPACT, COMPACT, R16>(s_c, d.maps[par], d.zchunk, rem % d.tiles_x, rem / d.tiles_x, local / per_z,
@@ -1060,7 +1063,7 @@ struct BatchStep {
         const int st = opt_in();
         if (st != FDTD_OK)
             return st;
-        fn<<<b.total_units, dim3(FTX, NTH / FTX), smem(b.max_classes), s>>>(b.descs, b.units);
+        fn<<<b.total_units, dim3(FTX, NTH / FTX), smem(b.max_classes), s>>>(b.descs, b.units, b.seen, b.epoch);
         const cudaError_t e = cudaGetLastError();
         return e == cudaSuccess ? FDTD_OK : (int)e;
     }

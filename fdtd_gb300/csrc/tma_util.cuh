@@ -102,6 +102,39 @@ __device__ __forceinline__ bool cells_barrier_or(bool v)
     return __any_sync(0xffffffffu, r != 0);  // a vote: known as uniform over the warp
 }
 
+// Tensor maps that a kernel reads from global memory, where host copies rewrite
+// them in place: TMA goes through the tensor-map proxy, whose cache on the SM may
+// hold an older map of the same address until a proxy fence names it (maps in
+// kernel parameters need none).  Called by the first warp of a block (lane),
+// before a barrier that the issuing thread passes too; the N maps are fenced
+// where this SM has not done so since they were written.  seen: one word per SM
+// slot, holding the epoch (never 0, new with every rewrite) of its last fence;
+// a block that finds the epoch there is ordered behind that fence.
+//
+// Fences in every block made its 17 map fetches wait on L2 again: 48 steps and
+// reads of 20 solves of 48-256 cells per axis (16-bit R) took 32.4 ms, of 24-128 (D
+// form) 8.0; without any fence 22.1 and 7.0; so 22.3 and 7.0.
+constexpr int SM_SLOTS = 256;  // an SM numbered higher fences every time
+
+template <int N>
+__device__ __forceinline__ void acquire_tensor_maps(const CUtensorMap *maps, unsigned *seen, unsigned epoch, int lane)
+{
+    static_assert(N <= 32, "a lane per map");
+    uint32_t sm, was = 0;
+    asm volatile("mov.u32 %0, %%smid;" : "=r"(sm));
+    if (sm < SM_SLOTS)
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(was) : "l"(seen + sm) : "memory");
+    if (!__any_sync(0xffffffffu, was != epoch))
+        return;
+    if (lane < N)
+        asm volatile("fence.proxy.tensormap::generic.acquire.sys [%0], 128;" ::"l"(
+                         reinterpret_cast<uint64_t>(maps + lane))
+                     : "memory");
+    __syncwarp();
+    if (lane == 0 && sm < SM_SLOTS)
+        asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(seen + sm), "r"(epoch) : "memory");
+}
+
 __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap *map, int x, int y, int z, uint32_t bar)
 {
     asm volatile(

@@ -1,0 +1,49 @@
+"""Orderings that a wrong result would show too rarely to be tested by results,
+checked in the kernels' sources, on the CPU."""
+from __future__ import annotations
+
+import re
+from pathlib import Path
+
+CSRC = Path(__file__).resolve().parent.parent / "fdtd_gb300" / "csrc"
+
+
+def _kernels():
+    """(file, name, parameters, body) of every __global__ function."""
+    for path in sorted([*CSRC.glob("*.cu"), *CSRC.glob("*.cuh")]):
+        text = re.sub(r"//[^\n]*", "", path.read_text())
+        for m in re.finditer(r"__global__\s+void\s+", text):
+            at = m.end()
+            bounds = re.match(r"__launch_bounds__\s*\(", text[at:])
+            if bounds:
+                at = _close(text, at + bounds.end() - 1, "()")
+            name = re.match(r"\s*(\w+)\s*\(", text[at:])
+            p0 = at + name.end() - 1
+            p1 = _close(text, p0, "()")
+            b0 = text.index("{", p1)
+            yield path.name, name.group(1), text[p0 + 1:p1 - 1], text[b0:_close(text, b0, "{}")]
+
+
+def _close(text, at, pair):
+    depth = 0
+    for k in range(at, len(text)):
+        depth += (text[k] == pair[0]) - (text[k] == pair[1])
+        if depth == 0:
+            return k + 1
+    raise AssertionError("unbalanced source")
+
+
+def test_tensor_maps_in_global_memory_are_acquired_before_use():
+    """A batch's tensor maps are rewritten in place by host copies whenever a
+    solve joins or leaves; a block that uses them must acquire them through the
+    tensor-map proxy first, with a barrier between."""
+    seen = 0
+    for file, name, params, body in _kernels():
+        if "BatchDesc" not in params or not re.search(r"\bd\.s?maps\[", body):
+            continue
+        seen += 1
+        acquire = body.find("acquire_tensor_maps<")
+        use = re.search(r"(strip|fused)_unit<", body).start()
+        assert 0 <= acquire < use, (file, name)
+        assert "__syncthreads();" in body[acquire:use], (file, name)
+    assert seen == 2
