@@ -149,6 +149,7 @@ def lib() -> C.CDLL:
         _sig(L, "fdtd_solver_run", _I, _V, _I)
         _sig(L, "fdtd_solver_synchronize", _I, _V)
         _sig(L, "fdtd_solver_test_stall", _I, _V)
+        _sig(L, "fdtd_solver_test_stall_store", _I, _V)
         _sig(L, "fdtd_solver_steps", _I, _V)
         _sig(L, "fdtd_solver_get_field", _I, _V, _I, _P)
         _sig(L, "fdtd_solver_stream", _V, _V)
@@ -353,6 +354,10 @@ class Solver:
         """Failure-path test hook: the next single-pass step's first CTA lets one
         bounded wait run out; synchronize() then raises FDTD_ERR_DEVICE_TIMEOUT."""
         check(lib().fdtd_solver_test_stall(self.handle), "fdtd_solver_test_stall")
+
+    def test_stall_store(self) -> None:
+        """The same for the warp that stores the finished tiles (compact forms)."""
+        check(lib().fdtd_solver_test_stall_store(self.handle), "fdtd_solver_test_stall_store")
 
     @property
     def steps(self) -> int:

@@ -40,7 +40,7 @@ __global__ void __launch_bounds__(32 * W + 32, MINB) batch_strip_kernel(const Ba
         acquire_tensor_maps<STRIP_MAPS>(d.smaps[par].m, seen + batch_seen_row(rec.solve, par), epoch, threadIdx.x);
     strip_load_coef(d.c[par], sm.coef, 32 * W + 32);
     __syncthreads();
-    strip_unit<RY, W, S, R16>(s_c, d.smaps[par], rec.zchunk, rec.bx, rec.by, rec.bz, rec.memless, sm, false);
+    strip_unit<RY, W, S, R16>(s_c, d.smaps[par], rec.zchunk, rec.bx, rec.by, rec.bz, rec.memless, sm, 0);
 }
 
 template <int SHAPE, bool R16>

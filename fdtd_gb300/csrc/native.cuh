@@ -52,9 +52,8 @@ struct NativeConsts {
     int step;              // step index n when step_counter is null
     int *step_counter;     // device step index (graph replay), may be null
     int *err;              // device error flag (a bounded wait gave up)
-    int *stall_once;       // test hook, may be null: when set, the first CTA of the next single-pass
-                           // launch clears it and arms one plane's barrier without issuing its
-                           // copies, so that CTA's bounded wait runs out (raises *err)
+    int *stall_once;       // test hook, may be null: when set (STALL_*), the first CTA of the next
+                           // single-pass launch clears it and lets one of its bounded waits give up
     int overlap_prev;      // single-pass launch may start while the previous step's Mur kernel runs
                            // (programmatic dependent launch; only where that kernel precedes it)
     int fuse_mur_x;        // the single-pass kernel applies the x-face Mur updates and the Mur
@@ -93,6 +92,11 @@ struct NativeConsts {
     // kernel does.
     int class_last;
 };
+
+// stall_once: STALL_LOAD arms one plane's barrier without issuing its copies, so
+// that the wait for them runs out; STALL_STORE (strip kernel) has the moving warp
+// give up at the unit's last plane, as if its wait for the cell warps had.
+constexpr int STALL_LOAD = 1, STALL_STORE = 2;
 
 NativeConsts make_consts(const fdtd_plan *p, const fdtd_native_fields *f, int n);
 

@@ -542,16 +542,20 @@ int fdtd_solver_synchronize(fdtd_solver *s)
 
 int fdtd_solver_steps(const fdtd_solver *s) { return s ? s->steps : -1; }
 
-int fdtd_solver_test_stall(fdtd_solver *s)
+static int set_stall(fdtd_solver *s, int what)
 {
-    if (!s)
-        return FDTD_ERR_INVALID;
     cudaSetDevice(s->device);
-    static const int one = 1;
-    int st = cu(cudaMemcpyAsync(s->plan->d_stall, &one, sizeof one, cudaMemcpyHostToDevice, s->stream));
+    int st = cu(cudaMemcpyAsync(s->plan->d_stall, &what, sizeof what, cudaMemcpyHostToDevice, s->stream));
     if (st == FDTD_OK)
         st = cu(cudaStreamSynchronize(s->stream));  // the source is host memory of this call
     return st;
+}
+
+int fdtd_solver_test_stall(fdtd_solver *s) { return s ? set_stall(s, STALL_LOAD) : FDTD_ERR_INVALID; }
+
+int fdtd_solver_test_stall_store(fdtd_solver *s)
+{
+    return s && stores_no_d(s->kernel) ? set_stall(s, STALL_STORE) : FDTD_ERR_INVALID;
 }
 
 fdtd_stream_t fdtd_solver_stream(const fdtd_solver *s) { return s ? s->stream : nullptr; }

@@ -39,9 +39,9 @@ __global__ void __launch_bounds__(32 * W + 32) strip_step_kernel(const __grid_co
             asm volatile("griddepcontrol.wait;" ::: "memory");
     }
     __syncthreads();
-    bool stall = false;
+    int stall = 0;
     if (c.stall_once && blockIdx.x == 0 && blockIdx.y == 0 && bz == 0 && threadIdx.x == G::CELL_THREADS)
-        stall = atomicExch(c.stall_once, 0) != 0;
+        stall = atomicExch(c.stall_once, 0);
     const unsigned long long memless =
         c.memless ? c.memless[((size_t)bz * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x] : 0ull;
     strip_unit<RY, W, S, R16>(c, maps, a.zchunk, blockIdx.x, blockIdx.y, bz, memless, sm, stall);

@@ -393,9 +393,10 @@ __device__ __forceinline__ void strip_mur_rows(const StripMove<RY, W, S, R16> &m
 // cell warps have consumed the plane, applies the x-face Mur updates, stores
 // the tiles the cell warps have left in its stage and refills the stage; all
 // but the updates by one elected lane.  Its waits are bounded; when one gives
-// up, or a cell warp's did (the stop word), the copies in flight land (bounded)
-// and the unit ends.  stall: leave the second plane's copies unissued (test
-// hook).
+// up, or a cell warp's did (the stop word), the error flag is raised (where only
+// stores are left the cell warps miss nothing, and the tiles would be lost in
+// silence), the copies in flight land (bounded) and the unit ends.  stall: test
+// hook (STALL_*).
 //
 // A plane's refill waits for this warp, so its own instructions count.  The
 // warp stays together, its lane chosen by elect.sync (the compiler then keeps
@@ -404,24 +405,22 @@ __device__ __forceinline__ void strip_mur_rows(const StripMove<RY, W, S, R16> &m
 // there once (the kernel's loops compete for the instruction cache: 930 us
 // with the first fill apart, 920 so; 512 x 512 x 400, 32-bit R and 16-bit R).
 template <int RY, int W, int S, bool R16>
-__device__ __forceinline__ void strip_run(const StripMove<RY, W, S, R16> &move, const StripXFaces &f, int lane,
-                                          bool stall)
+__device__ __forceinline__ void strip_run(const StripMove<RY, W, S, R16> &move, const StripXFaces &f, int *err,
+                                          int lane, int stall)
 {
     const auto &u = move.u;
     const bool one = elect_one();
-    stall = __any_sync(0xffffffffu, stall);  // one lane was told
+    stall = __shfl_sync(0xffffffffu, stall, 0);  // lane 0 was told
+    const int end = stall == STALL_STORE ? u.zc1 - 1 : u.zc1;
     // the ring's first fill is the loop's first S turns
-    for (int k = -S; u.p0 + k < u.zc1; k++) {
+    int k = -S;
+    for (; u.p0 + k < end; k++) {
         if (k >= 0) {
             bool ok = false;
             if (one)
                 ok = mbar_wait(u.consumed(k), u.parity(k)) && !*static_cast<volatile int *>(u.sm.stop);
-            if (!__any_sync(0xffffffffu, ok)) {
-                if (one)
-                    for (int j = k; j < u.nplanes && j < k + S; j++)
-                        mbar_wait(u.full(j), u.parity(j));
+            if (!__any_sync(0xffffffffu, ok))
                 break;
-            }
             const bool out = u.p0 + k >= u.zc0;
             if (out && (f.near || f.far)) {
                 __syncwarp();  // every lane sees what the waiting lane was given
@@ -434,8 +433,13 @@ __device__ __forceinline__ void strip_run(const StripMove<RY, W, S, R16> &move, 
         }
         if (one && k + S < u.nplanes) {
             bulk_wait_read<0>();  // the refill overwrites the tiles
-            move.issue(k + S, stall && k + S == 1);
+            move.issue(k + S, stall == STALL_LOAD && k + S == 1);
         }
+    }
+    if (one && u.p0 + k < u.zc1) {  // a wait gave up
+        atomicExch(err, 1);
+        for (int j = k; j < u.nplanes && j < k + S; j++)
+            mbar_wait(u.full(j), u.parity(j));
     }
     if (one)
         bulk_wait_all();
@@ -443,11 +447,11 @@ __device__ __forceinline__ void strip_run(const StripMove<RY, W, S, R16> &move, 
 
 // One work unit: column tile (bx, by), z chunk bz of one solve.  memless: bit
 // j set when plane zc0 + j of the tile holds no Debye memory.  stall: the
-// test hook of StripMove.  When a bounded wait gives up the error flag is
+// test hook of strip_run.  When a bounded wait gives up the error flag is
 // raised and the unit ends.
 template <int RY, int W, int S, bool R16, class C>
 __device__ __forceinline__ void strip_unit(const C &c, const StripMaps &maps, int zchunk, int bx, int by,
-                                           int bz, unsigned long long memless, const StripSmem &sm, bool stall)
+                                           int bz, unsigned long long memless, const StripSmem &sm, int stall)
 {
     using G = StripGeo<RY, W, R16>;
     constexpr int TY = G::TY;
@@ -473,7 +477,7 @@ __device__ __forceinline__ void strip_unit(const C &c, const StripMaps &maps, in
             move.faces.bytes = (uint32_t)min(TY, ny - y0) * 16u;
             move.faces.src = face_near ? c.mur_x + y0 : c.mur_x + (size_t)nz * ny + y0;
         }
-        strip_run(move, StripXFaces{c.mur_x, nx, ny, nz, c.scheme, face_near, face_far_cta}, lane, stall);
+        strip_run(move, StripXFaces{c.mur_x, nx, ny, nz, c.scheme, face_near, face_far_cta}, c.err, lane, stall);
         return;
     }
 

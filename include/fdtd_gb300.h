@@ -357,6 +357,10 @@ int fdtd_solver_steps(const fdtd_solver *s);
  * and fdtd_solver_synchronize returns FDTD_ERR_DEVICE_TIMEOUT (once).  The
  * fields of that step are not valid afterwards; the device context is. */
 int fdtd_solver_test_stall(fdtd_solver *s);
+/* The same for the other side of a tile's way (compact forms): the warp that
+ * stores the finished tiles gives up on the first CTA's last plane, which is
+ * not stored.  Reported in the same way. */
+int fdtd_solver_test_stall_store(fdtd_solver *s);
 
 /* Copies the current value of one field (after the last enqueued step) into
  * host memory (nx*ny*nz floats); synchronises the solver first. */
