@@ -55,9 +55,9 @@ constexpr int TX = 64, TY = 2;
 // / 83 / 82 / 90.
 constexpr int H_PLANES = 4, D_PLANES = 4;
 
-__global__ void __launch_bounds__(TX *TY) compat_h_kernel(float *__restrict__ hx, float *__restrict__ hy,
-                                                         float *__restrict__ hz, const float *__restrict__ ex,
-                                                         const float *__restrict__ ey, const float *__restrict__ ez)
+__global__ void __launch_bounds__(TX *TY) compat_h_kernel(float *hx, float *hy,
+                                                         float *hz, const float *ex,
+                                                         const float *ey, const float *ez)
 {
     pdl_begin();
     const int nx = c_sym.nx, ny = c_sym.ny, nz = c_sym.nz;
@@ -72,11 +72,11 @@ __global__ void __launch_bounds__(TX *TY) compat_h_kernel(float *__restrict__ hx
     h_column<H_PLANES>(x, y, blockIdx.y * H_PLANES, nx, ny, nz, nx, kx, ky, kz, ex, ey, ez, in, out);
 }
 
-__global__ void __launch_bounds__(TX *TY) compat_d_kernel(float *__restrict__ dxT, float *__restrict__ dyT,
-                                                         float *__restrict__ dzT, const float *__restrict__ dxS,
-                                                         const float *__restrict__ dyS, const float *__restrict__ dzS,
-                                                         const float *__restrict__ hx, const float *__restrict__ hy,
-                                                         const float *__restrict__ hz)
+__global__ void __launch_bounds__(TX *TY) compat_d_kernel(float *dxT, float *dyT,
+                                                         float *dzT, const float *dxS,
+                                                         const float *dyS, const float *dzS,
+                                                         const float *hx, const float *hy,
+                                                         const float *hz)
 {
     pdl_begin();
     constexpr int K = D_PLANES;
@@ -136,10 +136,10 @@ struct ETriplet {
     const float *e0[3], *e1[3], *d0[3], *d1[3], *d2[3];
 };
 
-__global__ void __launch_bounds__(TX *TY) compat_e_kernel(ETriplet a, const float *__restrict__ sigma,
-                                                         const float *__restrict__ eps_i,
-                                                         const float *__restrict__ eps_s,
-                                                         const float *__restrict__ tau_d)
+__global__ void __launch_bounds__(TX *TY) compat_e_kernel(ETriplet a, const float *sigma,
+                                                         const float *eps_i,
+                                                         const float *eps_s,
+                                                         const float *tau_d)
 {
     pdl_begin();
     const int nx = c_sym.nx, ny = c_sym.ny, nz = c_sym.nz;
@@ -175,8 +175,8 @@ __global__ void __launch_bounds__(TX *TY) compat_e_kernel(ETriplet a, const floa
             a.t[c][i] = debye_update(k, v[c][0], v[c][1], v[c][2], v[c][3], v[c][4]);
 }
 
-__global__ void compat_sources_kernel(float *__restrict__ dzT, const float *__restrict__ dzS,
-                                      const float *__restrict__ hx, const float *__restrict__ hy, int iter)
+__global__ void compat_sources_kernel(float *dzT, const float *dzS,
+                                      const float *hx, const float *hy, int iter)
 {
     pdl_begin();
     const int s = threadIdx.x;

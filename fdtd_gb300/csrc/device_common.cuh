@@ -32,7 +32,10 @@ inline dim3 tile_grid(int nx, int ny, int nz, int tx, int ty, int tz)
 // Programmatic dependent launch: lets the next launch's blocks be placed while
 // this grid finishes, and (before any access to memory) waits for the previous
 // grid to complete.  A stream's order is kept: every kernel launched this way
-// waits before it reads or writes.
+// waits before it reads or writes.  Such a kernel's lifetime begins before the
+// previous grid has ended, so none of its parameters is a const __restrict__
+// pointer: loads of data said to be constant for the kernel's lifetime may take
+// the read-only path, or move ahead of the wait.
 __device__ __forceinline__ void pdl_begin()
 {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

@@ -47,3 +47,16 @@ def test_tensor_maps_in_global_memory_are_acquired_before_use():
         assert 0 <= acquire < use, (file, name)
         assert "__syncthreads();" in body[acquire:use], (file, name)
     assert seen == 2
+
+
+def test_kernels_launched_early_take_no_read_only_pointers():
+    """A programmatic dependent begins while the grid before it still writes:
+    const __restrict__ promises the compiler data constant from the kernel's first
+    instruction on, ahead of griddepcontrol.wait."""
+    seen = 0
+    for file, name, params, body in _kernels():
+        if "pdl_begin();" not in body and "griddepcontrol.wait" not in body:
+            continue
+        seen += 1
+        assert not re.search(r"const\s+\w+\s*\*\s*__restrict__", params + body), (file, name)
+    assert seen >= 8
