@@ -568,6 +568,9 @@ int fdtd_solver_get_field(fdtd_solver *s, int field, float *host_out)
     if (!src)
         return FDTD_ERR_INVALID;
     int st = fdtd_solver_synchronize(s);
+    std::unique_lock<std::mutex> staging(s->scratch_mu, std::defer_lock);
+    if (s->scratch)  // threads that read at once share the staging area
+        staging.lock();
     if (st == FDTD_OK)
         st = cu(read_rows(host_out, src, (size_t)s->ny * s->nz, s->nx, s->pitch, s->scratch, s->scratch_floats,
                           s->stream));

@@ -44,6 +44,7 @@ struct fdtd_solver {
     int *counter = nullptr;
     float *scratch = nullptr;  // padded rows: staging of reads into pageable memory
     size_t scratch_floats = 0;
+    std::mutex scratch_mu;     // held by the thread that reads through it, to the end of its read
     int steps = 0;
     std::map<std::pair<int, int>, cudaGraphExec_t> graphs;  // (parity, length) -> exec
     // snapshots
