@@ -57,6 +57,8 @@ int launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t stream,
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+    if (e != cudaSuccess)
+        cudaGetLastError();  // reported here, not by a later call too
     return e == cudaSuccess ? FDTD_OK : (int)e;
 }
 
