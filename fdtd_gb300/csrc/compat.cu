@@ -277,7 +277,7 @@ int fdtd_update_h(float *hx, float *hy, float *hz, const float *exSource, const 
         return st;
     if (!hx || !hy || !hz || !exSource || !eySource || !ezSource)
         return FDTD_ERR_INVALID;
-    return launch_pdl(compat_h_kernel, cell_grid(s, H_PLANES), dim3(TX, TY), stream, hx, hy, hz, exSource, eySource,
+    return launch_pdl(false, compat_h_kernel, cell_grid(s, H_PLANES), dim3(TX, TY), stream, hx, hy, hz, exSource, eySource,
                       ezSource);
 }
 
@@ -290,7 +290,7 @@ int fdtd_update_d(float *dxTarget, float *dyTarget, float *dzTarget, const float
         return st;
     if (!dxTarget || !dyTarget || !dzTarget || !dxSource || !dySource || !dzSource || !hx || !hy || !hz)
         return FDTD_ERR_INVALID;
-    return launch_pdl(compat_d_kernel, cell_grid(s, D_PLANES), dim3(TX, TY), stream, dxTarget, dyTarget, dzTarget,
+    return launch_pdl(false, compat_d_kernel, cell_grid(s, D_PLANES), dim3(TX, TY), stream, dxTarget, dyTarget, dzTarget,
                       dxSource, dySource, dzSource, hx, hy, hz);
 }
 
@@ -316,7 +316,7 @@ int fdtd_update_e(float *exTarget, float *eyTarget, float *ezTarget, const float
             return FDTD_ERR_INVALID;
     if (!sigma || !epsI || !epsS || !tauD)
         return FDTD_ERR_INVALID;
-    return launch_pdl(compat_e_kernel, cell_grid(s, 1), dim3(TX, TY), stream, a, sigma, epsI, epsS, tauD);
+    return launch_pdl(false, compat_e_kernel, cell_grid(s, 1), dim3(TX, TY), stream, a, sigma, epsI, epsS, tauD);
 }
 
 int fdtd_update_sources(float *dzTarget, const float *dzSource, const float *hx, const float *hy, int currIteration,
@@ -330,7 +330,7 @@ int fdtd_update_sources(float *dzTarget, const float *dzSource, const float *hx,
         return FDTD_ERR_INVALID;
     if (s.nsources == 0)
         return FDTD_OK;
-    return launch_pdl(compat_sources_kernel, dim3(1), dim3(32), stream, dzTarget, dzSource, hx, hy, currIteration);
+    return launch_pdl(false, compat_sources_kernel, dim3(1), dim3(32), stream, dzTarget, dzSource, hx, hy, currIteration);
 }
 
 int fdtd_update_mur(float *exTarget, float *eyTarget, float *ezTarget, const float *exSource, const float *eySource,
@@ -355,7 +355,7 @@ int fdtd_update_mur(float *exTarget, float *eyTarget, float *ezTarget, const flo
     }
     const int rows = (most_v + MUR_ROWS - 1) / MUR_ROWS;
     const dim3 grid((unsigned)((most_u + MUR_THREADS - 1) / MUR_THREADS), (unsigned)std::min(rows, 65535), 12);
-    return launch_pdl(compat_mur_kernel, grid, dim3(MUR_THREADS), stream, a);
+    return launch_pdl(false, compat_mur_kernel, grid, dim3(MUR_THREADS), stream, a);
 }
 
 }  // extern "C"

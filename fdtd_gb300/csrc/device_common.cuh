@@ -42,10 +42,24 @@ __device__ __forceinline__ void pdl_begin()
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
+// Whether stream is being captured (an error is left to the launch to report).
+inline bool capturing(cudaStream_t stream)
+{
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &status) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return status != cudaStreamCaptureStatusNone;
+}
+
 // Launches kernel so that its blocks may be placed before the stream's
-// previous grid completes; the kernel must call pdl_begin() first.
+// previous grid completes; the kernel must call pdl_begin() first.  In a
+// caller's capture the launch is a plain one, unless own_graph says that the
+// graph is this library's: a graph with programmatic edges cannot be read by
+// code that knows plain ones (cudaGraphGetEdges without edge data fails).
 template <class... P, class... A>
-int launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t stream, A &&...args)
+int launch_pdl(bool own_graph, void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t stream, A &&...args)
 {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
@@ -55,7 +69,7 @@ int launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t stream,
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = own_graph || !capturing(stream) ? 1 : 0;
     const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
     if (e != cudaSuccess)
         cudaGetLastError();  // reported here, not by a later call too

@@ -203,7 +203,7 @@ int launch_monitor(fdtd_solver *s, int n)
     // the step that follows them (268 us per step instead of 249, 8 blocks per
     // SM on 224 x 208 x 176) than the launch costs.
     if (!s->dft_on)
-        return launch_pdl(monitor_kernel, dim3(1), dim3(256), s->stream, a);
+        return launch_pdl(true, monitor_kernel, dim3(1), dim3(256), s->stream, a);
     monitor_kernel<<<dft_blocks(), 256, 0, s->stream>>>(a);
     return cu(cudaGetLastError());
 }

@@ -401,7 +401,7 @@ int launch_mur(const NativeConsts &c, cudaStream_t s)
     }
     const int rows = (most_v + MUR_ROWS - 1) / MUR_ROWS;
     const dim3 grid((unsigned)((most_u + MUR_THREADS - 1) / MUR_THREADS), (unsigned)std::min(rows, 65535), 12);
-    return launch_pdl(native_mur_kernel, grid, dim3(MUR_THREADS), s, c);
+    return launch_pdl(c.overlap_prev != 0, native_mur_kernel, grid, dim3(MUR_THREADS), s, c);
 }
 
 int plan_error(const fdtd_plan *p)

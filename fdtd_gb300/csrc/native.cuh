@@ -54,8 +54,8 @@ struct NativeConsts {
     int *err;              // device error flag (a bounded wait gave up)
     int *stall_once;       // test hook, may be null: when set (STALL_*), the first CTA of the next
                            // single-pass launch clears it and lets one of its bounded waits give up
-    int overlap_prev;      // single-pass launch may start while the previous step's Mur kernel runs
-                           // (programmatic dependent launch; only where that kernel precedes it)
+    int overlap_prev;      // a step in the solver's own graphs: its single-pass launch may start
+                           // while the previous step's Mur kernel runs (programmatic dependent)
     int fuse_mur_x;        // the single-pass kernel applies the x-face Mur updates and the Mur
                            // kernel of the same step skips them (set for both launches or neither)
     const float4 *mur_x;   // per x-face cell: 1/(dt+q_self), dt-q_nbr, dt+q_nbr, dt-q_self, [face][z][y]
