@@ -14,6 +14,7 @@
 #include <cstring>
 #include <vector>
 
+#include "rows.h"
 #include "solver_internal.cuh"
 
 using namespace fdtd;
@@ -437,9 +438,11 @@ static int copy_block(fdtd_solver *s, void *dev, char *host, size_t bytes, size_
     const cudaMemcpyKind kind = to_host ? cudaMemcpyDeviceToHost : cudaMemcpyHostToDevice;
     if (elem == 0 || s->pitch == s->nx)
         return cu(cudaMemcpy(dst, src, bytes, kind));
-    const size_t dense = elem * s->nx, padded = elem * s->pitch;
-    return cu(cudaMemcpy2D(dst, to_host ? dense : padded, src, to_host ? padded : dense, dense,
-                           (size_t)s->ny * s->nz, kind));
+    std::lock_guard<std::mutex> staging(s->scratch_mu);
+    const cudaError_t e = move_rows(dev, host, elem, (size_t)s->ny * s->nz, s->nx, s->pitch, s->scratch,
+                                    sizeof(float) * s->scratch_floats, to_host, s->stream);
+    const cudaError_t sync = cudaStreamSynchronize(s->stream);
+    return cu(e == cudaSuccess ? sync : e);
 }
 
 int fdtd_solver_checkpoint(fdtd_solver *s, const char *path)

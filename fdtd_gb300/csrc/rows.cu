@@ -70,14 +70,48 @@ void launch_pack(float *dst, const float *src, size_t first, size_t n, int nx, i
     pack_rows_kernel<<<blocks_for((n + skew + 3) / 4, most), PACK_THREADS, 0, s>>>(dst, src, first, n, nx, pitch, skew);
 }
 
-__global__ void __launch_bounds__(PACK_THREADS) unpack_bytes_kernel(uint8_t *__restrict__ dst,
-                                                                    const uint8_t *__restrict__ src, size_t n,
-                                                                    unsigned nx, unsigned pitch)
+// n elements of dense rows, from `first` on, out of padded rows or (UNPACK) into them.
+template <class T, bool UNPACK>
+__global__ void __launch_bounds__(PACK_THREADS) move_rows_kernel(T *__restrict__ dst, const T *__restrict__ src,
+                                                                 size_t first, size_t n, unsigned nx, unsigned pitch)
 {
     for (size_t i = blockIdx.x * (size_t)PACK_THREADS + threadIdx.x; i < n; i += (size_t)gridDim.x * PACK_THREADS) {
-        const size_t row = i / nx;
-        dst[row * pitch + (i - row * nx)] = src[i];
+        const size_t row = (first + i) / nx, j = row * pitch + (first + i - row * nx);
+        if (UNPACK)
+            dst[j] = src[i];
+        else
+            dst[i] = src[j];
     }
+}
+
+template <class T, bool UNPACK>
+cudaError_t launch_move(T *dst, const T *src, size_t first, size_t n, int nx, int pitch, cudaStream_t s)
+{
+    move_rows_kernel<T, UNPACK><<<blocks_for(n, 152 * 4), PACK_THREADS, 0, s>>>(dst, src, first, n, nx, pitch);
+    return cudaGetLastError();
+}
+
+// A dense host volume to or from padded rows, through scratch in pieces.
+template <class T>
+cudaError_t move_block(void *dev, void *host, size_t n, int nx, int pitch, void *scratch, size_t scratch_bytes,
+                       bool to_host, cudaStream_t s)
+{
+    T *rows = static_cast<T *>(dev), *dense = static_cast<T *>(host), *piece = static_cast<T *>(scratch);
+    const size_t most = scratch_bytes / sizeof(T);
+    cudaError_t e = cudaSuccess;
+    for (size_t o = 0; o < n && e == cudaSuccess; o += most) {
+        const size_t m = std::min(most, n - o);
+        if (to_host) {
+            e = launch_move<T, false>(piece, rows, o, m, nx, pitch, s);
+            if (e == cudaSuccess)
+                e = cudaMemcpyAsync(dense + o, piece, sizeof(T) * m, cudaMemcpyDeviceToHost, s);
+        } else {
+            e = cudaMemcpyAsync(piece, dense + o, sizeof(T) * m, cudaMemcpyHostToDevice, s);
+            if (e == cudaSuccess)
+                e = launch_move<T, true>(rows, piece, o, m, nx, pitch, s);
+        }
+    }
+    return e;
 }
 
 // Whether a kernel may write host memory [p, p + bytes): floats on their own
@@ -146,8 +180,18 @@ cudaError_t write_byte_rows(uint8_t *dst, const uint8_t *host, size_t rows, int 
     const cudaError_t e = cudaMemcpyAsync(scratch, host, n, cudaMemcpyHostToDevice, s);
     if (e != cudaSuccess)
         return e;
-    unpack_bytes_kernel<<<blocks_for(n, 152 * 4), PACK_THREADS, 0, s>>>(dst, scratch, n, nx, pitch);
-    return cudaGetLastError();
+    return launch_move<uint8_t, true>(dst, scratch, 0, n, nx, pitch, s);
+}
+
+cudaError_t move_rows(void *dev, void *host, size_t elem, size_t rows, int nx, int pitch, void *scratch,
+                      size_t scratch_bytes, bool to_host, cudaStream_t s)
+{
+    const size_t n = rows * (size_t)nx;
+    if (scratch_bytes < elem)
+        return cudaErrorInvalidValue;
+    return elem == sizeof(uint16_t)
+               ? move_block<uint16_t>(dev, host, n, nx, pitch, scratch, scratch_bytes, to_host, s)
+               : move_block<uint32_t>(dev, host, n, nx, pitch, scratch, scratch_bytes, to_host, s);
 }
 
 }  // namespace fdtd
