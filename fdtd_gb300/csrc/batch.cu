@@ -838,7 +838,7 @@ int fdtd_batch_read_async(fdtd_batch *b, int id, int field, int z0, int nplanes,
         src = field < 6 ? v->d[slot][comp] : v->e[slot][comp];
     }
     src += (size_t)z0 * v->pitch * v->ny;
-    st = cu(read_rows(host_out, src, (size_t)v->ny * nplanes, v->nx, v->pitch, nullptr, 0, b->stream));
+    st = cu(read_rows(host_out, src, (size_t)v->ny * nplanes, v->nx, v->pitch, nullptr, b->stream));
     if (st != FDTD_OK)
         return st;
     return fdtd_batch_mark(b, ticket);
@@ -944,14 +944,13 @@ int fdtd_batch_get_field(fdtd_batch *b, int id, int field, int z0, int nplanes, 
     src += (size_t)z0 * v->pitch * v->ny;
     // staging for pageable memory (a strided copy where the pool has none left)
     const size_t rows = (size_t)v->ny * nplanes;
-    const size_t floats = v->pitch == v->nx ? 0 : std::min(rows * v->nx, size_t(4) << 20);
+    const size_t floats = v->pitch == v->nx ? 0 : rows * v->nx;
     void *scratch = nullptr;
     if (floats > 0 && pool_alloc(b, &scratch, sizeof(float) * floats, b->stream) != FDTD_OK) {
         scratch = nullptr;
         cudaGetLastError();
     }
-    st = cu(read_rows(host_out, src, rows, v->nx, v->pitch, static_cast<float *>(scratch), scratch ? floats : 0,
-                      b->stream));
+    st = cu(read_rows(host_out, src, rows, v->nx, v->pitch, static_cast<float *>(scratch), b->stream));
     if (scratch)
         cudaFreeAsync(scratch, b->stream);
     const int sync = cu(cudaStreamSynchronize(b->stream));

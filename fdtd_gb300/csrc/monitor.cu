@@ -440,7 +440,7 @@ static int copy_block(fdtd_solver *s, void *dev, char *host, size_t bytes, size_
         return cu(cudaMemcpy(dst, src, bytes, kind));
     std::lock_guard<std::mutex> staging(s->scratch_mu);
     const cudaError_t e = move_rows(dev, host, elem, (size_t)s->ny * s->nz, s->nx, s->pitch, s->scratch,
-                                    sizeof(float) * s->scratch_floats, to_host, s->stream);
+                                    to_host, s->stream);
     const cudaError_t sync = cudaStreamSynchronize(s->stream);
     return cu(e == cudaSuccess ? sync : e);
 }

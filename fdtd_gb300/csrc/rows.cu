@@ -6,7 +6,11 @@
 // are: 10 M floats to page-locked memory at 49 GB/s in rows of 61 and 115 in
 // rows of 217; bytes to the device at 15 - 58 GB/s against 590.  So the rows
 // are packed by a kernel instead: straight into page-locked memory, or through
-// a device scratch area and contiguous copies (164 GB/s into pageable memory).
+// a device scratch area and one contiguous copy.  The scratch area holds the
+// whole volume: in pieces of 16 MB a read into fresh host pages took 33 ms on
+// 301 x 245 x 187 and 18 - 235 on 497 x 500 x 300 (one piece 2.5 and 12.0, as
+// copies of dense rows take), into pages in use 0.39 and 2.00 (0.34 and 1.68; dense
+// 0.31 and 1.58).
 //
 // Page-locked memory is written by the kernel for dense rows as well.  One
 // contiguous copy of 420 MB ran at 107 - 191 GB/s, from one buffer and one
@@ -29,18 +33,18 @@ unsigned blocks_for(size_t n, unsigned most)
     return (unsigned)std::min<size_t>((n + PACK_THREADS - 1) / PACK_THREADS, most);
 }
 
-// n elements of dense rows, from `first` on (an offset into the dense
-// volume).  Each thread writes four at once, on 16 bytes: dst is `skew`
-// elements above such a boundary, and the first and last group may be partial.
+// n elements of dense rows.  Each thread writes four at once, on 16 bytes: dst
+// is `skew` elements above such a boundary, and the first and last group may be
+// partial.
 __global__ void __launch_bounds__(PACK_THREADS) pack_rows_kernel(float *__restrict__ dst,
-                                                                 const float *__restrict__ src, size_t first, size_t n,
-                                                                 unsigned nx, unsigned pitch, unsigned skew)
+                                                                 const float *__restrict__ src, size_t n, unsigned nx,
+                                                                 unsigned pitch, unsigned skew)
 {
     const size_t groups = (n + skew + 3) / 4;
     for (size_t g = blockIdx.x * (size_t)PACK_THREADS + threadIdx.x; g < groups; g += (size_t)gridDim.x * PACK_THREADS) {
         const size_t begin = g == 0 ? 0 : 4 * g - skew, end = min(4 * g + 4 - skew, n);
-        const size_t row = (first + begin) / nx;
-        unsigned x = (unsigned)(first + begin - row * nx);
+        const size_t row = begin / nx;
+        unsigned x = (unsigned)(begin - row * nx);
         const float *p = src + row * pitch + x;
         float v[4];
 #pragma unroll
@@ -64,19 +68,19 @@ __global__ void __launch_bounds__(PACK_THREADS) pack_rows_kernel(float *__restri
     }
 }
 
-void launch_pack(float *dst, const float *src, size_t first, size_t n, int nx, int pitch, unsigned most, cudaStream_t s)
+void launch_pack(float *dst, const float *src, size_t n, int nx, int pitch, unsigned most, cudaStream_t s)
 {
     const unsigned skew = (unsigned)(reinterpret_cast<uintptr_t>(dst) / sizeof(float) % 4);
-    pack_rows_kernel<<<blocks_for((n + skew + 3) / 4, most), PACK_THREADS, 0, s>>>(dst, src, first, n, nx, pitch, skew);
+    pack_rows_kernel<<<blocks_for((n + skew + 3) / 4, most), PACK_THREADS, 0, s>>>(dst, src, n, nx, pitch, skew);
 }
 
-// n elements of dense rows, from `first` on, out of padded rows or (UNPACK) into them.
+// n elements of dense rows, out of padded rows or (UNPACK) into them.
 template <class T, bool UNPACK>
 __global__ void __launch_bounds__(PACK_THREADS) move_rows_kernel(T *__restrict__ dst, const T *__restrict__ src,
-                                                                 size_t first, size_t n, unsigned nx, unsigned pitch)
+                                                                 size_t n, unsigned nx, unsigned pitch)
 {
     for (size_t i = blockIdx.x * (size_t)PACK_THREADS + threadIdx.x; i < n; i += (size_t)gridDim.x * PACK_THREADS) {
-        const size_t row = (first + i) / nx, j = row * pitch + (first + i - row * nx);
+        const size_t row = i / nx, j = row * pitch + (i - row * nx);
         if (UNPACK)
             dst[j] = src[i];
         else
@@ -85,33 +89,23 @@ __global__ void __launch_bounds__(PACK_THREADS) move_rows_kernel(T *__restrict__
 }
 
 template <class T, bool UNPACK>
-cudaError_t launch_move(T *dst, const T *src, size_t first, size_t n, int nx, int pitch, cudaStream_t s)
+cudaError_t launch_move(T *dst, const T *src, size_t n, int nx, int pitch, cudaStream_t s)
 {
-    move_rows_kernel<T, UNPACK><<<blocks_for(n, 152 * 4), PACK_THREADS, 0, s>>>(dst, src, first, n, nx, pitch);
+    move_rows_kernel<T, UNPACK><<<blocks_for(n, 152 * 4), PACK_THREADS, 0, s>>>(dst, src, n, nx, pitch);
     return cudaGetLastError();
 }
 
-// A dense host volume to or from padded rows, through scratch in pieces.
+// A dense host volume to or from padded rows, through scratch.
 template <class T>
-cudaError_t move_block(void *dev, void *host, size_t n, int nx, int pitch, void *scratch, size_t scratch_bytes,
-                       bool to_host, cudaStream_t s)
+cudaError_t move_block(void *dev, void *host, size_t n, int nx, int pitch, void *scratch, bool to_host, cudaStream_t s)
 {
-    T *rows = static_cast<T *>(dev), *dense = static_cast<T *>(host), *piece = static_cast<T *>(scratch);
-    const size_t most = scratch_bytes / sizeof(T);
-    cudaError_t e = cudaSuccess;
-    for (size_t o = 0; o < n && e == cudaSuccess; o += most) {
-        const size_t m = std::min(most, n - o);
-        if (to_host) {
-            e = launch_move<T, false>(piece, rows, o, m, nx, pitch, s);
-            if (e == cudaSuccess)
-                e = cudaMemcpyAsync(dense + o, piece, sizeof(T) * m, cudaMemcpyDeviceToHost, s);
-        } else {
-            e = cudaMemcpyAsync(piece, dense + o, sizeof(T) * m, cudaMemcpyHostToDevice, s);
-            if (e == cudaSuccess)
-                e = launch_move<T, true>(rows, piece, o, m, nx, pitch, s);
-        }
+    T *rows = static_cast<T *>(dev), *dense = static_cast<T *>(scratch);
+    if (to_host) {
+        const cudaError_t e = launch_move<T, false>(dense, rows, n, nx, pitch, s);
+        return e != cudaSuccess ? e : cudaMemcpyAsync(host, dense, sizeof(T) * n, cudaMemcpyDeviceToHost, s);
     }
-    return e;
+    const cudaError_t e = cudaMemcpyAsync(dense, host, sizeof(T) * n, cudaMemcpyHostToDevice, s);
+    return e != cudaSuccess ? e : launch_move<T, true>(rows, dense, n, nx, pitch, s);
 }
 
 // Whether a kernel may write host memory [p, p + bytes): floats on their own
@@ -145,30 +139,23 @@ bool kernel_may_write(const float *p, size_t bytes)
 
 }  // namespace
 
-cudaError_t read_rows(float *host, const float *src, size_t rows, int nx, int pitch, float *scratch,
-                      size_t scratch_floats, cudaStream_t s)
+cudaError_t read_rows(float *host, const float *src, size_t rows, int nx, int pitch, float *scratch, cudaStream_t s)
 {
     const size_t n = rows * (size_t)nx;
     if (n == 0)
         return cudaSuccess;
     if (kernel_may_write(host, sizeof(float) * n)) {
-        launch_pack(host, src, 0, n, nx, pitch, 152, s);
+        launch_pack(host, src, n, nx, pitch, 152, s);
         return cudaGetLastError();
     }
     if (pitch == nx)
         return cudaMemcpyAsync(host, src, sizeof(float) * n, cudaMemcpyDeviceToHost, s);
-    if (!scratch || scratch_floats == 0)
+    if (!scratch)
         return cudaMemcpy2DAsync(host, sizeof(float) * nx, src, sizeof(float) * pitch, sizeof(float) * nx, rows,
                                  cudaMemcpyDeviceToHost, s);
-    cudaError_t e = cudaSuccess;
-    for (size_t o = 0; o < n && e == cudaSuccess; o += scratch_floats) {
-        const size_t m = std::min(scratch_floats, n - o);
-        launch_pack(scratch, src, o, m, nx, pitch, 152 * 4, s);
-        e = cudaGetLastError();
-        if (e == cudaSuccess)
-            e = cudaMemcpyAsync(host + o, scratch, sizeof(float) * m, cudaMemcpyDeviceToHost, s);
-    }
-    return e;
+    launch_pack(scratch, src, n, nx, pitch, 152 * 4, s);
+    const cudaError_t e = cudaGetLastError();
+    return e != cudaSuccess ? e : cudaMemcpyAsync(host, scratch, sizeof(float) * n, cudaMemcpyDeviceToHost, s);
 }
 
 cudaError_t write_byte_rows(uint8_t *dst, const uint8_t *host, size_t rows, int nx, int pitch, uint8_t *scratch,
@@ -180,18 +167,15 @@ cudaError_t write_byte_rows(uint8_t *dst, const uint8_t *host, size_t rows, int 
     const cudaError_t e = cudaMemcpyAsync(scratch, host, n, cudaMemcpyHostToDevice, s);
     if (e != cudaSuccess)
         return e;
-    return launch_move<uint8_t, true>(dst, scratch, 0, n, nx, pitch, s);
+    return launch_move<uint8_t, true>(dst, scratch, n, nx, pitch, s);
 }
 
-cudaError_t move_rows(void *dev, void *host, size_t elem, size_t rows, int nx, int pitch, void *scratch,
-                      size_t scratch_bytes, bool to_host, cudaStream_t s)
+cudaError_t move_rows(void *dev, void *host, size_t elem, size_t rows, int nx, int pitch, void *scratch, bool to_host,
+                      cudaStream_t s)
 {
     const size_t n = rows * (size_t)nx;
-    if (scratch_bytes < elem)
-        return cudaErrorInvalidValue;
-    return elem == sizeof(uint16_t)
-               ? move_block<uint16_t>(dev, host, n, nx, pitch, scratch, scratch_bytes, to_host, s)
-               : move_block<uint32_t>(dev, host, n, nx, pitch, scratch, scratch_bytes, to_host, s);
+    return elem == sizeof(uint16_t) ? move_block<uint16_t>(dev, host, n, nx, pitch, scratch, to_host, s)
+                                    : move_block<uint32_t>(dev, host, n, nx, pitch, scratch, to_host, s);
 }
 
 }  // namespace fdtd

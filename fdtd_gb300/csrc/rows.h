@@ -15,10 +15,9 @@ inline int padded_rows_pitch(int nx) { return nx < 16 ? nx : (nx + 15) & ~15; }
 
 // Queues on s the copy of `rows` rows of nx floats, pitch floats apart, into
 // the dense host volume.  Page-locked memory is written by a kernel, other
-// memory through scratch (device memory that work on s may use, scratch_floats
-// long; without it a strided copy; dense rows are copied as they are).
-cudaError_t read_rows(float *host, const float *src, size_t rows, int nx, int pitch, float *scratch,
-                      size_t scratch_floats, cudaStream_t s);
+// memory through scratch (rows * nx floats of device memory that work on s may
+// use; without it a strided copy; dense rows are copied as they are).
+cudaError_t read_rows(float *host, const float *src, size_t rows, int nx, int pitch, float *scratch, cudaStream_t s);
 
 // Queues on s the copy of a dense host byte volume into rows pitch bytes
 // apart; scratch: rows * nx bytes of device memory (unused where pitch is nx).
@@ -27,9 +26,9 @@ cudaError_t write_byte_rows(uint8_t *dst, const uint8_t *host, size_t rows, int 
 
 // Queues on s the copy of a volume of 2- or 4-byte elements from padded rows
 // on the device to a dense pageable host volume, or back (checkpoints), through
-// scratch.  Strided copies of rows of 17 floats took five times as long as one
+// scratch (rows * nx elements).  Strided copies of rows of 17 floats took five times as long as one
 // copy of dense rows to the device, of 217 half as long again.
-cudaError_t move_rows(void *dev, void *host, size_t elem, size_t rows, int nx, int pitch, void *scratch,
-                      size_t scratch_bytes, bool to_host, cudaStream_t s);
+cudaError_t move_rows(void *dev, void *host, size_t elem, size_t rows, int nx, int pitch, void *scratch, bool to_host,
+                      cudaStream_t s);
 
 }  // namespace fdtd

@@ -83,10 +83,6 @@ namespace {
 
 int cu(cudaError_t e) { return e == cudaSuccess ? FDTD_OK : (int)e; }
 
-// Staging of padded rows read into pageable memory: 16 MB (10 M floats in
-// pieces of 4 MB went as fast as in one piece).
-constexpr size_t PACK_SCRATCH_FLOATS = size_t(4) << 20;
-
 int enqueue_step(fdtd_solver *s, int n)
 {
     NativeConsts c = solver_consts(s, n);
@@ -272,7 +268,7 @@ int enqueue_snapshot(fdtd_solver *s, int step)
     for (size_t k = 0; k < s->snap_fields.size() && st == FDTD_OK; k++) {
         const float *src = field_buffer(s, s->snap_fields[k], step + 1) + (size_t)s->snap.z0 * plane;
         st = cu(read_rows(sl->host + k * s->snap_floats_per_field, src, (size_t)s->snap.nplanes * s->ny, s->nx,
-                          s->pitch, nullptr, 0, s->copy_stream));
+                          s->pitch, nullptr, s->copy_stream));
     }
     if (st == FDTD_OK)
         st = cu(cudaEventRecord(s->ev_copy, s->copy_stream));
@@ -363,18 +359,18 @@ int fdtd_solver_create(const fdtd_solver_config *cfg, fdtd_solver **out)
     // 16 != 0: 4-byte cp.async) and takes 168 on padded ones, the compact form
     // on 301 x 245 x 187 384 and 159.  A grid that only fits with dense rows
     // keeps them.
-    size_t fbytes = 0, dbytes = 0, xbytes = 0, mbytes = 0, total = 0;
+    size_t fbytes = 0, dbytes = 0, xbytes = 0, mbytes = 0, total = 0, staging = 0;
     for (int pitch : {padded_rows_pitch(p->nx), p->nx}) {
         const size_t m = (size_t)pitch * p->ny * p->nz;
         s->pitch = pitch;
         s->pcell = m;
-        s->scratch_floats = pitch == p->nx ? 0 : std::min(n, PACK_SCRATCH_FLOATS);
+        staging = pitch == p->nx ? 0 : n * sizeof(float);
         fbytes = ((m * sizeof(float)) + 255) & ~size_t(255);
         dbytes = r16 ? ((m * sizeof(uint16_t)) + 255) & ~size_t(255) : fbytes;
         xbytes = r16 ? ((r16_words(p->nx, p->ny, p->nz) * sizeof(uint32_t)) + 255) & ~size_t(255) : 0;
         mbytes = (m + 255) & ~size_t(255);
         total = fbytes * (3 * nh + 6) + dbytes * 3 * nd + xbytes + mbytes + 256;
-        st = cu(cudaMalloc(&s->d_block, total + s->scratch_floats * sizeof(float)));
+        st = cu(cudaMalloc(&s->d_block, total + staging));
         if (st != cudaErrorMemoryAllocation || pitch == p->nx)
             break;
         cudaGetLastError();
@@ -403,7 +399,7 @@ int fdtd_solver_create(const fdtd_solver_config *cfg, fdtd_solver **out)
         s->mat = reinterpret_cast<uint8_t *>(q);
         q += mbytes;
         s->counter = reinterpret_cast<int *>(q);
-        if (s->scratch_floats > 0)
+        if (staging > 0)
             s->scratch = reinterpret_cast<float *>(s->d_block + total);
         st = cu(cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking));
     }
@@ -572,8 +568,7 @@ int fdtd_solver_get_field(fdtd_solver *s, int field, float *host_out)
     if (s->scratch)  // threads that read at once share the staging area
         staging.lock();
     if (st == FDTD_OK)
-        st = cu(read_rows(host_out, src, (size_t)s->ny * s->nz, s->nx, s->pitch, s->scratch, s->scratch_floats,
-                          s->stream));
+        st = cu(read_rows(host_out, src, (size_t)s->ny * s->nz, s->nx, s->pitch, s->scratch, s->stream));
     if (st == FDTD_OK)
         st = cu(cudaStreamSynchronize(s->stream));
     return st;

@@ -42,8 +42,7 @@ struct fdtd_solver {
     int memless_rows = 0;                     // tile rows and planes per chunk of those masks
     int memless_zchunk = 0;
     int *counter = nullptr;
-    float *scratch = nullptr;  // padded rows: staging of reads into pageable memory
-    size_t scratch_floats = 0;
+    float *scratch = nullptr;  // padded rows: staging of reads into pageable memory, a volume
     std::mutex scratch_mu;     // held by the thread that reads through it, to the end of its read
     int steps = 0;
     std::map<std::pair<int, int>, cudaGraphExec_t> graphs;  // (parity, length) -> exec
