@@ -12,11 +12,13 @@
 // copies of dense rows take), into pages in use 0.39 and 2.00 (0.34 and 1.68; dense
 // 0.31 and 1.58).
 //
-// Page-locked memory is written by the kernel for dense rows as well.  One
+// Page-locked memory is written by the kernel for long dense rows as well.  One
 // contiguous copy of 420 MB ran at 107 - 191 GB/s, from one buffer and one
 // moment to the next (now and then at a fifth of that); the kernel at 189 -
 // 191 every time, the link's rate, with 16-byte stores from 76 blocks on
-// (4-byte stores: 180 - 185).
+// (4-byte stores: 180 - 185).  Short ones go by the copy engine: reads of 0.13 /
+// 1.0 / 4.2 / 16.8 / 52 / 420 MB took 21.7 / 28.0 / 44.5 / 110 / 294.8 / 2195 us
+// so (in a quiet hour) and 25.5 / 30.3 / 46.8 / 112 / 296.7 / 2205 by the kernel.
 #include <cuda.h>
 
 #include <algorithm>
@@ -144,7 +146,7 @@ cudaError_t read_rows(float *host, const float *src, size_t rows, int nx, int pi
     const size_t n = rows * (size_t)nx;
     if (n == 0)
         return cudaSuccess;
-    if (kernel_may_write(host, sizeof(float) * n)) {
+    if ((pitch != nx || sizeof(float) * n >= LONG_READ_BYTES) && kernel_may_write(host, sizeof(float) * n)) {
         launch_pack(host, src, n, nx, pitch, 152, s);
         return cudaGetLastError();
     }
