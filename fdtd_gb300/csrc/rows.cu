@@ -141,6 +141,12 @@ bool kernel_may_write(const float *p, size_t bytes)
 
 }  // namespace
 
+cudaError_t pack_rows(float *dst, const float *src, size_t rows, int nx, int pitch, cudaStream_t s)
+{
+    launch_pack(dst, src, rows * (size_t)nx, nx, pitch, 152 * 4, s);
+    return cudaGetLastError();
+}
+
 cudaError_t read_rows(float *host, const float *src, size_t rows, int nx, int pitch, float *scratch, cudaStream_t s)
 {
     const size_t n = rows * (size_t)nx;
@@ -155,8 +161,7 @@ cudaError_t read_rows(float *host, const float *src, size_t rows, int nx, int pi
     if (!scratch)
         return cudaMemcpy2DAsync(host, sizeof(float) * nx, src, sizeof(float) * pitch, sizeof(float) * nx, rows,
                                  cudaMemcpyDeviceToHost, s);
-    launch_pack(scratch, src, n, nx, pitch, 152 * 4, s);
-    const cudaError_t e = cudaGetLastError();
+    const cudaError_t e = pack_rows(scratch, src, rows, nx, pitch, s);
     return e != cudaSuccess ? e : cudaMemcpyAsync(host, scratch, sizeof(float) * n, cudaMemcpyDeviceToHost, s);
 }
 

@@ -24,6 +24,9 @@ constexpr size_t LONG_READ_BYTES = size_t(64) << 20;
 // dense rows are copied as they are).
 cudaError_t read_rows(float *host, const float *src, size_t rows, int nx, int pitch, float *scratch, cudaStream_t s);
 
+// Queues on s the packing of such rows into device memory.
+cudaError_t pack_rows(float *dst, const float *src, size_t rows, int nx, int pitch, cudaStream_t s);
+
 // Queues on s the copy of a dense host byte volume into rows pitch bytes
 // apart; scratch: rows * nx bytes of device memory (unused where pitch is nx).
 cudaError_t write_byte_rows(uint8_t *dst, const uint8_t *host, size_t rows, int nx, int pitch, uint8_t *scratch,

@@ -256,19 +256,35 @@ int enqueue_snapshot(fdtd_solver *s, int step)
     }
     int st = FDTD_OK;
     if (s->copy_pending) {
-        // The previous copy read buffers that the next step overwrites.
+        // The previous copy reads buffers that the next step or this pack overwrites.
         st = cu(cudaStreamWaitEvent(s->stream, s->ev_copy, 0));
         s->copy_pending = false;
     }
+    // The copy engine takes the planes to the host beside the next steps (a
+    // kernel that waits for the link holds its SMs' slots).  Padded rows are
+    // packed first, in the steps' stream: a pack beside a step waits for its
+    // blocks to leave.  us per step with every E volume taken after every step,
+    // by the writing kernel and so: D form, 512 x 512 x 200 4000 and 3377, 217 x
+    // 253 x 181 815 and 704; 16-bit R 3726 and 3362, 772 and 701.
+    const size_t plane = (size_t)s->pitch * s->ny, per = s->snap_floats_per_field, nf = s->snap_fields.size();
+    const size_t rows = (size_t)s->snap.nplanes * s->ny;
+    const auto src = [&](size_t k) { return field_buffer(s, s->snap_fields[k], step + 1) + s->snap.z0 * plane; };
+    for (size_t k = 0; k < nf && s->snap_scratch && st == FDTD_OK; k++)
+        st = cu(pack_rows(s->snap_scratch + k * per, src(k), rows, s->nx, s->pitch, s->stream));
     if (st == FDTD_OK)
         st = cu(cudaEventRecord(s->ev_step, s->stream));
     if (st == FDTD_OK)
         st = cu(cudaStreamWaitEvent(s->copy_stream, s->ev_step, 0));
-    const size_t plane = (size_t)s->pitch * s->ny;
-    for (size_t k = 0; k < s->snap_fields.size() && st == FDTD_OK; k++) {
-        const float *src = field_buffer(s, s->snap_fields[k], step + 1) + (size_t)s->snap.z0 * plane;
-        st = cu(read_rows(sl->host + k * s->snap_floats_per_field, src, (size_t)s->snap.nplanes * s->ny, s->nx,
-                          s->pitch, nullptr, s->copy_stream));
+    if (s->snap_scratch) {
+        if (st == FDTD_OK)
+            st = cu(cudaMemcpyAsync(sl->host, s->snap_scratch, sizeof(float) * per * nf, cudaMemcpyDeviceToHost,
+                                    s->copy_stream));
+    } else {
+        for (size_t k = 0; k < nf && st == FDTD_OK; k++)
+            st = cu(s->pitch == s->nx
+                        ? cudaMemcpyAsync(sl->host + k * per, src(k), sizeof(float) * per, cudaMemcpyDeviceToHost,
+                                          s->copy_stream)
+                        : read_rows(sl->host + k * per, src(k), rows, s->nx, s->pitch, nullptr, s->copy_stream));
     }
     if (st == FDTD_OK)
         st = cu(cudaEventRecord(s->ev_copy, s->copy_stream));
@@ -299,6 +315,9 @@ void free_ring(fdtd_solver *s)
         if (sl.host)
             cudaFreeHost(sl.host);
     s->ring.clear();
+    if (s->snap_scratch)
+        cudaFree(s->snap_scratch);
+    s->snap_scratch = nullptr;
 }
 
 }  // namespace
@@ -618,6 +637,12 @@ int fdtd_solver_set_snapshots(fdtd_solver *s, const fdtd_snapshot_spec *spec)
             s->snap_fields.clear();
             return st;
         }
+    }
+    size_t free_bytes = 0, all_bytes = 0;
+    if (s->pitch != s->nx && cudaMemGetInfo(&free_bytes, &all_bytes) == cudaSuccess && bytes <= free_bytes / 4 &&
+        cudaMalloc(&s->snap_scratch, bytes) != cudaSuccess) {
+        s->snap_scratch = nullptr;
+        cudaGetLastError();
     }
     s->ring_next = 0;
     s->snap = sp;

@@ -51,6 +51,7 @@ struct fdtd_solver {
     std::string snap_dir;
     std::vector<int> snap_fields;
     size_t snap_floats_per_field = 0;
+    float *snap_scratch = nullptr;  // padded rows: staging of a snapshot's planes
     std::vector<fdtd::SnapshotSlot> ring;
     int ring_next = 0;
     cudaEvent_t ev_step = nullptr, ev_copy = nullptr;
