@@ -2,8 +2,8 @@
 //
 // Same argument lists and per-component index ranges as the reference's five
 // kernels, over the reference's float material arrays and three-slot state.
-// The grids differ: 64 x 2 thread tiles (of several z planes for H and D)
-// instead of 128 x 1 rows, sources as one warp instead of a full grid, Mur over
+// The grids differ: thread tiles (of several z planes for H and D) instead of
+// 128 x 1 rows, sources as one warp instead of a full grid, Mur over
 // the face cells only.  The kernels are programmatic dependents of the stream's
 // previous launch: one after another on a small grid they took 4.2-5.4 us each,
 // so 2.7-4.
@@ -44,8 +44,17 @@ int current_device_checked(int *dev)
 
 // Thread tile: long rows share their 32-byte sectors and E and H neighbours within
 // a block (five launchers on 256 x 256 x 200: 343 us with 32 x 8, 338 with 64 x 2, 335
-// with 256 x 1, which leaves most threads of a narrow grid idle)
-constexpr int TX = 64, TY = 2;
+// with 256 x 1).  Narrow grids take the power of two that holds a row, so that no
+// more than half of the threads idle: E kernel on 8 x 600 x 600 182 us in 64 x 2
+// tiles, 43 so (32 x 8: 115), 16 x 512 x 512 133 and 58 (95), 32 x 512 x 256 68 and
+// 57 (64).
+constexpr int TILE_THREADS = 128;
+
+dim3 cell_tile(int nx)
+{
+    const int tx = nx <= 8 ? 8 : nx <= 16 ? 16 : nx <= 32 ? 32 : 64;
+    return dim3(tx, TILE_THREADS / tx);
+}
 
 // z planes per thread of the H and D kernels, bound by HBM (36 bytes per cell).
 // With one plane per thread, each component loaded, updated and stored in
@@ -55,13 +64,13 @@ constexpr int TX = 64, TY = 2;
 // / 83 / 82 / 90.
 constexpr int H_PLANES = 4, D_PLANES = 4;
 
-__global__ void __launch_bounds__(TX *TY) compat_h_kernel(float *hx, float *hy,
+__global__ void __launch_bounds__(TILE_THREADS) compat_h_kernel(float *hx, float *hy,
                                                          float *hz, const float *ex,
                                                          const float *ey, const float *ez)
 {
     pdl_begin();
     const int nx = c_sym.nx, ny = c_sym.ny, nz = c_sym.nz;
-    const TileXY t(nx, TX, TY);
+    const TileXY t(nx, blockDim.x, blockDim.y);
     const int x = t.x0 + threadIdx.x, y = t.y0 + threadIdx.y;
     if (x >= nx - 1 || y >= ny - 1)
         return;
@@ -72,7 +81,7 @@ __global__ void __launch_bounds__(TX *TY) compat_h_kernel(float *hx, float *hy,
     h_column<H_PLANES>(x, y, blockIdx.y * H_PLANES, nx, ny, nz, nx, kx, ky, kz, ex, ey, ez, in, out);
 }
 
-__global__ void __launch_bounds__(TX *TY) compat_d_kernel(float *dxT, float *dyT,
+__global__ void __launch_bounds__(TILE_THREADS) compat_d_kernel(float *dxT, float *dyT,
                                                          float *dzT, const float *dxS,
                                                          const float *dyS, const float *dzS,
                                                          const float *hx, const float *hy,
@@ -81,7 +90,7 @@ __global__ void __launch_bounds__(TX *TY) compat_d_kernel(float *dxT, float *dyT
     pdl_begin();
     constexpr int K = D_PLANES;
     const int nx = c_sym.nx, ny = c_sym.ny, nz = c_sym.nz;
-    const TileXY t(nx, TX, TY);
+    const TileXY t(nx, blockDim.x, blockDim.y);
     const int x = t.x0 + threadIdx.x, y = t.y0 + threadIdx.y, z0 = blockIdx.y * K;
     if (x >= nx - 1 || y >= ny - 1)
         return;  // no D component is updated at x = nx-1, y = ny-1 or z = nz-1
@@ -136,14 +145,14 @@ struct ETriplet {
     const float *e0[3], *e1[3], *d0[3], *d1[3], *d2[3];
 };
 
-__global__ void __launch_bounds__(TX *TY) compat_e_kernel(ETriplet a, const float *sigma,
+__global__ void __launch_bounds__(TILE_THREADS) compat_e_kernel(ETriplet a, const float *sigma,
                                                          const float *eps_i,
                                                          const float *eps_s,
                                                          const float *tau_d)
 {
     pdl_begin();
     const int nx = c_sym.nx, ny = c_sym.ny, nz = c_sym.nz;
-    const TileXY t(nx, TX, TY);
+    const TileXY t(nx, blockDim.x, blockDim.y);
     const int x = t.x0 + threadIdx.x, y = t.y0 + threadIdx.y, z = blockIdx.y;
     if (x >= nx || y >= ny)
         return;
@@ -224,7 +233,11 @@ int prologue(SymbolBlock *sym)
 }
 
 // The cells in columns of `planes` z planes.
-dim3 cell_grid(const SymbolBlock &s, int planes) { return tile_grid(s.nx, s.ny, s.nz, TX, TY, planes); }
+dim3 cell_grid(const SymbolBlock &s, int planes)
+{
+    const dim3 t = cell_tile(s.nx);
+    return tile_grid(s.nx, s.ny, s.nz, t.x, t.y, planes);
+}
 
 }  // namespace
 }  // namespace fdtd
@@ -277,7 +290,7 @@ int fdtd_update_h(float *hx, float *hy, float *hz, const float *exSource, const 
         return st;
     if (!hx || !hy || !hz || !exSource || !eySource || !ezSource)
         return FDTD_ERR_INVALID;
-    return launch_pdl(false, compat_h_kernel, cell_grid(s, H_PLANES), dim3(TX, TY), stream, hx, hy, hz, exSource, eySource,
+    return launch_pdl(false, compat_h_kernel, cell_grid(s, H_PLANES), cell_tile(s.nx), stream, hx, hy, hz, exSource, eySource,
                       ezSource);
 }
 
@@ -290,7 +303,7 @@ int fdtd_update_d(float *dxTarget, float *dyTarget, float *dzTarget, const float
         return st;
     if (!dxTarget || !dyTarget || !dzTarget || !dxSource || !dySource || !dzSource || !hx || !hy || !hz)
         return FDTD_ERR_INVALID;
-    return launch_pdl(false, compat_d_kernel, cell_grid(s, D_PLANES), dim3(TX, TY), stream, dxTarget, dyTarget, dzTarget,
+    return launch_pdl(false, compat_d_kernel, cell_grid(s, D_PLANES), cell_tile(s.nx), stream, dxTarget, dyTarget, dzTarget,
                       dxSource, dySource, dzSource, hx, hy, hz);
 }
 
@@ -316,7 +329,7 @@ int fdtd_update_e(float *exTarget, float *eyTarget, float *ezTarget, const float
             return FDTD_ERR_INVALID;
     if (!sigma || !epsI || !epsS || !tauD)
         return FDTD_ERR_INVALID;
-    return launch_pdl(false, compat_e_kernel, cell_grid(s, 1), dim3(TX, TY), stream, a, sigma, epsI, epsS, tauD);
+    return launch_pdl(false, compat_e_kernel, cell_grid(s, 1), cell_tile(s.nx), stream, a, sigma, epsI, epsS, tauD);
 }
 
 int fdtd_update_sources(float *dzTarget, const float *dzSource, const float *hx, const float *hy, int currIteration,
