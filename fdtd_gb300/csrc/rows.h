@@ -13,6 +13,28 @@ namespace fdtd {
 // that padding never doubles a state.
 inline int padded_rows_pitch(int nx) { return nx < 16 ? nx : (nx + 15) & ~15; }
 
+// Row pitch of a single solve's arrays: padded where the padded rows' kernels
+// gain by it and the memory is there.  us per step on dense and padded rows:
+// * Compact forms: the strip kernel against the z-marching kernel fed by 4-byte
+//   cp.async; 301 x 245 x 187 384 and 159, 17 x 300 x 300 100 and 53.
+// * D form, the single-pass kernel (97 bytes per cell of a padded row) against
+//   the two-pass kernels (121 per cell): 217 x 253 x 181 208 and 165, 49 x 300 x
+//   300 (padding 1.31) 112 and 104, 36 (1.33) 100 and 101, 33 (1.45) 86 and 107, 17
+//   (1.88) 50 and 59.  Up to 4/3.
+// * Two-pass kernels need no TMA: 217 x 253 x 181 206 and 207, 44 x 300 x 300 103
+//   and 109, 17 51 and 63.  Never.
+// The padding, and the volume that stages reads of padded rows, may take a quarter
+// of what dense rows would leave free (cell_bytes: the state's bytes per cell), so
+// that monitors and other solves keep their room.
+inline int solve_rows_pitch(int nx, size_t rows, bool two_pass, bool compact, size_t cell_bytes, size_t free_bytes)
+{
+    const int pitch = padded_rows_pitch(nx);
+    if (two_pass || (!compact && 3ll * pitch > 4ll * nx))
+        return nx;
+    const size_t dense = rows * nx * cell_bytes, extra = rows * (pitch - nx) * cell_bytes + rows * nx * sizeof(float);
+    return free_bytes > dense && extra <= (free_bytes - dense) / 4 ? pitch : nx;
+}
+
 // Dense rows from here on are read into page-locked memory by a kernel: it costs
 // 0.6 % there (52 MB: 0.7 %), below up to 15 %.
 constexpr size_t LONG_READ_BYTES = size_t(64) << 20;

@@ -373,13 +373,16 @@ int fdtd_solver_create(const fdtd_solver_config *cfg, fdtd_solver **out)
     const bool r16 = cfg->kernel == FDTD_KERNEL_COMPACT_R16;
     const int nh = cfg->kernel == FDTD_KERNEL_TWO_PASS ? 1 : 2;
     const int nd = stores_no_d(cfg->kernel) ? 1 : 2;
-    // Rows are padded to a multiple of 16 cells so that every solve gets TMA
-    // staging: a 217 x 253 x 181 D-form step took 382 us on dense rows (nx %
-    // 16 != 0: 4-byte cp.async) and takes 168 on padded ones, the compact form
-    // on 301 x 245 x 187 384 and 159.  A grid that only fits with dense rows
-    // keeps them.
+    // Rows may be padded to a multiple of 16 cells for TMA (solve_rows_pitch).
+    // A grid that only fits with dense rows keeps them.
+    const size_t cell_bytes = sizeof(float) * (3 * nh + 6) + (r16 ? sizeof(uint16_t) : sizeof(float)) * 3 * nd + 1;
+    size_t free_bytes = 0, all_bytes = 0;
+    if (cudaMemGetInfo(&free_bytes, &all_bytes) != cudaSuccess)
+        cudaGetLastError();  // not known: dense rows
+    const int wanted = solve_rows_pitch(p->nx, (size_t)p->ny * p->nz, cfg->kernel == FDTD_KERNEL_TWO_PASS,
+                                        stores_no_d(cfg->kernel), cell_bytes, free_bytes);
     size_t fbytes = 0, dbytes = 0, xbytes = 0, mbytes = 0, total = 0, staging = 0;
-    for (int pitch : {padded_rows_pitch(p->nx), p->nx}) {
+    for (int pitch : {wanted, p->nx}) {
         const size_t m = (size_t)pitch * p->ny * p->nz;
         s->pitch = pitch;
         s->pcell = m;
