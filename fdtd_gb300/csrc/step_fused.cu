@@ -1097,6 +1097,15 @@ int launch_batch_step(const BatchLaunch &b, cudaStream_t s)
     return e == cudaSuccess ? FDTD_OK : (int)e;
 }
 
+// The two-pass D/E kernel as the second half of a single-pass step.
+static int launch_de_single_pass(const NativeConsts &c0, cudaStream_t s)
+{
+    NativeConsts c = c0;
+    c.h_edges_in = 1;
+    c.class_last = c.nclasses - 1;
+    return launch_de(c, s);
+}
+
 int launch_h_de_fused(const NativeConsts &c, cudaStream_t s)
 {
     FusedArgs a;
@@ -1111,10 +1120,8 @@ int launch_h_de_fused(const NativeConsts &c, cudaStream_t s)
     // single-pass kernel reading straight from global memory (tried, not
     // kept): 250 x 239 x 160 324 / 202 / 191, 123 x 131 x 90 76 / 35 / 40, 498
     // x 300 x 200 - / 604 / 575.
-    a.c.h_edges_in = 1;
-    a.c.class_last = c.nclasses - 1;
-    const int st = launch_h(a.c, s);
-    return st == FDTD_OK ? launch_de(a.c, s) : st;
+    const int st = launch_h(c, s);
+    return st == FDTD_OK ? launch_de_single_pass(c, s) : st;
 }
 
 // The compact forms run the strip kernel (step_strip.cu) wherever its TMA
@@ -1191,17 +1198,20 @@ int launch_step_compact16(const NativeConsts &c0, cudaStream_t s)
     return st;
 }
 
-int step_kernels(int kernel_kind, const NativeConsts &, StepKernel *out, int max)
+int step_kernels(int kernel_kind, const NativeConsts &c, StepKernel *out, int max)
 {
     static const StepKernel single[] = {{"fused_step", launch_h_de_fused}, {"mur", launch_mur}};
+    static const StepKernel untiled[] = {{"h", launch_h}, {"de", launch_de_single_pass}, {"mur", launch_mur}};
     static const StepKernel compact[] = {{"compact_step", launch_h_e_compact}, {"mur", launch_mur}};
     static const StepKernel compact16[] = {{"compact16_step", launch_h_e_compact16}, {"mur", launch_mur}};
     static const StepKernel two[] = {{"h", launch_h}, {"de", launch_de}, {"mur", launch_mur}};
-    const StepKernel *src = kernel_kind == FDTD_KERNEL_SINGLE_PASS ? single
-                            : kernel_kind == FDTD_KERNEL_COMPACT   ? compact
+    const bool no_tiles = kernel_kind == FDTD_KERNEL_SINGLE_PASS && !fused_uses_tma(c);
+    const StepKernel *src = no_tiles                                 ? untiled
+                            : kernel_kind == FDTD_KERNEL_SINGLE_PASS ? single
+                            : kernel_kind == FDTD_KERNEL_COMPACT     ? compact
                             : kernel_kind == FDTD_KERNEL_COMPACT_R16 ? compact16
                                                                      : two;
-    const int n = kernel_kind == FDTD_KERNEL_TWO_PASS ? 3 : 2;
+    const int n = no_tiles || kernel_kind == FDTD_KERNEL_TWO_PASS ? 3 : 2;
     for (int k = 0; k < n && k < max; k++)
         out[k] = src[k];
     return n;

@@ -252,11 +252,14 @@ int fdtd_step_h(const fdtd_plan *plan, const fdtd_native_fields *f, fdtd_stream_
  * faces of step n.  Reads H^{n+1/2} from hx_out..hz_out. */
 int fdtd_step_de(const fdtd_plan *plan, const fdtd_native_fields *f, int n, fdtd_stream_t stream);
 
-/* Whole step n in one z-marching pass plus the Mur faces.  hx_out..hz_out
- * must not alias hx..hz (H is double-buffered). */
+/* Whole step n: one z-marching pass plus the Mur faces where rows are a
+ * multiple of 16 cells and the arrays lie on 16 bytes (TMA addresses them), the
+ * kernels of fdtd_step_h and fdtd_step_de elsewhere.  hx_out..hz_out must not
+ * alias hx..hz (H is double-buffered).  A class byte beyond the plan's classes
+ * takes the last one. */
 int fdtd_step(const fdtd_plan *plan, const fdtd_native_fields *f, int n, fdtd_stream_t stream);
 
-/* One single-pass step (as fdtd_step) that allocates no device memory.
+/* One step (by the kernels that fdtd_step would take) that allocates no device memory.
  * No counterpart in the reference.  For callers that cannot call cudaMalloc:
  * a process whose device memory belongs to another allocator (a framework's
  * caching pool, a budget fixed at start-up) or code where an allocation is
@@ -290,7 +293,8 @@ int fdtd_step_static(const FdtdParams *p, const float *specs, int nclasses, int 
 typedef struct fdtd_solver fdtd_solver;
 
 enum {
-    FDTD_KERNEL_SINGLE_PASS = 0,  /* fdtd_step: one z-marching kernel per step */
+    FDTD_KERNEL_SINGLE_PASS = 0,  /* fdtd_step: one z-marching kernel per step, or the two-pass kernels
+                                   * where the solver keeps rows that TMA cannot address */
     FDTD_KERNEL_TWO_PASS = 1,     /* fdtd_step_h + fdtd_step_de */
     /* Single pass over nine stored fields instead of fifteen: D and E^{n-1}
      * are folded into one recursion variable per component,
