@@ -367,16 +367,13 @@ int rebuild(fdtd_batch *b)
     for (size_t i = 0; i < b->solves.size(); i++) {
         const BatchSolve *v = b->solves[i];
         const BatchDesc &d = descs[i];
-        if (strip && (d.tiles_x > 65535 || d.tiles_y > 65535 || d.chunks > 65535 || d.zchunk > 65535))
-            return FDTD_ERR_INVALID;
         if (strip)
             strip_unit_masks(v->memless8, v->nx, v->ny, v->nz, ty, d.zchunk, masks.data() + d.unit_begin);
         for (int j = 0; j < d.unit_count; j++) {
             const int per_z = d.tiles_x * d.tiles_y, rem = j % per_z;
             recs[(size_t)d.unit_begin + j] =
-                BatchUnit{masks[(size_t)d.unit_begin + j], v->counter,           (int)i,
-                          (unsigned short)(rem % d.tiles_x), (unsigned short)(rem / d.tiles_x),
-                          (unsigned short)(j / per_z),       (unsigned short)d.zchunk, d.steps_target};
+                BatchUnit{masks[(size_t)d.unit_begin + j], v->counter,      (int)i,    d.steps_target,
+                          rem % d.tiles_x,                 rem / d.tiles_x, j / per_z, d.zchunk};
         }
     }
     if (st == FDTD_OK && recs.size() > b->units_cap) {

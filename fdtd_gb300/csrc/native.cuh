@@ -203,15 +203,17 @@ struct alignas(128) BatchDesc {
 // kernel works out the tile and chunk from the index itself): the planes
 // of its tile that hold no Debye memory (bit j: plane zc0 + j), its solve's
 // step counter and step target, the solve, the tile (bx, by), the z chunk bz
-// and the chunk length.
+// and the chunk length.  Whole words: with 16-bit fields for tile, chunk
+// and length, one more use of them in the strip kernel ("is this the solve's
+// first unit?") made nvcc 13.0.88 compile it so that every block read by as 0 and
+// others wrong, at -Xptxas -O1 to -O3; the same source reads words right.
 struct alignas(16) BatchUnit {
     unsigned long long memless;
     const int *counter;
-    int solve;
-    unsigned short bx, by, bz, zchunk;
-    int steps_target;
+    int solve, steps_target;
+    int bx, by, bz, zchunk;
 };
-static_assert(sizeof(BatchUnit) == 32, "two 16-byte copies per record");
+static_assert(sizeof(BatchUnit) == 48, "three 16-byte copies per record");
 
 // First word of a solve's row in BatchLaunch::seen.
 __host__ __device__ constexpr size_t batch_seen_row(int solve, int par)

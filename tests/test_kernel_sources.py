@@ -60,3 +60,14 @@ def test_kernels_launched_early_take_no_read_only_pointers():
         seen += 1
         assert not re.search(r"const\s+\w+\s*\*\s*__restrict__", params + body), (file, name)
     assert seen >= 8
+
+
+def test_records_of_the_batched_kernels_have_no_fields_shorter_than_a_word():
+    """16-bit fields of a work unit's record were read wrong by compiled code."""
+    text = re.sub(r"//[^\n]*", "", (CSRC / "native.cuh").read_text())
+    for name in ("BatchUnit", "BatchMurBlock"):
+        body = re.search(rf"struct[^;{{]*\b{name}\s*{{([^}}]*)}}", text).group(1)
+        fields = [f.strip() for f in body.split(";") if f.strip()]
+        assert fields, name
+        for f in fields:
+            assert not re.search(r"\b(short|char|u?int8_t|u?int16_t|bool)\b", f), (name, f)
