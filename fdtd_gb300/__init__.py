@@ -150,6 +150,7 @@ def lib() -> C.CDLL:
         _sig(L, "fdtd_solver_synchronize", _I, _V)
         _sig(L, "fdtd_solver_test_stall", _I, _V)
         _sig(L, "fdtd_solver_test_stall_store", _I, _V)
+        _sig(L, "fdtd_batch_test_stall", _I, _V, _I)
         _sig(L, "fdtd_solver_steps", _I, _V)
         _sig(L, "fdtd_solver_get_field", _I, _V, _I, _P)
         _sig(L, "fdtd_solver_stream", _V, _V)
@@ -521,6 +522,10 @@ class Batch:
 
     def synchronize(self) -> None:
         check(lib().fdtd_batch_synchronize(self.handle), "fdtd_batch_synchronize")
+
+    def test_stall(self, sid: int) -> None:
+        """Solver.test_stall for the first unit of one solve (D form)."""
+        check(lib().fdtd_batch_test_stall(self.handle, sid), "fdtd_batch_test_stall")
 
     def autotune(self, steps_per_trial: int = 16) -> int:
         """Times each candidate z-chunk limit on the current solves (the trial

@@ -56,6 +56,7 @@ struct BatchSolve {
     uint32_t *rexp = nullptr;  // 16-bit R form: scale words
     int *counter = nullptr;
     int host_steps = 0;              // steps queued for this solve so far (its counter once they ran)
+    int stall = 0;                   // test hook of the next run's steps (BatchUnit::stall)
     cudaEvent_t ready = nullptr;     // its uploads on the side stream; waited for before its first step
     std::vector<unsigned char> memless8;  // compact forms: tile-planes (32 x 8) without Debye memory
 };
@@ -372,8 +373,9 @@ int rebuild(fdtd_batch *b)
         for (int j = 0; j < d.unit_count; j++) {
             const int per_z = d.tiles_x * d.tiles_y, rem = j % per_z;
             recs[(size_t)d.unit_begin + j] =
-                BatchUnit{masks[(size_t)d.unit_begin + j], v->counter,      (int)i,    d.steps_target,
-                          rem % d.tiles_x,                 rem / d.tiles_x, j / per_z, d.zchunk};
+                BatchUnit{masks[(size_t)d.unit_begin + j], v->counter,      (int)i,          d.steps_target,
+                          j == 0 ? v->stall : 0,           rem % d.tiles_x, rem / d.tiles_x, j / per_z,
+                          d.zchunk};
         }
     }
     if (st == FDTD_OK && recs.size() > b->units_cap) {
@@ -706,6 +708,11 @@ int fdtd_batch_run(fdtd_batch *b, int nsteps)
             st = cu(cudaGraphLaunch(g, b->stream));
         nsteps -= len;
     }
+    for (auto *v : b->solves)
+        if (v->stall) {  // the hook was for these steps
+            v->stall = 0;
+            b->dirty = true;
+        }
     if (b->timing && st == FDTD_OK) {
         st = cu(cudaEventRecord(t1, b->stream));
         if (st == FDTD_OK)
@@ -799,6 +806,16 @@ int fdtd_batch_synchronize(fdtd_batch *b)
     if (b->timing)
         collect_runs(b);
     return st;
+}
+
+int fdtd_batch_test_stall(fdtd_batch *b, int id)
+{
+    BatchSolve *v = b && !b->compact ? find(b, id) : nullptr;
+    if (!v)
+        return FDTD_ERR_INVALID;
+    v->stall = STALL_LOAD;
+    b->dirty = true;  // the units' records are made anew
+    return FDTD_OK;
 }
 
 int fdtd_batch_read_async(fdtd_batch *b, int id, int field, int z0, int nplanes, float *host_out,

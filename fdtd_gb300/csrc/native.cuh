@@ -211,6 +211,7 @@ struct alignas(16) BatchUnit {
     unsigned long long memless;
     const int *counter;
     int solve, steps_target;
+    int stall;  // test hook, D form: this unit's bounded wait gives up (STALL_LOAD)
     int bx, by, bz, zchunk;
 };
 static_assert(sizeof(BatchUnit) == 48, "three 16-byte copies per record");

@@ -785,7 +785,7 @@ __global__ void __launch_bounds__((fused_threads<TY, !COMPACT>()), COMPACT ? 4 :
     __syncthreads();
     const int local = (int)blockIdx.x - d.unit_begin, per_z = d.tiles_x * d.tiles_y, rem = local % per_z;
     fused_unit<TY, S, true, !COMPACT, COMPACT, R16>(s_c, d.maps[par], d.zchunk, rem % d.tiles_x, rem / d.tiles_x, local / per_z,
-                                          smem, coef, bars);
+                                          smem, coef, bars, rec.stall != 0);
 }
 
 __global__ void __launch_bounds__(256) batch_mur_kernel(const BatchDesc *__restrict__ descs,

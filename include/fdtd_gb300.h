@@ -510,6 +510,11 @@ int fdtd_batch_autotune(fdtd_batch *b, int steps_per_trial, int *chosen);
  * pair. */
 int fdtd_batch_tuning(const fdtd_batch *b, int *zchunk_max, int *tile_rows, int *strip_shape);
 int fdtd_batch_synchronize(fdtd_batch *b);
+/* fdtd_solver_test_stall for the first work unit of solve id, in every step of
+ * the next fdtd_batch_run: the fdtd_batch_synchronize after it returns
+ * FDTD_ERR_DEVICE_TIMEOUT (once).  D form only: the compact forms' units are the
+ * single solver's, where the hook costs nothing. */
+int fdtd_batch_test_stall(fdtd_batch *b, int id);
 /* Completed steps of one solve (synchronises; -1 on error). */
 int fdtd_batch_steps(fdtd_batch *b, int id);
 /* Copies planes [z0, z0 + nplanes) (nplanes 0 = all) of one field of one
