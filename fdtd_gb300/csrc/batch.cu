@@ -115,7 +115,7 @@ struct fdtd_batch {
     size_t descs_cap = 0;
     BatchMurBlock *d_mur = nullptr;
     size_t mur_cap = 0;
-    int *d_work = nullptr;
+    int *d_err = nullptr;  // set by a bounded wait that gave up
     BatchLaunch launch{};
     std::map<int, cudaGraphExec_t> graphs;  // steps per graph -> exec
     size_t bytes = 0;
@@ -251,9 +251,6 @@ NativeConsts solve_consts(const BatchSolve *v, int parity, int *err)
     return c;
 }
 
-// Word of the batch's work buffer that a bounded wait which gave up sets.
-constexpr int BATCH_ERR_WORD = 32;
-
 int rebuild(fdtd_batch *b)
 {
     std::vector<BatchDesc> descs(b->solves.size());
@@ -265,7 +262,7 @@ int rebuild(fdtd_batch *b)
     bool strip = b->compact && b->strip_shape >= 0;
     for (auto *v : b->solves)
         if (strip) {
-            NativeConsts c = solve_consts(v, 0, b->d_work + BATCH_ERR_WORD);
+            NativeConsts c = solve_consts(v, 0, b->d_err);
             strip = strip_usable(c, b->r16);
         }
     const int ty = strip ? strip_shape_rows(b->strip_shape) : fused_tile_height();
@@ -293,7 +290,7 @@ int rebuild(fdtd_batch *b)
         BatchDesc &d = descs[i];
         std::memset(&d, 0, sizeof d);
         for (int par = 0; par < 2; par++) {
-            d.c[par] = solve_consts(v, par, b->d_work + BATCH_ERR_WORD);
+            d.c[par] = solve_consts(v, par, b->d_err);
             // the step kernel applies the x-face Mur updates (D form, 20 solves of
             // 48-256 cells per axis: 605 us per step, 631 with the strided faces
             // in the Mur launch; of 24-128: 131 and 136)
@@ -506,9 +503,9 @@ int fdtd_batch_create_form(int device, int kernel, fdtd_batch **out)
     for (int k = 0; k < 2 && st == FDTD_OK; k++)
         st = cu(cudaEventCreateWithFlags(&b->stage[k].done, cudaEventDisableTiming));
     if (st == FDTD_OK)
-        st = cu(cudaMalloc(&b->d_work, 256));
+        st = cu(cudaMalloc(&b->d_err, sizeof(int)));
     if (st == FDTD_OK)
-        st = cu(cudaMemset(b->d_work, 0, 256));
+        st = cu(cudaMemset(b->d_err, 0, sizeof(int)));
     if (st != FDTD_OK) {
         fdtd_batch_destroy(b);
         return st;
@@ -540,7 +537,7 @@ int fdtd_batch_destroy(fdtd_batch *b)
         cudaFreeAsync(b->d_units, s);
     if (s)
         cudaStreamSynchronize(s);
-    cudaFree(b->d_work);
+    cudaFree(b->d_err);
     for (auto &sb : b->stage) {
         if (sb.host)
             cudaFreeHost(sb.host);
@@ -798,9 +795,9 @@ int fdtd_batch_synchronize(fdtd_batch *b)
     int st = cu(cudaStreamSynchronize(b->stream));
     int flag = 0;
     if (st == FDTD_OK)
-        st = cu(cudaMemcpy(&flag, b->d_work + BATCH_ERR_WORD, sizeof flag, cudaMemcpyDeviceToHost));
+        st = cu(cudaMemcpy(&flag, b->d_err, sizeof flag, cudaMemcpyDeviceToHost));
     if (st == FDTD_OK && flag) {
-        cudaMemset(b->d_work + BATCH_ERR_WORD, 0, sizeof flag);
+        cudaMemset(b->d_err, 0, sizeof flag);
         st = FDTD_ERR_DEVICE_TIMEOUT;
     }
     if (b->timing)

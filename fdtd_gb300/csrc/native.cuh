@@ -249,7 +249,6 @@ struct BatchLaunch {
 };
 
 // Tensor maps of a single-pass launch over c's buffers (false: not encodable).
-bool encode_fused_maps(const NativeConsts &c, FusedMaps *maps);
 bool encode_step_maps(const NativeConsts &c, bool compact, FusedMaps *maps, bool r16 = false);
 int fused_tile_height();
 int zchunk_limited(int nz, int max_planes);  // nz in equal chunks of at most max_planes planes

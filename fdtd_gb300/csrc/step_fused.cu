@@ -103,10 +103,10 @@ __device__ void issue_plane_tma(const FusedMaps &maps, unsigned char *stage, uin
         tma_load_3d(smem_addr(stage + G::OFF_X), &maps.m[7 + NT], y0, x0 / FTX, z, bar);
 }
 
-// Generic: every thread copies part of each box with 4-byte cp.async
-// (zero-filled outside the grid); the material classes are read separately,
-// and so are 16-bit R and its scale words (no tiles staged for them).
-template <int TY, int NT = 9, int TB = 4, int XB = 0>
+// Generic (compact forms): every thread copies part of each box with 4-byte
+// cp.async (zero-filled outside the grid); the material classes are read
+// separately, and so are 16-bit R and its scale words (no tiles staged for them).
+template <int TY, int NT, int TB, int XB>
 __device__ void issue_plane_generic(const NativeConsts &c, unsigned char *stage, int kind, int x0, int y0, int z,
                                     int tid)
 {
@@ -130,11 +130,9 @@ __device__ void issue_plane_generic(const NativeConsts &c, unsigned char *stage,
         box(c.h_in[k], smem_addr(stage + G::OFF_H + k * pad128(G::H_BYTES)), x0 - 4, y0 - 1, G::HW, G::HH);
     if (kind == PLANE_PRO)
         return;
-    const float *tiles[9] = {c.d_cur[0], c.d_cur[1], c.d_cur[2], c.d_prev[0], c.d_prev[1],
-                             c.d_prev[2], c.e_prev[0], c.e_prev[1], c.e_prev[2]};
-    if (TB == 4)
-        for (int k = 0; k < NT; k++)
-            box(tiles[k], smem_addr(stage + G::OFF_T + k * pad128(G::T_BYTES)), x0, y0, FTX, TY);
+    if (TB == 4)  // R
+        for (int k = 0; k < 3; k++)
+            box(c.d_cur[k], smem_addr(stage + G::OFF_T + k * pad128(G::T_BYTES)), x0, y0, FTX, TY);
 }
 
 // ---------------------------------------------------------------- the kernel
@@ -178,6 +176,7 @@ __device__ __forceinline__ void fused_unit(const NativeConsts &c, const FusedMap
 {
     static_assert(COMPACT || !R16, "16-bit R is a compact-form layout");
     static_assert(TMA || !MOVER, "a moving warp issues TMA loads");
+    static_assert(TMA || COMPACT, "D-form arrays that TMA cannot address take the two-pass kernels");
     constexpr int NT = COMPACT ? 3 : 9, TB = R16 ? 2 : 4, XB = R16 ? TY * 4 : 0;
     using G = Geo<TY, NT, TB, XB>;
     const int nx = c.nx, ny = c.ny, nz = c.nz;
@@ -553,14 +552,7 @@ __device__ __forceinline__ void fused_unit(const NativeConsts &c, const FusedMap
                 const float dn0 = T[0 * TS + t], dn1 = T[1 * TS + t], dn2 = T[2 * TS + t];
                 const float dp0 = T[3 * TS + t], dp1 = T[4 * TS + t], dp2 = T[5 * TS + t];
                 const float ep0 = T[6 * TS + t], ep1 = T[7 * TS + t], ep2 = T[8 * TS + t];
-                uint8_t cls;
-                if (TMA) {
-                    cls = (stage_k + G::OFF_M)[t];
-                } else {
-                    cls = mat_next;
-                    if (z + 1 < zc1)
-                        mat_next = c.mat[i + plane];
-                }
+                const uint8_t cls = (stage_k + G::OFF_M)[t];
                 // H^{n+1/2}: write the updated components
                 if (x >= 1 && x < nx - 1 && y < ny - 1 && zlo)
                     c.h_out[0][i] = hxn;
@@ -1029,8 +1021,6 @@ bool encode_step_maps(const NativeConsts &c, bool compact, FusedMaps *maps, bool
     }
     return ok;
 }
-
-bool encode_fused_maps(const NativeConsts &c, FusedMaps *maps) { return encode_step_maps(c, false, maps); }
 
 int fused_tile_height() { return TY_SEL; }
 
